@@ -74,6 +74,7 @@ __device__ __forceinline__ int varint_len(uint64_t v) {
   int bits = 64 - __clzll((long long)v);
   return bits == 0 ? 1 : (bits + 6) / 7;
 }
+__device__ __forceinline__ int varint_len32(uint32_t v) { return (38 - __clz((int)(v | 1u))) / 7; }
 __device__ __forceinline__ int varint_len(u128 v) {
   int bits = 128 - clz_key(v);
   return bits == 0 ? 1 : (bits + 6) / 7;

@@ -565,10 +565,13 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   T* sorted = ctx->keys_a.as<T>();
   T* scratch = ctx->keys_b.as<T>();
   const T* tile_spl = nullptr;  // the splitters that cut every bucket into its S tiles
-  std::vector<TileDesc> ht;  // one tile per bucket (S == 1): made on the host
-  uint32_t dev_tiles = 0;    // S > 1: the tiles made on the device
   if (S == 1) {
-    for (uint32_t b = 0; b < PT; ++b) ht.push_back(TileDesc{boff[b], (uint32_t)bcount[b], b});
+    // one tile per bucket
+    KCU(ctx->tiles.ensure((size_t)PT * sizeof(TileDesc)));
+    KCU(ctx->tile_fill.ensure((size_t)PT * 4));
+    launch_make_tiles(ctx->bucket_off.as<unsigned long long>(), PT, 1, 1, N, ctx->tiles.as<TileDesc>(),
+                      ctx->tile_fill.as<uint32_t>(), s);
+    st.kernel_launches += 1;
   } else {
     // Splitters: SAMPLED = histogram only; LEARNED = train the CDF and keep
     // it unless its predicted max/mean tile load exceeds imbalance_bound AND
@@ -725,15 +728,11 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     launch_make_tiles(ctx->tile_off.as<unsigned long long>(), (uint32_t)nt, S, G, N, ctx->tiles.as<TileDesc>(),
                       ctx->tile_fill.as<uint32_t>(), s);
     KCU(cudaGetLastError());
-    // the tile lengths stay on the device: the oversized tiles are listed
-    // there and the sort follows without a host round trip
-    dev_tiles = (uint32_t)nt;
     sorted = level_out;
     scratch = level_in;
   }
   KCU(cudaEventRecord(ctx->ev[4], s));
-  const uint32_t ntiles = dev_tiles ? dev_tiles : (uint32_t)ht.size();
-  const uint32_t Sl = ntiles / PT;  // tiles per bucket
+  const uint32_t ntiles = PT * S;
   const T kmax = 2 * k >= (uint32_t)KeyTraits<T>::kBits ? ~T(0) : ((T(1) << (2 * k)) - T(1));
   // Bucket groups: each group's tiles are sorted, linked and encoded in turn,
   // so one group's payload copies to the host while the next one sorts.
@@ -746,65 +745,27 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     static const uint32_t cw[9] = {0, 6, 12, 18, 24, 30, 35, 38, 40};
     for (uint32_t g = 0; g <= NG; ++g) gb[g] = (uint32_t)((uint64_t)PT * cw[g] / 40);
   }
-  // Oversized tiles, group by group: those sorted on chip at twice the
-  // capacity (list A) and those sorted through global memory (list B).  From
-  // device-made tiles the lists are made on the device (group g's entries
-  // from index gb[g] * S, counts lcnt[2g], lcnt[2g+1]) and walked by a fixed
-  // grid; from host tiles on the host, one CTA per listed tile.
-  std::vector<uint32_t> big, gbig(NG + 1, 0), glarge(NG, 0);
-  KCU(ctx->big_ids.ensure((size_t)2 * ntiles * 4 + 8));
+  // The tiles that the tile sort's tables leave to the binning sort, group by
+  // group, listed by the sort itself (group g's entries from index gb[g] * S,
+  // its counters at lcnt[4g]) and walked by a fixed grid: those within the
+  // on-chip capacity, within twice it (list A), and those sorted through global
+  // memory (B).  The tile lengths and lists stay on the device: no host round
+  // trip.
+  KCU(ctx->big_ids.ensure((size_t)3 * ntiles * 4 + 8));
   uint32_t* ids_a = ctx->big_ids.as<uint32_t>();
   uint32_t* ids_b = ids_a + ntiles;
-  unsigned* lcnt = nullptr;
-  const size_t lhead = (size_t)(2 * NG + 8) * 8;  // counts, then the group bounds
-  const size_t lbytes = lhead + (size_t)(4 + S) * 8;
-  if (dev_tiles) {
-    KCU(ctx->tile_lists.ensure(lbytes + 64));
-    lcnt = ctx->tile_lists.as<unsigned>();
-    // [0] largest tile, [1] keys, [2] non-empty tiles, [3] keys in tiles above
-    // capacity, then the S range sums
-    unsigned long long* lstats = reinterpret_cast<unsigned long long*>(ctx->tile_lists.as<uint8_t>() + lhead);
-    KCU(cudaMemsetAsync(ctx->tile_lists.p, 0, lbytes, s));
-    uint32_t* dgb = reinterpret_cast<uint32_t*>(lcnt + 2 * NG);
-    KCU(ctx->h_tiles.ensure(lbytes + 64));
-    std::memcpy(ctx->h_tiles.p, gb.data(), (NG + 1) * 4);
-    KCU(cudaMemcpyAsync(dgb, ctx->h_tiles.p, (NG + 1) * 4, cudaMemcpyHostToDevice, s));
-    launch_tile_lists(ctx->tile_fill.as<uint32_t>(), ntiles, S, dgb, NG, CAP, ids_a, ids_b, lcnt, lstats, lstats + 4,
-                      s);
-    st.kernel_launches += 1;
-    st.tiles = ntiles;
-  } else {
-    for (uint32_t g = 0; g < NG; ++g) {
-      gbig[g] = (uint32_t)big.size();
-      for (uint32_t t = gb[g] * Sl; t < gb[g + 1] * Sl; ++t)
-        if (ht[t].len > CAP && ht[t].len <= 2 * CAP) big.push_back(t);
-      glarge[g] = (uint32_t)big.size() - gbig[g];
-      for (uint32_t t = gb[g] * Sl; t < gb[g + 1] * Sl; ++t)
-        if (ht[t].len > 2 * CAP) big.push_back(t);
-    }
-    gbig[NG] = (uint32_t)big.size();
-    uint64_t tmax = 0, tsum = 0, tne = 0;
-    for (uint32_t t = 0; t < ntiles; ++t)
-      if (ht[t].len) {
-        tmax = std::max<uint64_t>(tmax, ht[t].len);
-        tsum += ht[t].len;
-        tne++;
-      }
-    st.tiles = ntiles;
-    st.big_tiles = (uint32_t)big.size();
-    for (uint32_t t : big) st.big_tile_keys += ht[t].len;
-    st.tile_imbalance = tne ? (double)tmax / ((double)tsum / (double)tne) : 0.0;
-    st.range_imbalance = 1.0;  // one tile per bucket
-    KCU(ctx->h_tiles.ensure(ht.size() * sizeof(TileDesc) + big.size() * 4 + 64));
-    std::memcpy(ctx->h_tiles.p, ht.data(), ht.size() * sizeof(TileDesc));
-    KCU(ctx->tiles.ensure(ht.size() * sizeof(TileDesc)));
-    KCU(cudaMemcpyAsync(ctx->tiles.p, ctx->h_tiles.p, ht.size() * sizeof(TileDesc), cudaMemcpyHostToDevice, s));
-    if (!big.empty()) {
-      uint8_t* hb2 = ctx->h_tiles.as<uint8_t>() + ht.size() * sizeof(TileDesc);
-      std::memcpy(hb2, big.data(), big.size() * 4);
-      KCU(cudaMemcpyAsync(ids_a, hb2, big.size() * 4, cudaMemcpyHostToDevice, s));
-    }
-  }
+  uint32_t* ids_1 = ids_b + ntiles;
+  const bool some_above = S > 1 || maxb > CAP;  // one tile per bucket: the host knows their sizes
+  const size_t lhead = (size_t)(2 * NG + 8) * 8;  // per group: list counts, tiles handed out; tiles met; then the statistics
+  const size_t lbytes = lhead + (size_t)(8 + S) * 8;
+  KCU(ctx->tile_lists.ensure(lbytes + 64));
+  KCU(ctx->h_tiles.ensure(lbytes + 64));
+  unsigned* lcnt = ctx->tile_lists.as<unsigned>();
+  unsigned long long* lstats = reinterpret_cast<unsigned long long*>(ctx->tile_lists.as<uint8_t>() + lhead);
+  KCU(cudaMemsetAsync(ctx->tile_lists.p, 0, lbytes, s));
+  launch_tile_stats(ctx->tile_fill.as<uint32_t>(), ntiles, S, CAP, lstats, lstats + 8, s);
+  st.kernel_launches += 1;
+  st.tiles = ntiles;
   int sm_count = 0;
   cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, ctx->cfg.device);
   const uint32_t walk_grid = (uint32_t)std::max(1, sm_count);
@@ -822,8 +783,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   ctx->res_on_host = false;
   ctx->res_meta.assign(PT, BucketMeta{});
   st.kernel_launches += 1 + (uint64_t)NG * 3 + (uint64_t)NG * 3;  // memset, per group: sort, link, offsets, encode
-  for (uint32_t g = 0; g < NG; ++g)
-    st.kernel_launches += dev_tiles ? 2 : (glarge[g] ? 1 : 0) + (gbig[g + 1] - gbig[g] > glarge[g] ? 1 : 0);
+  st.kernel_launches += (uint64_t)NG * (some_above ? 3 : 1);  // the listed tiles
   cudaEvent_t* gev = ctx->gev.data();  // per group: sort, large, link | encode | copy start/end
   TileOut<T>* tout = ctx->tile_out.as<TileOut<T>>();
   BucketMeta* meta = ctx->meta.as<BucketMeta>();
@@ -836,29 +796,26 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
 
   // ---- K4 tile sort + RLE, K5 link and byte offsets (one group) --------------
   auto queue_sort = [&](uint32_t g) -> cudaError_t {
-    const uint32_t t0 = gb[g] * Sl, nt = (gb[g + 1] - gb[g]) * Sl, nb = gb[g + 1] - gb[g];
+    const uint32_t t0 = gb[g] * S, nt = (gb[g + 1] - gb[g]) * S, nb = gb[g + 1] - gb[g];
+    unsigned long long* sstats = ctx->sort_stats.as<unsigned long long>();
     cudaEventRecord(gev[8 * g], s);
-    launch_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>() + t0, nt, tout + t0,
-                        ctx->sort_stats.as<unsigned long long>(), TileRanges<T>{tile_spl, Sl, t0, kmax, ctx->cfg.tile_wait_polls}, s);
+    launch_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>() + t0, nt, tout + t0, sstats,
+                        TileRanges<T>{tile_spl, S, t0, kmax, ctx->cfg.tile_wait_polls},
+                        TileRetry{ids_1 + t0, ids_a + t0, ids_b + t0, lcnt + 4 * g, lcnt + 4 * g + 3, lcnt + 4 * NG, t0,
+                                  CAP},
+                        s);
+    launch_tile_sort_listed<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_1 + t0, walk_grid,
+                               lcnt + 4 * g + 2, tout, sstats,
+                               TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls}, s);
     cudaEventRecord(gev[8 * g + 1], s);
-    if (dev_tiles) {
-      launch_tile_sort_large<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_a + t0, walk_grid,
-                                lcnt + 2 * g, tout, ctx->sort_stats.as<unsigned long long>(),
-                                TileRanges<T>{tile_spl, Sl, 0, kmax, ctx->cfg.tile_wait_polls}, s);
-      launch_big_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), scratch, ctx->tiles.as<TileDesc>(), ids_b + t0,
-                              walk_grid, lcnt + 2 * g + 1, tout, ctx->status.as<DevStatus>(),
-                              ctx->sort_stats.as<unsigned long long>(), s);
-    } else {
-      launch_tile_sort_large<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_a + gbig[g],
-                                glarge[g], nullptr, tout, ctx->sort_stats.as<unsigned long long>(),
-                                TileRanges<T>{tile_spl, Sl, 0, kmax, ctx->cfg.tile_wait_polls}, s);
-      launch_big_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), scratch, ctx->tiles.as<TileDesc>(),
-                              ids_a + gbig[g] + glarge[g], gbig[g + 1] - gbig[g] - glarge[g], nullptr, tout,
-                              ctx->status.as<DevStatus>(), ctx->sort_stats.as<unsigned long long>(), s);
-    }
+    if (some_above) launch_tile_sort_large<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_a + t0, walk_grid,
+                              lcnt + 4 * g, tout, sstats, TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls},
+                              s);
+    if (some_above) launch_big_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), scratch, ctx->tiles.as<TileDesc>(), ids_b + t0,
+                            walk_grid, lcnt + 4 * g + 1, tout, ctx->status.as<DevStatus>(), sstats, s);
     cudaEventRecord(gev[8 * g + 2], s);
     // ---- K5: per-bucket tile links, byte offsets from the group's start
-    launch_tile_link<T>(tout + t0, nb, Sl, ctx->tile_boff.as<unsigned long long>() + t0, ctx->tile_prev.as<T>() + t0,
+    launch_tile_link<T>(tout + t0, nb, S, ctx->tile_boff.as<unsigned long long>() + t0, ctx->tile_prev.as<T>() + t0,
                         meta + gb[g], s);
     launch_bucket_offsets(meta + gb[g], nb, hmeta_dev + gb[g], s);
     cudaEventRecord(gev[8 * g + 3], s);
@@ -902,7 +859,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     if (g + 1 < NG) KCU(queue_sort(g + 1));
     rc = wait_event(ctx, gev[8 * g + 3]);
     if (rc) return rc;
-    const uint32_t t0 = gb[g] * Sl, nt = (gb[g + 1] - gb[g]) * Sl;
+    const uint32_t t0 = gb[g] * S, nt = (gb[g + 1] - gb[g]) * S;
     uint64_t gbytes = 0;
     for (uint32_t b = gb[g]; b < gb[g + 1]; ++b) {
       BucketMeta m = hmeta[b];
@@ -937,7 +894,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   KCU(cudaStreamWaitEvent(s, gev[8 * (NG - 1) + 5], 0));
   KCU(cudaEventRecord(ctx->ev[7], s));
   KCU(cudaMemcpyAsync(ctx->h_small.p, ctx->sort_stats.p, 16, cudaMemcpyDeviceToHost, s));
-  if (dev_tiles) KCU(cudaMemcpyAsync(ctx->h_tiles.p, ctx->tile_lists.p, lbytes, cudaMemcpyDeviceToHost, s));
+  KCU(cudaMemcpyAsync(ctx->h_tiles.p, ctx->tile_lists.p, lbytes, cudaMemcpyDeviceToHost, s));
   rc = wait_stream(ctx, s);
   const auto wall2 = clk::now();
   if (!rc && to_host) rc = wait_stream(ctx, ctx->copy_stream);
@@ -949,17 +906,14 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   std::memcpy(&st.big_tile_rows, ctx->h_small.as<uint8_t>() + 8, 8);
   // the tile sort adds 2^40 to its statistics when a tile's bulk load did not complete
   if (st.sort_fallbacks >> 40) return fail(ctx, KITE_ERR_TIMEOUT, "tile sort: a bulk load of a tile did not complete");
-  if (dev_tiles) {
-    const unsigned* hc = ctx->h_tiles.as<unsigned>();
+  {
     const unsigned long long* hs2 = reinterpret_cast<const unsigned long long*>(ctx->h_tiles.as<uint8_t>() + lhead);
-    uint32_t nbig = 0;
-    for (uint32_t g = 0; g < 2 * NG; ++g) nbig += hc[g];
-    st.big_tiles = nbig;
+    st.big_tiles = (uint32_t)hs2[4];
     st.tile_imbalance = hs2[2] ? (double)hs2[0] / ((double)hs2[1] / (double)hs2[2]) : 0.0;
     unsigned long long rmax = 0;
-    for (uint32_t t = 0; t < S; ++t) rmax = std::max(rmax, hs2[4 + t]);
+    for (uint32_t t = 0; t < S; ++t) rmax = std::max(rmax, hs2[8 + t]);
     st.big_tile_keys = hs2[3];
-    st.range_imbalance = (double)rmax / ((double)N / S);
+    st.range_imbalance = S > 1 ? (double)rmax / ((double)N / S) : 1.0;  // 1: one tile per bucket
   }
   rc = check_status(ctx, "count");
   if (rc) return rc;

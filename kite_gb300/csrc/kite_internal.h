@@ -197,11 +197,39 @@ struct TileRanges {
 // `fallbacks` (device counters): [0] tiles that took the LSD fallback (plus
 // 2^40 for a tile whose bulk load did not complete), [1] rows of the tiles
 // above the on-chip capacity (double-capacity and global-memory sorts).
+// The lists of the tiles that the tile sort's tables leave to the binning sort.
+struct TileRetry {
+  uint32_t* ids1;   // tiles of at most tile_capacity keys
+  uint32_t* ids;    // of at most 2 * tile_capacity
+  uint32_t* ids2;   // larger ones
+  unsigned* cnt;    // [0] entries of ids, [1] of ids2, [2] of ids1
+  unsigned* taken;  // tiles handed out beyond the CTAs' first ones (zero before the launch)
+  unsigned* met;    // [0] tiles tried, [1] those better binned, over the whole count
+  uint32_t tile0;   // id of the launch's first tile
+  uint32_t cap;     // tile_capacity
+#ifdef __CUDACC__
+  __device__ __forceinline__ void add(uint32_t i, uint32_t n) const {  // the launch's tile i, of n keys
+    if (n <= cap) ids1[atomicAdd(&cnt[2], 1u)] = tile0 + i;
+    else if (n <= 2 * cap) ids[atomicAdd(&cnt[0], 1u)] = tile0 + i;
+    else ids2[atomicAdd(&cnt[1], 1u)] = tile0 + i;
+  }
+  __device__ __forceinline__ void met_tile(bool better_binned) const {
+    atomicAdd(&met[0], 1u);
+    if (better_binned) atomicAdd(&met[1], 1u);
+  }
+#endif
+};
 template <class T>
 void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t ntiles, TileOut<T>* out,
-                      unsigned long long* fallbacks, TileRanges<T> rg, cudaStream_t s);
+                      unsigned long long* fallbacks, TileRanges<T> rg, TileRetry retry, cudaStream_t s);
+// The binning sort of the tiles listed in ids (at most tile_capacity keys each),
+// their number on the device; two CTAs for each of `grid`.
+template <class T>
+void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
+                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+                             TileRanges<T> rg, cudaStream_t s);
 // Tiles of tile_capacity < len <= 2 * tile_capacity, listed in ids: the same
-// on-chip sort with twice the shared memory (one CTA per SM).  With nids_dev,
+// binning sort with twice the shared memory (one CTA per SM).  With nids_dev,
 // the list's length is on the device and the nids CTAs walk it in turn.
 template <class T>
 void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
@@ -214,10 +242,8 @@ template <class T>
 void launch_big_tile_sort(T* keys, uint32_t* counts, T* scratch, const TileDesc* tiles, const uint32_t* big_ids,
                           uint32_t nbig, const unsigned* nbig_dev, TileOut<T>* out, DevStatus* st,
                           unsigned long long* sort_stats, cudaStream_t s);
-// Per bucket group, the tiles above capacity (lists and counts on the
-// device) and the tile statistics; see k_tile_lists.
-void launch_tile_lists(const uint32_t* lens, uint32_t ntiles, uint32_t S, const uint32_t* gb, uint32_t NG,
-                       uint32_t cap, uint32_t* ids, uint32_t* ids2, unsigned* cnt, unsigned long long* stats,
+// Tile statistics; see k_tile_stats.
+void launch_tile_stats(const uint32_t* lens, uint32_t ntiles, uint32_t S, uint32_t cap, unsigned long long* stats,
                        unsigned long long* range, cudaStream_t s);
 
 // ---- encode_kernels.cu ----

@@ -2,11 +2,14 @@
 // radix_sort_u64_kmer / radix_sort_u128_kmer src/count/sorter.rs:67-93,
 // :388-437, then rle_compress_typed :514-530 with u32 saturation).
 //
-// A tile is a key range of one hash bucket.  One CTA loads the whole tile into
-// shared memory, orders it by a 16384-bin counting pass over its key span (bins
+// A tile is a key range of one hash bucket, sorted by one CTA.  Tiles whose keys
+// repeat (reads at some depth) are counted in a table of distinct keys; the
+// others are ordered by a 16384-bin counting pass over their key span (bins
 // holding several distinct keys are finished by a thread or a warp, rare
-// pathological ones by LSD passes), then emits unique (key, count) rows in
-// place and the tile's DVLE size for every row but the first.
+// pathological ones by LSD passes).  Either way unique (key, count) rows come
+// out in place, with the tile's DVLE size for every row but the first.
+#include <algorithm>
+
 #include "kite_internal.h"
 
 namespace kite {
@@ -130,7 +133,6 @@ constexpr int kBinBits = 14, kBins = 1 << kBinBits;
 constexpr unsigned kSmallBin = 16;     // marked bins a single thread sorts
 constexpr unsigned kMaxMixed = 256;    // largest bin ranked by counting when it has many distinct keys
 constexpr unsigned kMaxDistinct = 32;  // distinct keys a warp extracts from one large bin
-constexpr int kLoadBatch = 8;          // global loads a thread keeps in flight
 
 // MULT = 1: the regular tile (8192 u64 / 4096 u128 keys, two CTAs per SM);
 // MULT = 2: twice that, with twice the threads, for the oversized tiles (one
@@ -571,6 +573,712 @@ __device__ __forceinline__ void sort_tile(uint32_t tid, T* __restrict__ keys, ui
   }
 }
 
+// ---------------------------------------------------------------------------
+// Tile sort by an order-preserving hash table.  The keys of a tile are counted
+// in a shared-memory table of distinct keys whose home slots grow with the
+// key, so that reading the table out is already almost sorted:
+//  1. a key's home slot is its place in the tile's key range [lo, hi] (its
+//     splitters), scaled to the table; a key that finds another one there takes
+//     the next free slot (linear probing, no wrap-around).  Every slot from a
+//     key's home to its place is then occupied, so the keys of one run of
+//     occupied slots (a cluster) all lie below those of the next run;
+//  2. the clusters of two and more are put in order, one lane each (insertion;
+//     typically two keys), and the occupied slots are listed in order;
+//  3. the listed keys and counts go out as rows over the tile's keys in global
+//     memory, with the DVLE size of every row but the first.
+// Copies of a key never move: a duplicate costs one compare-and-swap that finds
+// it and one counter add.  The binning sort moves every key twice and then
+// finishes the bins that hold several keys, 6.5 warp instructions per key in
+// all; the table takes 4.9 on the same tiles and is bound by instruction issue
+// (about 55%) and shared-memory wavefronts (about 55%) alike, with the latency
+// of both between its five barriers.
+// Measured (150 bp reads, k = 31, 30-fold, one distinct key in 3.6): 10M reads
+// 12.4 -> 7.9 ms, 1M reads 1.58 -> 0.96 ms.
+// Two CTAs per SM walk the tiles; a tile's descriptor, key range and first keys
+// are fetched while the one before it is worked on.
+// A key that would land kProbeLimit slots or more from home (keys clustered in
+// a small part of the range, or too many distinct keys for the table) has the
+// tile counted again with hashed homes, where only too many distinct keys fail:
+// its distinct keys are then binned and ranked.  A tile that fails there too
+// goes to the binning sort, through a list; data that often does so is listed
+// without the try (choose_next).
+//
+// The keys (u64, k <= 31) sit in the table themselves, claimed by a 64-bit
+// compare-and-swap on an all-ones slot, which no key of at most 62 bits is;
+// they stream through registers, so a tile may hold any number of keys.
+// ---------------------------------------------------------------------------
+constexpr unsigned kProbeLimit = 32;
+constexpr unsigned kHashProbes = 96;   // with hashed homes
+constexpr unsigned kMaxRanked = 512;   // distinct keys of a bin ranked by counting
+constexpr unsigned kHashAny = 1024;  // u128 tiles of at most so many keys always suit the table
+
+struct TableSmem {
+  static constexpr int NT = 512, NW = NT / 32, SLOTS = 7168, HSLOTS = 6144, BINS = 4096;
+  static constexpr size_t o_tab = 0;                              // keys
+  static constexpr size_t o_cnt = o_tab + (size_t)SLOTS * 8;      // their counts (u32)
+  static constexpr size_t o_ord = o_cnt + (size_t)SLOTS * 4;      // the occupied slots in order (u16)
+  // hashed homes: fewer slots, and behind them the slots in bin order (u16)
+  static constexpr size_t o_hcnt = o_tab + (size_t)HSLOTS * 8;
+  static constexpr size_t o_tmp = o_hcnt + (size_t)HSLOTS * 4;
+  static_assert(o_tmp + (size_t)HSLOTS * 2 <= o_ord, "the hashed layout fits the other's table and counts");
+  // per warp: 64 keys that probe on, or 256 clusters (u16); hashed homes: 4096 bins (u16)
+  static constexpr size_t o_queue = o_ord + (size_t)SLOTS * 2;
+  static constexpr size_t o_edge = o_queue + (size_t)NW * 512;    // the warps' totals
+  static constexpr size_t o_misc = o_edge + (size_t)NW * 4;
+  static constexpr size_t total = o_misc + 32;
+};
+
+// A key's place in the tile's key range [lo, hi]: the 32 bits of its distance
+// from lo that start at hi's top bit (a monotone map of the range).
+template <class T>
+struct RangeMap {
+  T lo;
+  int lz;
+  __device__ __forceinline__ RangeMap(T mn, T mx) : lo(mn), lz(mx == mn ? 0 : clz_key(T(mx - mn))) {}
+  __device__ __forceinline__ uint32_t at(T key) const {
+    const T v = key - lo;
+    if constexpr (sizeof(T) == 8) {
+      return (uint32_t)((v << lz) >> 32);
+    } else {
+      const uint64_t vh = hi64(v), vl = (uint64_t)v;
+      const uint64_t h = lz < 64 ? vh : vl, l = lz < 64 ? vl : 0ull;
+      const uint32_t a = (lz & 32) ? (uint32_t)h : (uint32_t)(h >> 32), b = (lz & 32) ? (uint32_t)(l >> 32) : (uint32_t)h;
+      return __funnelshift_l(b, a, lz & 31);
+    }
+  }
+};
+
+// width * 2^32 / gap, rounded down a little, so that the places x < gap of an
+// interval are spread over `width` slots by __umulhi(x, scale).
+__device__ __forceinline__ uint32_t home_scale(uint32_t width, uint32_t gap) {
+  const float f = __fdividef((float)width * 4294967296.f, (float)gap) * 0.999999f;
+  return gap == 0 ? 0u : f < 4294960000.f ? (uint32_t)f : 0xffffffffu;
+}
+
+// Home slot of a key: its place in the range scaled to the homes.
+template <class T>
+struct HomeLinear {
+  RangeMap<T> map;
+  uint32_t scale, last;
+  __device__ __forceinline__ HomeLinear(const RangeMap<T>& m, T mx, uint32_t homes)
+      : map(m), scale(home_scale(homes, m.at(mx))), last(homes - 1) {}
+  __device__ __forceinline__ uint32_t operator()(T key) const {
+    const uint32_t b = __umulhi(map.at(key), scale);
+    return b < last ? b : last;  // a key outside the range cannot leave the table
+  }
+};
+
+template <class T>
+__device__ __forceinline__ void empty_tile(TileOut<T>* out) {
+  TileOut<T> o;
+  o.first_key = o.last_key = T(0);
+  o.rows = 0;
+  o.first_count = 0;
+  o.rest_bytes = 0;
+  *out = o;
+}
+
+// A tile as the sort meets it: its keys and its key range.
+template <class T>
+struct TileIn {
+  uint64_t start;
+  uint32_t n;
+  T mn, mx;
+};
+template <class T>
+__device__ __forceinline__ TileIn<T> tile_in(const TileDesc* tiles, uint32_t i, uint32_t ntiles, const TileRanges<T>& rg) {
+  TileIn<T> t;
+  t.start = 0;
+  t.n = 0;
+  t.mn = T(0);
+  t.mx = rg.kmax;
+  if (i >= ntiles) return t;
+  const TileDesc td = tiles[i];
+  t.start = td.start;
+  t.n = td.len;
+  const uint32_t tl = rg.tile0 + i - td.bucket * rg.S;  // the tile's range in its bucket
+  if (tl > 0) t.mn = rg.spl[tl - 1];
+  if (tl + 1 < rg.S) {
+    const T e = rg.spl[tl];
+    t.mx = e > t.mn ? T(e - T(1)) : t.mn;
+  }
+  return t;
+}
+
+// The CTA's next tile, chosen by thread 0 while the one before it is worked
+// on: next[0] = the tile, next[1] = 1 when it is the first of 32 taken at once,
+// of which list_others leaves the others to the binning sort.  That is so while
+// the tables have met 16 tiles and more than a quarter of them were better
+// binned; one tile in 32 (and, of the CTAs' first ones, one CTA in 32) still
+// tries.  (1M random 150 bp reads, every key once:
+// 1.68 ms binned, 6.9 ms when every tile tried the u64 table first, 1.72 ms so.)
+__device__ __forceinline__ bool mostly_binned(const TileRetry& r) {
+  const unsigned a = *(volatile unsigned*)&r.met[0], f = *(volatile unsigned*)&r.met[1];
+  return a >= 16 && 4 * f > a;
+}
+__device__ __forceinline__ void choose_next(const TileRetry& r, unsigned* next) {
+  const bool many = mostly_binned(r);
+  next[0] = gridDim.x + atomicAdd(r.taken, many ? 32u : 1u);
+  next[1] = many;
+}
+template <class T>
+__device__ __forceinline__ void list_others(const TileRetry& r, const unsigned* next, const TileDesc* tiles,
+                                            uint32_t ntiles, TileOut<T>* tout) {
+  if (threadIdx.x == 0 || threadIdx.x >= 32 || !next[1] || next[0] + threadIdx.x >= ntiles) return;
+  const uint32_t i = next[0] + threadIdx.x, n = tiles[i].len;
+  if (n) r.add(i, n);
+  else empty_tile(&tout[i]);
+}
+
+__device__ __forceinline__ unsigned warp_inclusive(unsigned v, unsigned lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= (unsigned)o) v += y;
+  }
+  return v;
+}
+
+// The U rows of a sorted tile (row(u, &key, &count)) to global memory, and the
+// tile's record.  Each warp takes consecutive rows; a lane's previous key comes
+// from the lane below, and from the round before for the first lane.  `rest`
+// is a zeroed counter, zeroed again; one barrier inside, after the last row has
+// been read.
+template <int NT, class T, class F>
+__device__ __forceinline__ void write_rows(unsigned U, T* g, uint32_t* gc, unsigned* rest_sum, TileOut<T>* out, F&& row) {
+  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned per = (U + NT - 1) / NT * 32;  // rows per warp
+  const unsigned ub = wid * per, ue = min(U, ub + per);
+  unsigned rest = 0;
+  if (ub < ue) {
+    T below = T(0);  // the key before the round's first row
+    uint32_t x;
+    if (ub) row(ub - 1, &below, &x);
+    for (unsigned u0 = ub; u0 < ue; u0 += 32) {
+      const unsigned u = u0 + lane;
+      T key = T(0);
+      uint32_t c = 0;
+      if (u < ue) row(u, &key, &c);
+      T prev = shfl_up_key(key, 1);
+      if (lane == 0) prev = below;
+      below = shfl_key(key, 31);
+      if (u < ue) {
+        g[u] = key;
+        gc[u] = c;
+        if (u) rest += varint_len(T(key - prev)) + varint_len32(c);
+      }
+    }
+  }
+  rest = __reduce_add_sync(0xffffffffu, rest);
+  if (lane == 0 && rest) atomicAdd(rest_sum, rest);
+  TileOut<T> o;
+  if (threadIdx.x == 0) {
+    uint32_t x;
+    row(0, &o.first_key, &o.first_count);
+    row(U - 1, &o.last_key, &x);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    o.rows = U;
+    o.rest_bytes = *rest_sum;
+    *out = o;
+    *rest_sum = 0;
+  }
+}
+
+__global__ void __launch_bounds__(TableSmem::NT, 2)
+    k_tile_table(uint64_t* __restrict__ keys, uint32_t* __restrict__ counts, const TileDesc* __restrict__ tiles,
+                 uint32_t ntiles, TileOut<uint64_t>* __restrict__ tout, unsigned long long* fallbacks,
+                 TileRanges<uint64_t> rg, TileRetry retry) {
+  using L = TableSmem;
+  constexpr int NT = L::NT, NW = L::NW;
+  constexpr unsigned long long kFree = ~0ull;
+  extern __shared__ __align__(16) uint8_t sm[];
+  unsigned long long* tab = reinterpret_cast<unsigned long long*>(sm + L::o_tab);
+  uint16_t* ord = reinterpret_cast<uint16_t*>(sm + L::o_ord);
+  unsigned* edge = reinterpret_cast<unsigned*>(sm + L::o_edge);
+  // [0] probe limit, [2 + parity] rest, [4], [5] the next tile
+  unsigned* misc = reinterpret_cast<unsigned*>(sm + L::o_misc);
+  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  unsigned long long* queue = reinterpret_cast<unsigned long long*>(sm + L::o_queue) + wid * 64;
+  // the thread's next two keys, a pair of the tile's 16-byte aligned span
+  uint4 ka = make_uint4(0, 0, 0, 0);
+  auto fetch = [&](const TileIn<uint64_t>& t, uint32_t p) {
+    if (p < ((uint32_t)(t.start & 1u) + t.n + 1) >> 1) ka = reinterpret_cast<const uint4*>(keys + (t.start & ~1ull))[p];
+  };
+  if (threadIdx.x < 8) misc[threadIdx.x] = threadIdx.x == 6 && (blockIdx.x & 31u) && mostly_binned(retry);
+  __syncthreads();
+  bool skip = misc[6] || rg.wait_polls;  // a bound on the binning sort's wait (tests of its timeout): every tile goes there
+  TileIn<uint64_t> t = tile_in(tiles, blockIdx.x, ntiles, rg);
+  fetch(t, threadIdx.x);
+  uint32_t clustered = 0;  // tiles in a row that went to hashed homes
+  for (uint32_t i = blockIdx.x, par = 0; i < ntiles; par ^= 1) {
+    const uint32_t n = t.n;
+    if (threadIdx.x == 0) choose_next(retry, &misc[4]);
+    if (n == 0 || skip) {
+      if (threadIdx.x == 0) {
+        if (n == 0) empty_tile(&tout[i]);
+        else retry.add(i, n);
+      }
+      skip = rg.wait_polls;
+      __syncthreads();
+      i = misc[4];
+      list_others(retry, &misc[4], tiles, ntiles, tout);
+      t = tile_in(tiles, i, ntiles, rg);
+      fetch(t, threadIdx.x);
+      __syncthreads();
+      continue;
+    }
+    // Keys clustered in a small part of the range (an AT-rich genome) go to
+    // hashed homes and are binned afterwards.  After two such tiles in a row
+    // the CTA's next ones start there; every eighth tries the order again.
+    bool hashed = clustered >= 2 && (clustered & 7u);
+    unsigned* cnt = reinterpret_cast<unsigned*>(sm + (hashed ? L::o_hcnt : L::o_cnt));
+    // slots: twice the keys, in whole threads' shares
+    uint32_t slots = n < (uint32_t)L::SLOTS / 2 - 288 ? (2 * n + 64 + 511) & ~511u : (uint32_t)L::SLOTS;
+    auto clear = [&]() {
+      if (hashed && slots > (uint32_t)L::HSLOTS) slots = L::HSLOTS;
+      uint4* t4 = reinterpret_cast<uint4*>(tab);
+      for (uint32_t j = threadIdx.x; j < slots / 2; j += NT) t4[j] = make_uint4(~0u, ~0u, ~0u, ~0u);
+      uint4* c4 = reinterpret_cast<uint4*>(cnt);
+      for (uint32_t j = threadIdx.x; j < slots / 4; j += NT) c4[j] = make_uint4(0, 0, 0, 0);
+    };
+    clear();
+    __syncthreads();
+    const uint32_t ni = misc[4];
+    list_others(retry, &misc[4], tiles, ntiles, tout);
+    const TileIn<uint64_t> next = tile_in(tiles, ni, ntiles, rg);
+    // ---- the keys, counted.  A key whose home holds another one is queued;
+    // the warp probes on for 32 such keys at a time, so that the others do not
+    // wait for the few ----
+    auto count_keys = [&](auto home, uint32_t limit) {
+      bool far = false;
+      uint32_t nq = 0;
+      auto probe = [&](uint32_t m) {  // the last m queued keys
+        __syncwarp();
+        nq -= m;
+        if (lane < m) {
+          const unsigned long long v = queue[nq + lane];
+          uint32_t s = home(v);
+          const uint32_t end = s + limit;
+          for (;;) {
+            if (++s == end) {
+              far = true;
+              break;
+            }
+            const unsigned long long x = atomicCAS(&tab[s], kFree, v);
+            if (x == kFree || x == v) {
+              atomicAdd(&cnt[s], 1u);
+              break;
+            }
+          }
+        }
+        __syncwarp();
+      };
+      const uint32_t head = (uint32_t)(t.start & 1u);
+      for (uint32_t p = threadIdx.x; p - lane < (head + n + 1) >> 1; p += NT) {
+        const unsigned long long v[2] = {(unsigned long long)ka.y << 32 | ka.x, (unsigned long long)ka.w << 32 | ka.z};
+        fetch(t, p + NT);
+        const uint32_t i0 = 2 * p - head;
+        unsigned long long old[2];
+        uint32_t h[2];
+        bool in[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          in[q] = i0 + q < n;
+          h[q] = home(v[q]);
+          old[q] = in[q] ? atomicCAS(&tab[h[q]], kFree, v[q]) : kFree;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const bool hit = old[q] == kFree || old[q] == v[q];
+          if (hit && in[q]) atomicAdd(&cnt[h[q]], 1u);
+          const unsigned miss = __ballot_sync(0xffffffffu, !hit);
+          if (miss) {
+            if (!hit) queue[nq + __popc(miss & lt)] = v[q];
+            nq += __popc(miss);
+            if (nq >= 32) probe(32);
+          }
+        }
+        if (__any_sync(0xffffffffu, far || *(volatile unsigned*)&misc[0])) break;
+      }
+      if (nq) probe(nq);
+      if (far) misc[0] = 1;
+    };
+    const RangeMap<uint64_t> map(t.mn, t.mx);
+    if (!hashed) {
+      count_keys(HomeLinear<uint64_t>(map, t.mx, slots - 2 * kProbeLimit), kProbeLimit);  // probes end inside the table
+      __syncthreads();
+      hashed = misc[0] != 0;
+      if (hashed) {
+        __syncthreads();
+        if (threadIdx.x == 0) misc[0] = 0;
+        cnt = reinterpret_cast<unsigned*>(sm + L::o_hcnt);
+        clear();
+        fetch(t, threadIdx.x);
+        __syncthreads();
+      } else {
+        clustered = 0;
+      }
+    }
+    if (hashed) {
+      const uint32_t homes = slots - kHashProbes;
+      count_keys([homes](uint64_t v) { return __umulhi((uint32_t)((v * 0xD6E8FEB86659FD93ull) >> 32), homes); },
+                 kHashProbes);
+      __syncthreads();
+      ++clustered;
+    }
+    fetch(next, threadIdx.x);
+    if (misc[0]) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        retry.add(i, n);
+        retry.met_tile(true);
+        misc[0] = 0;
+      }
+      i = ni;
+      t = next;
+      continue;
+    }
+    // ---- the thread's 16 slots, listed; clusters in order ----
+    unsigned U;
+    {
+      // a slot is in use when its count is not zero
+      const uint32_t a = threadIdx.x * 16;
+      uint32_t mine = 0, before = 0, after = 0;
+      if (a < slots) {
+        const uint4* c4 = reinterpret_cast<const uint4*>(cnt + a);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 x = c4[j];
+          mine |= (x.x ? 1u << (4 * j) : 0u) | (x.y ? 2u << (4 * j) : 0u) | (x.z ? 4u << (4 * j) : 0u) |
+                  (x.w ? 8u << (4 * j) : 0u);
+        }
+        before = a && cnt[a - 1];
+        after = a + 16 < slots && cnt[a + 16];
+      }
+      // occupied slots, and clusters of at least two that start here
+      const uint32_t multi = hashed ? 0u : mine & ~((mine << 1) | before) & ((mine >> 1) | (after << 15));
+      const unsigned both = __popc(mine) | (__popc(multi) << 16);
+      const unsigned inc = warp_inclusive(both, lane), ex = inc - both;
+      const unsigned tot = __shfl_sync(0xffffffffu, inc, 31), nc = tot >> 16;
+      if (lane == 0) edge[wid] = tot & 0xffffu;
+      // the warp's clusters (first slots), one lane each
+      uint16_t* list = reinterpret_cast<uint16_t*>(queue);
+      unsigned p = ex >> 16;
+      for (uint32_t m = multi; m; m &= m - 1) list[p++] = (uint16_t)(a + __ffs(m) - 1);
+      __syncthreads();  // every warp has read the counts, and the totals are there
+      const unsigned wt = lane < (unsigned)NW ? edge[lane] : 0u;
+      const unsigned wi = warp_inclusive(wt, lane);
+      U = __shfl_sync(0xffffffffu, wi, NW - 1);
+      unsigned u = __shfl_sync(0xffffffffu, wi - wt, wid) + (ex & 0xffffu);
+      for (uint32_t m = mine; m; m &= m - 1) ord[u++] = (uint16_t)(a + __ffs(m) - 1);
+      for (unsigned j = lane; j < nc; j += 32) {
+        const uint32_t first = list[j];
+        unsigned long long last = tab[first];
+        for (uint32_t e = first + 1; e < slots; ++e) {
+          const unsigned long long v = tab[e];
+          if (v == kFree) break;
+          if (v > last) {
+            last = v;
+            continue;
+          }
+          const unsigned c = cnt[e];
+          uint32_t q = e;
+          do {
+            tab[q] = tab[q - 1];
+            cnt[q] = cnt[q - 1];
+            --q;
+          } while (q > first && tab[q - 1] > v);
+          tab[q] = v;
+          cnt[q] = c;
+        }
+      }
+    }
+    __syncthreads();
+    if (hashed) {
+      // the slots hold the distinct keys in no order: into bins by their place
+      // in the range, then ranked inside their bin by counting
+      unsigned* bins = reinterpret_cast<unsigned*>(sm + L::o_queue);
+      uint16_t* tmp = reinterpret_cast<uint16_t*>(sm + L::o_tmp);
+      const HomeLinear<uint64_t> place(map, t.mx, L::BINS);
+      for (uint32_t j = threadIdx.x; j < L::BINS / 2; j += NT) bins[j] = 0;
+      __syncthreads();
+      for (uint32_t j = threadIdx.x; j < U; j += NT) bin_add(bins, place(tab[ord[j]]));
+      __syncthreads();
+      {
+        static_assert(L::BINS / 2 == 4 * NT, "four words of bins per thread");
+        const uint4 x = reinterpret_cast<const uint4*>(bins)[threadIdx.x];
+        const unsigned w[4] = {x.x, x.y, x.z, x.w};
+        unsigned sum = 0;
+        bool full = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          full |= (w[j] & 0xffffu) > kMaxRanked || (w[j] >> 16) > kMaxRanked;
+          sum += (w[j] & 0xffffu) + (w[j] >> 16);
+        }
+        if (full) misc[0] = 1;
+        const unsigned inc = warp_inclusive(sum, lane);
+        if (lane == 31) edge[wid] = inc;
+        __syncthreads();
+        const unsigned wt = lane < (unsigned)NW ? edge[lane] : 0u;
+        const unsigned wi = warp_inclusive(wt, lane);
+        unsigned o = __shfl_sync(0xffffffffu, wi - wt, wid) + inc - sum;
+        unsigned y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          y[j] = o | ((o + (w[j] & 0xffffu)) << 16);
+          o += (w[j] & 0xffffu) + (w[j] >> 16);
+        }
+        reinterpret_cast<uint4*>(bins)[threadIdx.x] = make_uint4(y[0], y[1], y[2], y[3]);
+      }
+      __syncthreads();
+      if (misc[0]) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          retry.add(i, n);
+          retry.met_tile(true);
+          misc[0] = 0;
+        }
+        i = ni;
+        t = next;
+        continue;
+      }
+      for (uint32_t j = threadIdx.x; j < U; j += NT) {
+        const uint16_t s = ord[j];
+        tmp[bin_add(bins, place(tab[s]))] = s;
+      }
+      __syncthreads();
+      for (uint32_t j = threadIdx.x; j < U; j += NT) {
+        const uint16_t s = tmp[j];
+        const unsigned long long v = tab[s];
+        const uint32_t b = place(v);
+        const uint32_t a = b ? bin_get(bins, b - 1) : 0u, z = bin_get(bins, b);
+        uint32_t r = a;
+        if (z - a > 1)
+          for (uint32_t q = a; q < z; ++q) r += tab[tmp[q]] < v ? 1u : 0u;
+        ord[r] = s;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0 && fallbacks) atomicAdd(fallbacks, 1ull);
+    }
+    write_rows<NT>(
+        U, keys + t.start, counts + t.start, &misc[2 + par], &tout[i],
+        [&](unsigned u, uint64_t* key, uint32_t* c) {
+          const uint32_t s = ord[u];
+          *key = tab[s];
+          *c = cnt[s];
+        });
+    if (threadIdx.x == 0) {
+      retry.met_tile(hashed && 2 * U > n);  // mostly distinct keys: the binning sort is the faster one
+      if (n > tile_capacity<uint64_t>() && fallbacks) atomicAdd(&fallbacks[1], (unsigned long long)U);
+    }
+    i = ni;
+    t = next;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Tile sort of u128 keys (32 <= k <= 64).  Long k-mers come in clumps: the reads
+// that cover one place of the genome give a k-mer and its copies with an error,
+// and those with the error in the second half agree in their first 64 bits and
+// more, so no linear map of the range keeps them apart (a table with homes in
+// key order probed 7 slots per key on 250 bp reads at k = 63).  Here the keys
+// are counted in a table of hashed homes, where clumps do not matter, and only
+// the distinct ones (half of the keys there, a quarter at k = 31) are sorted:
+// binned by their place in the range, then ranked inside their bin by counting.
+// Measured on 1M x 250 bp reads of an AT-rich genome at k = 63 (188M keys):
+// 11.8 -> 3.5 ms; half of its tiles had needed LSD passes or many-key bins.
+// ---------------------------------------------------------------------------
+struct HashSmem {
+  static constexpr int NT = 512, NW = NT / 32, CAP = kTileThreads * tile_items<u128>(), SLOTS = 2 * CAP, BINS = CAP;
+  static constexpr size_t o_buf = 0;                              // the tile's keys
+  static constexpr size_t o_tab = o_buf + (size_t)CAP * 16;       // 6 bits of hash | index + 1 | count
+  static constexpr size_t o_bin = o_tab;                          // after the counting: bins, and the keys in bin order
+  static constexpr size_t o_ord = o_bin + (size_t)BINS * 4;
+  static constexpr size_t o_list = o_tab + (size_t)SLOTS * 4;     // the distinct keys: count << 16 | index
+  static constexpr size_t o_edge = o_list + (size_t)CAP * 4;
+  static constexpr size_t o_misc = o_edge + (size_t)NW * 4;
+  static constexpr size_t o_bar = o_misc + 32;
+  static constexpr size_t total = o_bar + 16;
+  static_assert(CAP <= 4096, "13-bit indices and counts");
+};
+
+__global__ void __launch_bounds__(HashSmem::NT, 2)
+    k_tile_hash(u128* __restrict__ keys, uint32_t* __restrict__ counts, const TileDesc* __restrict__ tiles,
+                uint32_t ntiles, TileOut<u128>* __restrict__ tout, unsigned long long* fallbacks,
+                TileRanges<u128> rg, TileRetry retry) {
+  using L = HashSmem;
+  constexpr int NT = L::NT, NW = L::NW;
+  extern __shared__ __align__(16) uint8_t sm[];
+  const u128* buf = reinterpret_cast<const u128*>(sm + L::o_buf);
+  unsigned* tab = reinterpret_cast<unsigned*>(sm + L::o_tab);
+  unsigned* bin = reinterpret_cast<unsigned*>(sm + L::o_bin);
+  unsigned* ord = reinterpret_cast<unsigned*>(sm + L::o_ord);
+  unsigned* list = reinterpret_cast<unsigned*>(sm + L::o_list);
+  unsigned* edge = reinterpret_cast<unsigned*>(sm + L::o_edge);
+  // [0] full bin, [1] copy timeout, [2 + parity] rest, [4], [5] the next tile
+  unsigned* misc = reinterpret_cast<unsigned*>(sm + L::o_misc);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::o_bar);
+  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t used = 0;  // completed uses of the tile buffer
+  auto taken = [&](const TileIn<u128>& t) { return t.n && t.n <= (uint32_t)L::CAP && !rg.wait_polls; };
+  auto load = [&](const TileIn<u128>& t) {
+    if (threadIdx.x == 0 && taken(t)) bulk_load(sm + L::o_buf, keys + t.start, t.n * 16, bar);
+  };
+  // exclusive prefix of v over the threads and the total; one barrier inside
+  auto scan = [&](unsigned v, unsigned* total) {
+    const unsigned inc = warp_inclusive(v, lane);
+    if (lane == 31) edge[wid] = inc;
+    __syncthreads();
+    const unsigned wt = lane < (unsigned)NW ? edge[lane] : 0u;
+    const unsigned wi = warp_inclusive(wt, lane);
+    *total = __shfl_sync(0xffffffffu, wi, NW - 1);
+    return __shfl_sync(0xffffffffu, wi - wt, wid) + inc - v;
+  };
+  if (threadIdx.x == 0) mbar_init(bar);
+  if (threadIdx.x < 8) misc[threadIdx.x] = threadIdx.x == 6 && (blockIdx.x & 31u) && mostly_binned(retry);
+  __syncthreads();
+  bool skip = misc[6];
+  TileIn<u128> t = tile_in(tiles, blockIdx.x, ntiles, rg);
+  if (!skip) load(t);
+  for (uint32_t i = blockIdx.x, par = 0; i < ntiles; par ^= 1) {
+    const uint32_t n = t.n;
+    if (threadIdx.x == 0) choose_next(retry, &misc[4]);
+    if (skip || !taken(t)) {
+      skip = false;
+      // larger tiles, and (a bound on the binning sort's wait: tests of its timeout) every tile
+      if (threadIdx.x == 0) {
+        if (n == 0) empty_tile(&tout[i]);
+        else retry.add(i, n);
+      }
+      __syncthreads();
+      i = misc[4];
+      list_others(retry, &misc[4], tiles, ntiles, tout);
+      t = tile_in(tiles, i, ntiles, rg);
+      load(t);
+      __syncthreads();
+      continue;
+    }
+    // a power of two of at least twice the keys
+    const uint32_t slots = n <= 128 ? 256u : 1u << (33 - __clz((int)(n - 1)));
+    for (uint32_t j = threadIdx.x; j < slots / 4; j += NT) reinterpret_cast<uint4*>(tab)[j] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const uint32_t ni = misc[4];
+    list_others(retry, &misc[4], tiles, ntiles, tout);
+    const TileIn<u128> next = tile_in(tiles, ni, ntiles, rg);
+    if (!mbar_wait(bar, used & 1u, kBulkWaitPolls)) {
+      misc[1] = 1;
+      mbar_wait(bar, used & 1u, kBulkDrainPolls);
+    }
+    ++used;
+    // ---- the keys, counted: the table has more slots than the tile keys, so
+    // every probe ends ----
+    for (uint32_t j = threadIdx.x; j < n; j += NT) {
+      const u128 v = buf[j];
+      const uint64_t m = ((uint64_t)v ^ (hi64(v) * 0x9E3779B97F4A7C15ull)) * 0xD6E8FEB86659FD93ull;
+      const uint32_t h = (uint32_t)(m >> 32);
+      const unsigned word = (h & 0xFC000000u) | ((j + 1) << 13) | 1u;
+      for (uint32_t s = h & (slots - 1);; s = (s + 1) & (slots - 1)) {
+        const unsigned x = atomicCAS(&tab[s], 0u, word);
+        if (x == 0) break;
+        if (((x ^ word) >> 26) == 0 && buf[((x >> 13) & 0x1fffu) - 1] == v) {
+          atomicAdd(&tab[s], 1u);
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    // ---- the distinct keys, listed ----
+    unsigned U;
+    {
+      unsigned c = 0;
+      for (uint32_t j = threadIdx.x; j < slots; j += NT) c += tab[j] != 0;
+      unsigned o = scan(c, &U);
+      for (uint32_t j = threadIdx.x; j < slots; j += NT) {
+        const unsigned x = tab[j];
+        if (x) list[o++] = ((x & 0x1fffu) << 16) | (((x >> 13) & 0x1fffu) - 1);
+      }
+    }
+    __syncthreads();
+    // ---- their bins ----
+    const uint32_t bins = U <= 1024 ? 2048u : (uint32_t)L::BINS;
+    const RangeMap<u128> map(t.mn, t.mx);
+    const HomeLinear<u128> bin_of_key(map, t.mx, bins);
+    for (uint32_t j = threadIdx.x; j < bins / 4; j += NT) reinterpret_cast<uint4*>(bin)[j] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < U; j += NT) atomicAdd(&bin[bin_of_key(buf[list[j] & 0xffffu])], 1u);
+    __syncthreads();
+    {
+      const uint32_t per = bins / NT;  // 4 or 8 consecutive bins per thread
+      unsigned v[8], sum = 0;
+      bool full = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = (uint32_t)j < per ? bin[threadIdx.x * per + j] : 0u;
+        full |= v[j] > kMaxRanked;
+        sum += v[j];
+      }
+      if (full) misc[0] = 1;
+      unsigned tot;
+      unsigned o = scan(sum, &tot);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if ((uint32_t)j < per) {
+          bin[threadIdx.x * per + j] = o;
+          o += v[j];
+        }
+    }
+    __syncthreads();
+    if (misc[0] || misc[1]) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (misc[1]) {
+          if (fallbacks) atomicAdd(fallbacks, kBulkTimeoutFlag);
+          empty_tile(&tout[i]);
+        } else {
+          retry.add(i, n);
+          retry.met_tile(true);
+        }
+        misc[0] = misc[1] = 0;
+      }
+      load(next);
+      i = ni;
+      t = next;
+      continue;
+    }
+    for (uint32_t j = threadIdx.x; j < U; j += NT) {
+      const unsigned e = list[j];
+      ord[atomicAdd(&bin[bin_of_key(buf[e & 0xffffu])], 1u)] = e;
+    }
+    __syncthreads();
+    // bin[b] is now the end of bin b; a key's place among its bin's by counting
+    for (uint32_t j = threadIdx.x; j < U; j += NT) {
+      const unsigned e = ord[j];
+      const u128 v = buf[e & 0xffffu];
+      const uint32_t b = bin_of_key(v);
+      const uint32_t a = b ? bin[b - 1] : 0u, z = bin[b];
+      uint32_t r = a;
+      if (z - a > 1)
+        for (uint32_t q = a; q < z; ++q) r += buf[ord[q] & 0xffffu] < v ? 1u : 0u;
+      list[r] = e;
+    }
+    __syncthreads();
+    write_rows<NT>(U, keys + t.start, counts + t.start, &misc[2 + par], &tout[i],
+                   [&](unsigned u, u128* key, uint32_t* c) {
+                     const unsigned e = list[u];
+                     *key = buf[e & 0xffffu];
+                     *c = e >> 16;
+                   });
+    // mostly distinct keys: the binning sort is the faster one
+    if (threadIdx.x == 0) retry.met_tile(n > kHashAny && 4 * U > 3 * n);
+    load(next);
+    i = ni;
+    t = next;
+  }
+}
+
 // One CTA per tile: tile blockIdx.x (+ the launch's first) or ids[blockIdx.x];
 // with a device count, CTAs walk ids[0 .. *nids) in turn.
 template <class T, int MULT>
@@ -601,8 +1309,25 @@ static void tile_sort_with(T* keys, uint32_t* counts, const TileDesc* tiles, con
 
 template <class T>
 void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t ntiles, TileOut<T>* out,
-                      unsigned long long* fallbacks, TileRanges<T> rg, cudaStream_t s) {
-  tile_sort_with<T, 1>(keys, counts, tiles, nullptr, nullptr, ntiles, out, fallbacks, rg, s);
+                      unsigned long long* fallbacks, TileRanges<T> rg, TileRetry retry, cudaStream_t s) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const uint32_t grid = std::min<uint32_t>(ntiles, 2 * (uint32_t)sms);
+  if (!ntiles) return;
+  auto go = [&](auto kern, size_t smem, int nt) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    kern<<<grid, nt, smem, s>>>(keys, counts, tiles, ntiles, out, fallbacks, rg, retry);
+  };
+  if constexpr (sizeof(T) == 8) go(k_tile_table, TableSmem::total, TableSmem::NT);
+  else go(k_tile_hash, HashSmem::total, HashSmem::NT);
+}
+template <class T>
+void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
+                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+                             TileRanges<T> rg, cudaStream_t s) {
+  tile_sort_with<T, 1>(keys, counts, tiles, ids, nids_dev, 2 * grid, out, fallbacks, rg, s);
 }
 template <class T>
 void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
@@ -611,9 +1336,15 @@ void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, co
   tile_sort_with<T, 2>(keys, counts, tiles, ids, nids_dev, nids, out, fallbacks, rg, s);
 }
 template void launch_tile_sort<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, uint32_t, TileOut<uint64_t>*,
-                                         unsigned long long*, TileRanges<uint64_t>, cudaStream_t);
+                                         unsigned long long*, TileRanges<uint64_t>, TileRetry, cudaStream_t);
 template void launch_tile_sort<u128>(u128*, uint32_t*, const TileDesc*, uint32_t, TileOut<u128>*, unsigned long long*,
-                                     TileRanges<u128>, cudaStream_t);
+                                     TileRanges<u128>, TileRetry, cudaStream_t);
+template void launch_tile_sort_listed<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
+                                                const unsigned*, TileOut<uint64_t>*, unsigned long long*,
+                                                TileRanges<uint64_t>, cudaStream_t);
+template void launch_tile_sort_listed<u128>(u128*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
+                                            const unsigned*, TileOut<u128>*, unsigned long long*, TileRanges<u128>,
+                                            cudaStream_t);
 template void launch_tile_sort_large<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
                                                const unsigned*, TileOut<uint64_t>*, unsigned long long*,
                                                TileRanges<uint64_t>, cudaStream_t);
@@ -827,37 +1558,42 @@ template void launch_big_tile_sort<u128>(u128*, uint32_t*, u128*, const TileDesc
                                          const unsigned*, TileOut<u128>*, DevStatus*, unsigned long long*,
                                          cudaStream_t);
 
-// Oversized tiles listed on the device, per bucket group: group g (buckets
-// gb[g] .. gb[g+1]) lists its tiles above the on-chip capacity (up to twice
-// it) from ids[gb[g] * S] on and those above twice it from ids2[gb[g] * S] on,
-// with the counts in cnt[2g] and cnt[2g + 1].  Also the tile statistics:
-// stats[0] largest tile, [1] keys, [2] non-empty tiles, [3] keys in the tiles
-// above capacity, range[t] keys in tile index t of every bucket.
-__global__ void k_tile_lists(const uint32_t* __restrict__ lens, uint32_t ntiles, uint32_t S,
-                             const uint32_t* __restrict__ gb, uint32_t NG, uint32_t cap, uint32_t* __restrict__ ids,
-                             uint32_t* __restrict__ ids2, unsigned* __restrict__ cnt,
-                             unsigned long long* __restrict__ stats, unsigned long long* __restrict__ range) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  const uint32_t len = lens[t];
-  if (len == 0) return;
-  const uint32_t b = t / S;
-  uint32_t g = 0;
-  while (g + 1 < NG && gb[g + 1] <= b) ++g;
-  if (len > 2 * cap) ids2[(size_t)gb[g] * S + atomicAdd(&cnt[2 * g + 1], 1u)] = t;
-  else if (len > cap) ids[(size_t)gb[g] * S + atomicAdd(&cnt[2 * g], 1u)] = t;
-  if (len > cap) atomicAdd(&stats[3], (unsigned long long)len);
-  atomicMax(&stats[0], (unsigned long long)len);
-  atomicAdd(&stats[1], (unsigned long long)len);
-  atomicAdd(&stats[2], 1ull);
-  atomicAdd(&range[t % S], (unsigned long long)len);
+// Statistics of the tiles: stats[0] largest tile, [1] keys, [2] non-empty
+// tiles, [3] keys in the tiles above `cap`, [4] those tiles, range[t] keys in
+// tile index t of every bucket.  One atomic per statistic and CTA.
+__global__ void __launch_bounds__(256) k_tile_stats(const uint32_t* __restrict__ lens, uint32_t ntiles, uint32_t S,
+                                                    uint32_t cap, unsigned long long* __restrict__ stats,
+                                                    unsigned long long* __restrict__ range) {
+  __shared__ unsigned long long red[8][5];
+  const uint32_t t = blockIdx.x * 256 + threadIdx.x;
+  const uint32_t len = t < ntiles ? lens[t] : 0u;
+  if (len && S > 1) atomicAdd(&range[t % S], (unsigned long long)len);
+  unsigned long long v[5] = {len, len, len ? 1ull : 0ull, len > cap ? (unsigned long long)len : 0ull,
+                             len > cap ? 1ull : 0ull};
+#pragma unroll
+  for (int j = 0; j < 5; ++j)
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const unsigned long long y = __shfl_xor_sync(0xffffffffu, v[j], o);
+      v[j] = j == 0 ? (y > v[j] ? y : v[j]) : v[j] + y;
+    }
+  if ((threadIdx.x & 31) == 0)
+    for (int j = 0; j < 5; ++j) red[threadIdx.x >> 5][j] = v[j];
+  __syncthreads();
+  if (threadIdx.x < 5) {
+    unsigned long long x = red[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) {
+      const unsigned long long y = red[w][threadIdx.x];
+      x = threadIdx.x == 0 ? (y > x ? y : x) : x + y;
+    }
+    if (threadIdx.x == 0) atomicMax(&stats[0], x);
+    else if (x) atomicAdd(&stats[threadIdx.x], x);
+  }
 }
 
-void launch_tile_lists(const uint32_t* lens, uint32_t ntiles, uint32_t S, const uint32_t* gb, uint32_t NG,
-                       uint32_t cap, uint32_t* ids, uint32_t* ids2, unsigned* cnt, unsigned long long* stats,
+void launch_tile_stats(const uint32_t* lens, uint32_t ntiles, uint32_t S, uint32_t cap, unsigned long long* stats,
                        unsigned long long* range, cudaStream_t s) {
-  if (ntiles)
-    k_tile_lists<<<(ntiles + 255) / 256, 256, 0, s>>>(lens, ntiles, S, gb, NG, cap, ids, ids2, cnt, stats, range);
+  if (ntiles) k_tile_stats<<<(ntiles + 255) / 256, 256, 0, s>>>(lens, ntiles, S, cap, stats, range);
 }
 
 }  // namespace kite
