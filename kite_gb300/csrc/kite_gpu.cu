@@ -524,15 +524,17 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
 
   // ---- K3b tile split -----------------------------------------------------
   // Tiles per bucket: the largest bucket's keys over the target tile load
-  // (cfg.tile_fill of the on-chip capacity), rounded up to a multiple of 32
-  // for one split level (up to 1024 tiles); beyond that a power of two, so
-  // that the two levels divide it evenly.
+  // (cfg.tile_fill of the on-chip capacity), for one split level (up to 1024
+  // tiles) as it is; beyond that a power of two, so that the two levels divide
+  // it evenly.  (A tile's fixed cost is that of about 1,500 keys: 16 samples of
+  // 50,000 reads in 6 tiles per bucket instead of 32 sort in 1.03 ms instead of
+  // 2.28.)
   const double fill = std::min(4.0, std::max(0.05, ctx->cfg.tile_fill));
   uint32_t S = 1;
   if ((double)maxb > fill * CAP) {
     const double want = std::ceil((double)maxb / (fill * CAP));
     if (want <= 1024.0) {
-      S = std::min<uint32_t>(1024, ((uint32_t)want + 31) & ~31u);
+      S = (uint32_t)want;
     } else {
       S = 2048;
       while ((double)S < want && S < 4096) S <<= 1;
@@ -736,7 +738,12 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   const T kmax = 2 * k >= (uint32_t)KeyTraits<T>::kBits ? ~T(0) : ((T(1) << (2 * k)) - T(1));
   // Bucket groups: each group's tiles are sorted, linked and encoded in turn,
   // so one group's payload copies to the host while the next one sorts.
-  const uint32_t NG = std::min<uint32_t>(kSortGroups, PT);
+  // Results that stay on the device take one group (nothing overlaps there,
+  // and every group costs its launches and a last wave of tiles: one group
+  // instead of eight took 1M reads at k = 31 from 4.41 to 4.19 ms); copies to the host
+  // take one per 8M keys, up to eight.
+  const uint32_t NG =
+      std::min<uint32_t>({kSortGroups, PT, to_host ? (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(N >> 23, 8)) : 1u});
   std::vector<uint32_t> gb(NG + 1);  // first bucket of each group
   for (uint32_t g = 0; g <= NG; ++g) gb[g] = (uint32_t)((uint64_t)PT * g / NG);
   if (NG == 8 && PT >= 64) {
