@@ -118,8 +118,6 @@ struct MergeTile {
   uint32_t partition;
 };
 
-__device__ __forceinline__ bool is_term(uint8_t b) { return (b & 0x80u) == 0; }
-
 // Warp shuffle-up of a 64- or 128-bit value, a wrapping inclusive warp sum,
 // and a broadcast from one lane.
 template <class T>
@@ -152,167 +150,85 @@ __device__ __forceinline__ T warp_bcast_t(T v, int src) {
     return ((T)hi << 64) | (T)lo;
   }
 }
-template <class T>
-__device__ __forceinline__ T warp_sum_t(T v) {
-  return warp_bcast_t(warp_incl_sum(v), 31);
-}
-
 // ---- warp-cooperative DVLE decode ----------------------------------------------
 // A segment (kSeg bytes of one stream's varint area) is decoded by one warp in
 // rounds of 512 bytes: every lane loads 16 bytes (one coalesced 512-byte load
 // per warp) into a per-warp shared-memory window that also holds the 32 bytes
-// before the round, marks the terminator bytes (top bit clear) and decodes
-// the varints whose terminator lies in its own 16 bytes, reading back to the
-// previous terminator in the window (a varint is at most 19 bytes).  A varint
-// belongs to the segment holding its terminator; the stream's bytes before
-// its varint area (the raw head row) bound the first varint.  A final varint
-// without a terminator at the stream's end belongs to the last segment.
+// before the round, and lists where the varints that end in its bytes end (top
+// bit clear).  A varint is at most 19 bytes, so the one that a round's first
+// byte lies in begins in the window.  Then each lane takes a whole row: the
+// 32 rows' key deltas (8-byte loads from the window, their 7-bit groups packed
+// by shifts of whole words) go through one warp scan, and keys and counts out
+// as coalesced runs.  Key deltas and counts alternate, so which terminators end
+// a row follows from the number of varints before the segment.  A row belongs
+// to the segment holding its count's terminator; a final varint without one at
+// the stream's end counts as ending there.
+//
+// Passes: varints per segment (k_seg_count), their scan per stream, rows with
+// keys relative to the segment's start (k_seg_rows), the scan of the segments'
+// delta sums, and the start keys added (k_seg_base).  Decoding every varint
+// byte by byte in the lane that held its last byte, twice (sums first, then
+// rows), took 37 warp instructions per row; this takes 15, and the 64.6M rows of 2M
+// reads decode in 1.36 ms instead of 3.63.
 constexpr int kDecWarps = 8;                    // warps per decode CTA
 constexpr uint32_t kRound = 512;                // bytes per warp round
 constexpr uint32_t kWinBytes = kRound + 32;     // window: 32 bytes before the round + the round
 
-struct DecWindow {
-  uint8_t b[kWinBytes];
+struct alignas(16) DecWindow {
+  uint8_t b[kWinBytes + 32];   // and room for whole-word reads past the last varint
+  uint16_t end[kRound + 4];    // [0], [1]: ends before the round; then its own varints' (window offset past the last byte)
 };
+static_assert(sizeof(DecWindow) % 16 == 0, "every window is read by 16-byte loads");
 
 // Terminator bits of 16 bytes (bit i: byte i has its top bit clear).
 __device__ __forceinline__ uint32_t term_bits16(uint4 w) {
-  auto m4 = [](uint32_t x) {
-    const uint32_t t = ~x & 0x80808080u;
-    return ((t >> 7) & 1u) | ((t >> 14) & 2u) | ((t >> 21) & 4u) | ((t >> 28) & 8u);
-  };
+  auto m4 = [](uint32_t x) { return (((~x & 0x80808080u) >> 7) * 0x10204080u) >> 28; };
   return m4(w.x) | (m4(w.y) << 4) | (m4(w.z) << 8) | (m4(w.w) << 12);
 }
 
-// Loads the round at `base` (16-byte aligned) into the window: bytes
-// [base - 32, base + 512); blocks at or beyond lim_pad (the padded end of
-// the byte buffer) and before byte 0 read as zero.
-__device__ __forceinline__ void load_round(const uint8_t* __restrict__ bytes, uint64_t base, uint64_t lim_pad,
-                                           DecWindow* win, uint32_t lane) {
-  uint4* wv = reinterpret_cast<uint4*>(win->b);
-  const uint64_t o = base + 16ull * lane;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (o < lim_pad) v = *reinterpret_cast<const uint4*>(bytes + o);
-  wv[2 + lane] = v;
-  if (lane < 2) {
-    uint4 p = make_uint4(0, 0, 0, 0);
-    if (base >= 32) p = *reinterpret_cast<const uint4*>(bytes + base - 32 + 16 * lane);
-    wv[lane] = p;
-  }
-  __syncwarp();
+// The terminators of the 16 bytes at stream offset o that lie in [lo, hi),
+// with one at the byte `forced` (the last of a stream that ends inside a varint).
+__device__ __forceinline__ uint32_t own_terms(uint4 w, uint64_t o, uint64_t lo, uint64_t hi, uint64_t forced) {
+  uint32_t m = term_bits16(w);
+  if (forced - o < 16) m |= 1u << (uint32_t)(forced - o);
+  if (o < lo) m &= lo - o >= 16 ? 0u : ~((1u << (uint32_t)(lo - o)) - 1u);
+  if (o + 16 > hi) m &= hi <= o ? 0u : ((1u << (uint32_t)(hi - o)) - 1u);
+  return m;
 }
 
-// The value of the varint ending at window byte t (32 <= t < 48) of the
-// lane's 48-byte view: bytes from one past the previous boundary bit of
-// `bound` below t up to t.
-template <class T>
-__device__ __forceinline__ T varint_at(const DecWindow* win, uint64_t bound, uint32_t lane_off, int t) {
-  const uint64_t below = bound & ((1ull << t) - 1ull);
-  const int start = below ? 64 - __clzll(below) : 0;
-  T val = 0;
-  unsigned sh = 0;
-  for (int j = start; j <= t; ++j) {
-    const uint8_t b = win->b[lane_off + j];
-    if (sh < (unsigned)KeyTraits<T>::kBits) val |= (T)(b & 0x7f) << sh;
-    sh += 7;
-  }
-  return val;
-}
-
-// Per lane and round: `bound` marks over the lane's 48-byte view (window
-// bytes [16 lane, 16 lane + 48) = stream bytes base - 32 + 16 lane + i) the
-// terminators and every byte before the varint area (so the first varint
-// starts at the area); `own` marks the terminators of the lane's own 16 bytes
-// (view bits 32..47) inside [seg_lo, seg_hi).
-__device__ __forceinline__ void round_masks(const DecWindow* win, uint32_t lane, uint64_t base, uint64_t area,
-                                            uint64_t seg_lo, uint64_t seg_hi, uint64_t& bound, uint32_t& own) {
-  const uint4* wv = reinterpret_cast<const uint4*>(win->b);
-  const uint64_t t0 = term_bits16(wv[lane]), t1 = term_bits16(wv[lane + 1]), t2 = term_bits16(wv[lane + 2]);
-  bound = t0 | (t1 << 16) | (t2 << 32);
-  const uint64_t ob = base + 16ull * lane;  // stream byte of view bit 32
-  const int64_t nb = (int64_t)(32 + area) - (int64_t)ob;  // view bits below the varint area
-  if (nb > 0) bound |= nb >= 48 ? 0xFFFFFFFFFFFFull : ((1ull << nb) - 1ull);
-  const int64_t lo = (int64_t)seg_lo - (int64_t)ob, hi = (int64_t)seg_hi - (int64_t)ob;
-  uint32_t keep = 0xFFFFu;
-  if (lo > 0) keep &= lo >= 16 ? 0u : ~((1u << lo) - 1u);
-  if (hi < 16) keep &= hi <= 0 ? 0u : ((1u << hi) - 1u);
-  own = (uint32_t)t2 & keep;
-}
-
-// Pass A, one warp per segment: the varints the segment owns, and the
-// wrapping sums of those at even / odd positions within the segment (which
-// of the two are key deltas follows from the parity of the segment's first
-// varint index, known after the per-stream scan).
-template <class T>
+// Pass A, one warp per segment: the varints the segment owns.
 __global__ void __launch_bounds__(32 * kDecWarps)
-    k_seg_pass_a(const uint8_t* __restrict__ bytes, uint64_t lim_pad, const SegDesc* __restrict__ segs,
-                 uint32_t nseg, const StreamDesc* __restrict__ streams, uint32_t* __restrict__ terms,
-                 T* __restrict__ sum_even, T* __restrict__ sum_odd) {
-  __shared__ __align__(16) DecWindow wins[kDecWarps];
-  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t si = blockIdx.x * kDecWarps + wid;
+    k_seg_count(const uint8_t* __restrict__ bytes, uint64_t lim_pad, const SegDesc* __restrict__ segs, uint32_t nseg,
+                const StreamDesc* __restrict__ streams, uint32_t* __restrict__ terms) {
+  const uint32_t lane = threadIdx.x & 31, si = blockIdx.x * kDecWarps + (threadIdx.x >> 5);
   if (si >= nseg) return;
-  DecWindow* win = &wins[wid];
   const SegDesc d = segs[si];
   const StreamDesc sd = streams[d.stream];
-  const uint64_t area = sd.byte_off + sd.head, lim = sd.byte_off + sd.byte_len;
-  uint32_t n = 0;  // varints owned so far (the same in every lane)
-  T se = 0, so = 0;
-  for (uint64_t base = d.start & ~15ull; base < d.end; base += kRound) {
-    load_round(bytes, base, lim_pad, win, lane);
-    uint64_t bound;
-    uint32_t own;
-    round_masks(win, lane, base, area, d.start, d.end, bound, own);
-    const uint32_t c = __popc(own);
-    uint32_t incl = c;
+  const uint64_t lim = sd.byte_off + sd.byte_len;
+  uint32_t n = 0;
+  constexpr int kAhead = 4;
+  for (uint64_t o0 = (d.start & ~15ull) + 16 * lane; o0 - 16 * lane < d.end; o0 += kAhead * kRound) {
+    uint4 w[kAhead];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
+    for (int j = 0; j < kAhead; ++j) {
+      const uint64_t o = o0 + (uint64_t)j * kRound;
+      w[j] = o < lim_pad && o < d.end ? *reinterpret_cast<const uint4*>(bytes + o) : make_uint4(~0u, ~0u, ~0u, ~0u);
     }
-    uint32_t idx = n + incl - c;
-    for (uint32_t m = own; m; m &= m - 1, ++idx) {
-      const T v = varint_at<T>(win, bound, 16 * lane, 32 + __ffs(m) - 1);
-      if (idx & 1u) so += v;
-      else se += v;
-    }
-    n += __shfl_sync(0xffffffffu, incl, 31);
-    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) n += __popc(own_terms(w[j], o0 + (uint64_t)j * kRound, d.start, d.end, lim - 1));
   }
-  // a final varint without its terminator (the stream ends inside it)
-  if (d.end == lim && lim > area && lane == 0 && !is_term(bytes[lim - 1])) {
-    uint64_t p = lim;
-    while (p > area && !is_term(bytes[p - 1])) --p;
-    T val = 0;
-    unsigned sh = 0;
-    for (uint64_t q = p; q < lim; ++q) {
-      if (sh < (unsigned)KeyTraits<T>::kBits) val |= (T)(bytes[q] & 0x7f) << sh;
-      sh += 7;
-    }
-    if (n & 1u) so += val;
-    else se += val;
-    ++n;
-  }
-  n = __shfl_sync(0xffffffffu, n, 0);
-  se = warp_sum_t(se);
-  so = warp_sum_t(so);
-  if (lane == 0) {
-    terms[si] = n;
-    sum_even[si] = se;
-    sum_odd[si] = so;
-  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) terms[si] = n;
 }
 
-// Per stream of the list sids (one warp each): first varint index and start
-// key of every segment [seg_first, seg_end) of the stream (exclusive scans of
-// the terminator counts and of the delta sums), and the check that the stream
-// holds the 2 * (rows - 1) varints its rows need.
-template <class T>
-__global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const T* __restrict__ sum_even,
-                                  const T* __restrict__ sum_odd, const uint32_t* __restrict__ seg_first,
+// Per stream of the list sids (one warp each): the first varint index of every
+// segment [seg_first, seg_end) of the stream (exclusive scan of the terminator
+// counts), and the check that the stream holds the 2 * (rows - 1) varints its
+// rows need.
+__global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const uint32_t* __restrict__ seg_first,
                                   const uint32_t* __restrict__ seg_end, const StreamDesc* __restrict__ streams,
-                                  const T* __restrict__ first_keys, const uint32_t* __restrict__ sids, uint32_t nsid,
-                                  unsigned long long* __restrict__ vstart, T* __restrict__ kstart, DevStatus* st) {
+                                  const uint32_t* __restrict__ sids, uint32_t nsid,
+                                  unsigned long long* __restrict__ vstart, DevStatus* st) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   if (w >= nsid) return;
@@ -320,35 +236,84 @@ __global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const T* _
   const StreamDesc sd = streams[si];
   const uint32_t f = seg_first[si], e = seg_end[si];
   unsigned long long cv = 0;
-  T ck = f < e ? first_keys[si] : T(0);
   for (uint32_t b = f; b < e; b += 32) {
     const uint32_t s = b + lane;
     const unsigned long long t = s < e ? terms[s] : 0ull;
     const unsigned long long ti = warp_incl_sum<unsigned long long>(t);
-    const unsigned long long v = cv + ti - t;
-    T dv = 0;
-    if (s < e) dv = (v & 1ull) ? sum_odd[s] : sum_even[s];
-    const T di = warp_incl_sum(dv);
-    if (s < e) {
-      vstart[s] = v;
-      kstart[s] = ck + (di - dv);
-    }
+    if (s < e) vstart[s] = cv + ti - t;
     cv += __shfl_sync(0xffffffffu, ti, 31);
-    ck += warp_bcast_t(di, 31);
   }
   if (lane == 0 && sd.head && sd.rows && cv < 2 * (sd.rows - 1)) dev_fail(st, KITE_DEV_SHORT_VARINTS, si);
 }
 
-// Pass B, one warp per segment: (key, u64 count) rows of the varints the
-// segment owns.  Varint index v (within the stream's varint area): even =
-// key delta of row v/2+1, odd = count of row (v-1)/2+1.  Keys are the running
-// wrapping sum of the deltas (as the reference's wrapping_add), from the
-// segment's start key: each round a warp scan of the lanes' delta sums.
+// Per stream of the list sids (one warp each): the key before every segment's
+// first row, from the stream's head key and the segments' delta sums.
+template <class T>
+__global__ void k_stream_base_scan(const T* __restrict__ sums, const uint32_t* __restrict__ seg_first,
+                                   const uint32_t* __restrict__ seg_end, const T* __restrict__ first_keys,
+                                   const uint32_t* __restrict__ sids, uint32_t nsid, T* __restrict__ kstart) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t w = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (w >= nsid) return;
+  const uint32_t si = sids[w], f = seg_first[si], e = seg_end[si];
+  T ck = f < e ? first_keys[si] : T(0);
+  for (uint32_t b = f; b < e; b += 32) {
+    const uint32_t s = b + lane;
+    const T dv = s < e ? sums[s] : T(0);
+    const T di = warp_incl_sum(dv);
+    if (s < e) kstart[s] = ck + (di - dv);
+    ck += warp_bcast_t(di, 31);
+  }
+}
+
+// The 7-bit groups of eight varint bytes (continuation bits cleared), packed.
+__device__ __forceinline__ uint64_t pack7(uint32_t lo, uint32_t hi) {
+  auto p4 = [](uint32_t v) {
+    v &= 0x7f7f7f7fu;
+    v = (v & 0x007f007fu) | ((v & 0x7f007f00u) >> 1);
+    return (v & 0x3fffu) | ((v & 0x3fff0000u) >> 2);
+  };
+  return (uint64_t)p4(lo) | ((uint64_t)p4(hi) << 28);
+}
+
+// The varint of window bytes [a, e): its low kBits bits.
+template <class T>
+__device__ __forceinline__ T varint_in(const DecWindow* win, uint32_t a, uint32_t e) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(win->b) + (a >> 2);
+  const uint32_t sh = (a & 3u) * 8;
+  const uint32_t n = e - a;
+  T v = 0;
+  uint32_t x0 = w[0], x1 = w[1];
+#pragma unroll
+  for (uint32_t g = 0; g < (sizeof(T) == 8 ? 2u : 3u); ++g) {
+    if (8 * g >= n) break;
+    const uint32_t x2 = w[2 * g + 2];
+    uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+    const uint32_t left = n - 8 * g;
+    if (left < 4) {
+      lo &= (1u << (8 * left)) - 1u;
+      hi = 0;
+    } else if (left < 8) {
+      hi &= (1u << (8 * (left - 4))) - 1u;
+    }
+    const uint64_t p = pack7(lo, hi);
+    if constexpr (sizeof(T) == 8) v |= g == 0 ? p : p << 56;
+    else v |= (T)p << (56 * g);
+    if (left <= 8) break;
+    x0 = x2;
+    x1 = w[2 * g + 3];
+  }
+  return v;
+}
+
+// Pass B, one warp per segment: (key, u64 count) rows of the segment, keys
+// relative to the segment's start (wrapping sums of the deltas, as the
+// reference's wrapping_add), and the segment's delta sum.
 template <class T>
 __global__ void __launch_bounds__(32 * kDecWarps)
-    k_seg_rows(const uint8_t* __restrict__ bytes, uint64_t lim_pad, const SegDesc* __restrict__ segs,
-               uint32_t nseg, const StreamDesc* __restrict__ streams, const unsigned long long* __restrict__ vstart,
-               const T* __restrict__ kstart, T* __restrict__ keys, unsigned long long* __restrict__ counts) {
+    k_seg_rows(const uint8_t* __restrict__ bytes, uint64_t lim_pad, const SegDesc* __restrict__ segs, uint32_t nseg,
+               const StreamDesc* __restrict__ streams, const unsigned long long* __restrict__ vstart,
+               T* __restrict__ keys, unsigned long long* __restrict__ counts, T* __restrict__ sums) {
   __shared__ __align__(16) DecWindow wins[kDecWarps];
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t si = blockIdx.x * kDecWarps + wid;
@@ -356,78 +321,111 @@ __global__ void __launch_bounds__(32 * kDecWarps)
   DecWindow* win = &wins[wid];
   const SegDesc d = segs[si];
   const StreamDesc sd = streams[d.stream];
-  const uint64_t area = sd.byte_off + sd.head, lim = sd.byte_off + sd.byte_len;
-  const unsigned long long nvar = sd.rows ? 2ull * (sd.rows - 1) : 0ull;
+  const uint64_t area = sd.byte_off + sd.head, forced = sd.byte_off + sd.byte_len - 1;
   unsigned long long v0 = vstart[si];  // stream varint index of the segment's next owned varint
-  T key = kstart[si];                  // key before that varint
-  for (uint64_t base = d.start & ~15ull; base < d.end; base += kRound) {
-    load_round(bytes, base, lim_pad, win, lane);
-    uint64_t bound;
-    uint32_t own;
-    round_masks(win, lane, base, area, d.start, d.end, bound, own);
+  uint64_t base = d.start & ~15ull;
+  // the 32 bytes before the round, and the ends of the two varints before the
+  // segment's first own byte (the area's start is the first varint's)
+  uint4 w = make_uint4(0, 0, 0, 0);
+  if (lane < 2 && base >= 32) w = *reinterpret_cast<const uint4*>(bytes + base - 32 + 16 * lane);
+  if (lane < 2) reinterpret_cast<uint4*>(win->b)[lane] = w;
+  {
+    uint64_t m = 0;  // window offset i: a varint ends at i (past its last byte)
+    if (base >= 32) {
+      const uint32_t t0 = __shfl_sync(0xffffffffu, own_terms(w, base - 32 + 16 * lane, area, d.start, forced), 0);
+      const uint32_t t1 = __shfl_sync(0xffffffffu, own_terms(w, base - 32 + 16 * lane, area, d.start, forced), 1);
+      m = (uint64_t)(t0 | (t1 << 16)) << 1;
+    }
+    // the bytes of the first round before the segment (its start rounded down)
+    const uint32_t pre = (uint32_t)(d.start - base);
+    uint32_t t2 = 0;
+    if (pre) t2 = own_terms(*reinterpret_cast<const uint4*>(bytes + base), base, area, d.start, forced);
+    m |= (uint64_t)t2 << 33;
+    const int64_t at = (int64_t)(area + 32) - (int64_t)base;  // the area's window offset
+    if (at >= 0 && at <= 48) m |= 1ull << at;
+    const int e1 = m ? 63 - __clzll((long long)m) : 0;
+    m &= ~(1ull << e1);
+    const int e0 = m ? 63 - __clzll((long long)m) : 0;
+    if (lane == 0) {
+      win->end[0] = (uint16_t)e0;
+      win->end[1] = (uint16_t)e1;
+    }
+  }
+  T run = 0;  // the deltas of the segment's rows so far
+  for (; base < d.end; base += kRound) {
+    const uint64_t o = base + 16ull * lane;
+    w = make_uint4(0, 0, 0, 0);
+    if (o < lim_pad) w = *reinterpret_cast<const uint4*>(bytes + o);
+    reinterpret_cast<uint4*>(win->b)[2 + lane] = w;
+    uint32_t own = own_terms(w, o, d.start, d.end, forced);
     const uint32_t c = __popc(own);
     uint32_t incl = c;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
+    for (int q = 1; q < 32; q <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, q);
+      if (lane >= (uint32_t)q) incl += y;
     }
-    const unsigned long long vl = v0 + incl - c;  // index of the lane's first owned varint
-    // the lane's key deltas (kept: a lane owns at most 16 varints, so at most
-    // 8 deltas, the j-th owned varint's delta in slot j / 2 whichever parity
-    // the lane starts on), then the key before each lane's first (warp scan)
-    T dsum = 0;
-    T dv[8];
-    {
-      uint32_t m = own;
-      unsigned long long v = vl;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (m) {
-          const int t = __ffs(m) - 1;
-          m &= m - 1;
-          if ((v & 1ull) == 0 && v < nvar) {
-            dv[j >> 1] = varint_at<T>(win, bound, 16 * lane, 32 + t);
-            dsum += dv[j >> 1];
-          }
-          ++v;
-        }
+    for (uint32_t at = 2 + incl - c; own; own &= own - 1, ++at) win->end[at] = (uint16_t)(32 + 16 * lane + __ffs(own));
+    const uint32_t n = __shfl_sync(0xffffffffu, incl, 31);
+    __syncwarp();
+    // row j of the round: its count is own varint i = i0 + 2 j, its key the one before
+    const uint32_t i0 = (v0 & 1ull) ? 0u : 1u;
+    const uint32_t nr = n > i0 ? (n - i0 + 1) / 2 : 0u;
+    const unsigned long long row0 = (v0 + i0 + 1) / 2;
+    for (uint32_t j0 = 0; j0 < nr; j0 += 32) {
+      const uint32_t j = j0 + lane, i = i0 + 2 * j;
+      const bool in = j < nr && row0 + j < sd.rows;  // bytes after the last row are ignored, as the reference decodes row_count rows
+      T delta = 0;
+      unsigned long long cnt = 0;
+      if (in) {
+        const uint32_t a = win->end[i], b = win->end[i + 1], e = win->end[i + 2];
+        delta = varint_in<T>(win, a, b);
+        cnt = e - b == 1 ? (unsigned long long)(win->b[b] & 0x7fu) : (unsigned long long)(uint64_t)varint_in<T>(win, b, e);
       }
-    }
-    const T dincl = warp_incl_sum(dsum);
-    T k = key + (dincl - dsum);
-    {
-      uint32_t m = own;
-      unsigned long long v = vl;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (m == 0 || v >= nvar) break;  // bytes after the last row are ignored, as the reference decodes row_count rows
-        const int t = __ffs(m) - 1;
-        m &= m - 1;
-        if ((v & 1ull) == 0) {
-          k += dv[j >> 1];
-          keys[sd.row_off + v / 2 + 1] = k;
-        } else {
-          counts[sd.row_off + (v - 1) / 2 + 1] = (unsigned long long)(uint64_t)varint_at<T>(win, bound, 16 * lane, 32 + t);
-        }
-        ++v;
+      const T sum = warp_incl_sum(delta);
+      if (in) {
+        keys[sd.row_off + row0 + j] = run + sum;
+        counts[sd.row_off + row0 + j] = cnt;
       }
+      run += warp_bcast_t(sum, 31);
     }
-    key += warp_bcast_t(dincl, 31);
-    v0 += __shfl_sync(0xffffffffu, incl, 31);
+    v0 += n;
+    // for the next round: the last 32 bytes and the last two ends
+    __syncwarp();
+    const uint16_t e0 = win->end[n], e1 = win->end[n + 1];
+    const uint4 tail = reinterpret_cast<const uint4*>(win->b)[lane < 2 ? 32 + lane : 32];
+    __syncwarp();
+    if (lane < 2) {
+      reinterpret_cast<uint4*>(win->b)[lane] = tail;
+      const uint16_t x = lane ? e1 : e0;
+      win->end[lane] = x > kRound ? (uint16_t)(x - kRound) : (uint16_t)0;
+    }
     __syncwarp();
   }
-  if (d.end == lim && lim > area && lane == 0 && !is_term(bytes[lim - 1]) && v0 < nvar) {
-    uint64_t p = lim;
-    while (p > area && !is_term(bytes[p - 1])) --p;
-    T val = 0;
-    unsigned sh = 0;
-    for (uint64_t q = p; q < lim; ++q) {
-      if (sh < (unsigned)KeyTraits<T>::kBits) val |= (T)(bytes[q] & 0x7f) << sh;
-      sh += 7;
-    }
-    if ((v0 & 1ull) == 0) keys[sd.row_off + v0 / 2 + 1] = key + val;
-    else counts[sd.row_off + (v0 - 1) / 2 + 1] = (unsigned long long)(uint64_t)val;
+  if (lane == 0) sums[si] = run;
+}
+
+// The segments' start keys added to their rows, one warp per segment.
+template <class T>
+__global__ void __launch_bounds__(32 * kDecWarps)
+    k_seg_base(const SegDesc* __restrict__ segs, uint32_t nseg, const StreamDesc* __restrict__ streams,
+               const uint32_t* __restrict__ terms, const unsigned long long* __restrict__ vstart,
+               const T* __restrict__ kstart, T* __restrict__ keys) {
+  const uint32_t lane = threadIdx.x & 31, si = blockIdx.x * kDecWarps + (threadIdx.x >> 5);
+  if (si >= nseg) return;
+  const StreamDesc sd = streams[segs[si].stream];
+  const unsigned long long v = vstart[si], a = (v >> 1) + 1;
+  const unsigned long long e = min((v + terms[si]) / 2 + 1, (unsigned long long)sd.rows);
+  const T k = kstart[si];
+  T* r = keys + sd.row_off;
+  constexpr int kAhead = 4;
+  for (unsigned long long i0 = a + lane; i0 < e; i0 += 32 * kAhead) {
+    T x[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) x[j] = i0 + 32 * j < e ? r[i0 + 32 * j] : T(0);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      if (i0 + 32 * j < e) r[i0 + 32 * j] = x[j] + k;
   }
 }
 
@@ -1023,7 +1021,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   stat->h2d_bytes += total_bytes;
   MergePool* pool = ex ? ex->pool : nullptr;
   Dev d_bytes(pool, 0), d_streams(pool, 1), d_segs(pool, 2), d_terms(pool, 3), d_vstart(pool, 4), d_dsum(pool, 5),
-      d_dsum2(pool, 6), d_sfirst(pool, 7), d_send(pool, 8), d_sids(pool, 9), d_kstart(pool, 10), d_keys(pool, 11),
+      d_sfirst(pool, 7), d_send(pool, 8), d_sids(pool, 9), d_kstart(pool, 10), d_keys(pool, 11),
       d_counts(pool, 12), d_first(pool, 13), d_raw(pool, 14);
   if (!d_bytes.ensure(total_bytes + 64)) return fail(KITE_ERR_OOM, "device bytes");
   // ---- decode segments, grouped by input: each input's bytes come in on a
@@ -1060,7 +1058,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   const uint32_t nseg = (uint32_t)segs.size(), nst = (uint32_t)streams.size(), nsid = (uint32_t)sids.size();
   if (!d_streams.ensure(nst * sizeof(StreamDesc) + 8) || !d_segs.ensure(nseg * sizeof(SegDesc) + 8) ||
       !d_terms.ensure(nseg * 4 + 8) || !d_vstart.ensure(nseg * 8 + 8) || !d_dsum.ensure(nseg * sizeof(T) + 16) ||
-      !d_dsum2.ensure(nseg * sizeof(T) + 16) || !d_kstart.ensure(nseg * sizeof(T) + 16) ||
+      !d_kstart.ensure(nseg * sizeof(T) + 16) ||
       !d_keys.ensure(total_rows * sizeof(T) + 16) || !d_counts.ensure(total_rows * 8 + 16) ||
       !d_first.ensure(nst * sizeof(T) + 16) || !d_raw.ensure(raw_ids.size() * 4 + 8) ||
       !d_sfirst.ensure(nst * 4 + 8) || !d_send.ensure(nst * 4 + 8) || !d_sids.ensure(nsid * 4 + 8))
@@ -1117,22 +1115,27 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       launches++;
     }
     if (ns) {
-      // DVLE varints: pass A (per-segment counts and parity sums), the
-      // per-stream scans, pass B (rows); no host round trip
+      // DVLE varints: counts per segment and their scan, relative rows, the
+      // scan of the delta sums, start keys; no host round trip
       const unsigned gsegs = (ns + kDecWarps - 1) / kDecWarps;
-      k_seg_pass_a<T><<<gsegs, 32 * kDecWarps, 0, s>>>(d_bytes.as<uint8_t>(), lim_pad, d_segs.as<SegDesc>() + s0, ns,
-                                                       d_streams.as<StreamDesc>(), d_terms.as<uint32_t>() + s0,
-                                                       d_dsum.as<T>() + s0, d_dsum2.as<T>() + s0);
-      k_stream_seg_scan<T><<<(nq + 7) / 8, 256, 0, s>>>(d_terms.as<uint32_t>(), d_dsum.as<T>(), d_dsum2.as<T>(),
-                                                        d_sfirst.as<uint32_t>(), d_send.as<uint32_t>(),
-                                                        d_streams.as<StreamDesc>(), d_first.as<T>(),
-                                                        d_sids.as<uint32_t>() + q0, nq,
-                                                        d_vstart.as<unsigned long long>(), d_kstart.as<T>(), dst);
+      k_seg_count<<<gsegs, 32 * kDecWarps, 0, s>>>(d_bytes.as<uint8_t>(), lim_pad, d_segs.as<SegDesc>() + s0, ns,
+                                                   d_streams.as<StreamDesc>(), d_terms.as<uint32_t>() + s0);
+      k_stream_seg_scan<<<(nq + 7) / 8, 256, 0, s>>>(d_terms.as<uint32_t>(), d_sfirst.as<uint32_t>(),
+                                                     d_send.as<uint32_t>(), d_streams.as<StreamDesc>(),
+                                                     d_sids.as<uint32_t>() + q0, nq,
+                                                     d_vstart.as<unsigned long long>(), dst);
       k_seg_rows<T><<<gsegs, 32 * kDecWarps, 0, s>>>(d_bytes.as<uint8_t>(), lim_pad, d_segs.as<SegDesc>() + s0, ns,
                                                      d_streams.as<StreamDesc>(), d_vstart.as<unsigned long long>() + s0,
-                                                     d_kstart.as<T>() + s0, d_keys.as<T>(),
-                                                     d_counts.as<unsigned long long>());
-      launches += 3;
+                                                     d_keys.as<T>(), d_counts.as<unsigned long long>(),
+                                                     d_dsum.as<T>() + s0);
+      k_stream_base_scan<T><<<(nq + 7) / 8, 256, 0, s>>>(d_dsum.as<T>(), d_sfirst.as<uint32_t>(), d_send.as<uint32_t>(),
+                                                         d_first.as<T>(), d_sids.as<uint32_t>() + q0, nq,
+                                                         d_kstart.as<T>());
+      k_seg_base<T><<<gsegs, 32 * kDecWarps, 0, s>>>(d_segs.as<SegDesc>() + s0, ns, d_streams.as<StreamDesc>(),
+                                                     d_terms.as<uint32_t>() + s0,
+                                                     d_vstart.as<unsigned long long>() + s0, d_kstart.as<T>() + s0,
+                                                     d_keys.as<T>());
+      launches += 5;
     }
     MCU(cudaEventRecord(cl.tev[3 + 2 * i], s));
   }
