@@ -25,15 +25,17 @@ struct MergePoolSlot {
   size_t cap = 0;
 };
 struct MergePool {
-  static constexpr int kSlots = 32;
+  static constexpr int kSlots = 34;
   MergePoolSlot slot[kSlots];
-  MergePoolSlot host;  // pinned host memory: the tile stream lists on their way to the device
+  MergePoolSlot host;     // pinned host memory: the tile stream lists on their way to the device
+  MergePoolSlot records;  // pinned host memory: a merge's partition records
   MergePool() = default;
   MergePool(const MergePool&) = delete;
   MergePool& operator=(const MergePool&) = delete;
   ~MergePool() {
     for (auto& s : slot) cudaFree(s.p);
     if (host.p) cudaFreeHost(host.p);
+    if (records.p) cudaFreeHost(records.p);
   }
 };
 
@@ -46,7 +48,7 @@ struct MergeExtra {
   size_t nq = 0;
   uint64_t* counts_out = nullptr;     // query: u64 sum per key, 0 when absent
   MlpModel* mlp = nullptr;            // learned CDF for the tile cut (null: sampled histogram only)
-  int splitter_mode = 0;              // KITE_SPLIT_*: AUTO keeps whichever predicts the lower imbalance
+  int splitter_mode = 0;              // KITE_SPLIT_LEARNED: cut by the learned CDF; else by the histogram
   MergePool* pool = nullptr;          // the context's buffers (null: allocated and freed by the call)
 };
 

@@ -62,7 +62,7 @@ enum MergeMode : int {
   kModeMerge = 0,  // kite merge: per-input filter, u64 sums, u32 overflow recorded
   kModeDump = 1,   // kite dump: sum clamped to u32, then the header filter; TSV byte counts
   kModeHisto = 2,  // kite histo: per-input filter on the u64 sum, then count -> frequency
-  kModeRows = 3,   // kite query: every key with its u64 sum, no filter
+  kModeQuery = 3,  // kite query: keys looked up in the decoded streams, no merge kernel
 };
 
 // Outputs of the histo and query modes.
@@ -71,7 +71,6 @@ struct MergeAux {
   unsigned long long* spill;     // counts >= kHistBins, one entry per key (histo)
   unsigned long long* spill_n;   // entries written to spill
   unsigned long long spill_cap;
-  unsigned long long* counts64;  // u64 sum of every output row (query)
   uint32_t line_k;               // k, for TSV line lengths (dump)
 };
 
@@ -222,19 +221,19 @@ __global__ void __launch_bounds__(32 * kDecWarps)
 }
 
 // Per stream of the list sids (one warp each): the first varint index of every
-// segment [seg_first, seg_end) of the stream (exclusive scan of the terminator
+// segment [first[w], first[w + 1]) of stream sids[w] (exclusive scan of the terminator
 // counts), and the check that the stream holds the 2 * (rows - 1) varints its
 // rows need.
-__global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const uint32_t* __restrict__ seg_first,
-                                  const uint32_t* __restrict__ seg_end, const StreamDesc* __restrict__ streams,
-                                  const uint32_t* __restrict__ sids, uint32_t nsid,
+__global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const uint32_t* __restrict__ first,
+                                  const StreamDesc* __restrict__ streams, const uint32_t* __restrict__ sids,
+                                  uint32_t nsid,
                                   unsigned long long* __restrict__ vstart, DevStatus* st) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   if (w >= nsid) return;
   const uint32_t si = sids[w];
   const StreamDesc sd = streams[si];
-  const uint32_t f = seg_first[si], e = seg_end[si];
+  const uint32_t f = first[w], e = first[w + 1];
   unsigned long long cv = 0;
   for (uint32_t b = f; b < e; b += 32) {
     const uint32_t s = b + lane;
@@ -249,13 +248,13 @@ __global__ void k_stream_seg_scan(const uint32_t* __restrict__ terms, const uint
 // Per stream of the list sids (one warp each): the key before every segment's
 // first row, from the stream's head key and the segments' delta sums.
 template <class T>
-__global__ void k_stream_base_scan(const T* __restrict__ sums, const uint32_t* __restrict__ seg_first,
-                                   const uint32_t* __restrict__ seg_end, const T* __restrict__ first_keys,
-                                   const uint32_t* __restrict__ sids, uint32_t nsid, T* __restrict__ kstart) {
+__global__ void k_stream_base_scan(const T* __restrict__ sums, const uint32_t* __restrict__ first,
+                                   const T* __restrict__ first_keys, const uint32_t* __restrict__ sids,
+                                   uint32_t nsid, T* __restrict__ kstart) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   if (w >= nsid) return;
-  const uint32_t si = sids[w], f = seg_first[si], e = seg_end[si];
+  const uint32_t si = sids[w], f = first[w], e = first[w + 1];
   T ck = f < e ? first_keys[si] : T(0);
   for (uint32_t b = f; b < e; b += 32) {
     const uint32_t s = b + lane;
@@ -485,6 +484,114 @@ __global__ void k_lower_bound(const T* __restrict__ keys, const uint64_t* __rest
   out[i] = lo;
 }
 
+// Segment descriptors: segment i belongs to the stream sids[q] with
+// first[q] <= i < first[q + 1].
+__global__ void k_make_segs(const StreamDesc* __restrict__ streams, const uint32_t* __restrict__ sids,
+                            const uint32_t* __restrict__ first, uint32_t nsid, uint32_t nseg,
+                            SegDesc* __restrict__ segs) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nseg) return;
+  uint32_t lo = 0, hi = nsid;
+  while (hi - lo > 1) {
+    const uint32_t m = (lo + hi) >> 1;
+    if (first[m] <= i) lo = m;
+    else hi = m;
+  }
+  const StreamDesc sd = streams[sids[lo]];
+  SegDesc d;
+  d.start = sd.byte_off + sd.head + (uint64_t)(i - first[lo]) * kSeg;
+  d.end = min(d.start + kSeg, sd.byte_off + sd.byte_len);
+  d.stream = sids[lo];
+  d.first = i == first[lo];
+  segs[i] = d;
+}
+
+// The sum over the partition's streams of a key's counts (u64, saturating:
+// load_partition_counts src/kiteops/mod.rs:433-473), 0 when absent, for
+// `kite query`: one lower bound per stream, no merge.
+template <class T>
+__global__ void k_query_streams(const T* __restrict__ keys, const unsigned long long* __restrict__ counts,
+                                const StreamDesc* __restrict__ streams, const uint32_t* __restrict__ part_first,
+                                const T* __restrict__ qk, const uint32_t* __restrict__ qp, uint32_t nq,
+                                unsigned long long* __restrict__ out) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nq) return;
+  const T key = qk[q];
+  const uint32_t p = qp[q];
+  unsigned long long c = 0;
+  for (uint32_t si = part_first[p]; si < part_first[p + 1]; ++si) {
+    uint64_t lo = streams[si].row_off, hi = lo + streams[si].rows;
+    const uint64_t end = hi;
+    while (lo < hi) {
+      const uint64_t mid = lo + (hi - lo) / 2;
+      if (keys[mid] < key) lo = mid + 1;
+      else hi = mid;
+    }
+    for (; lo < end && keys[lo] == key; ++lo) c = c > ~0ull - counts[lo] ? ~0ull : c + counts[lo];
+  }
+  out[q] = c;
+}
+
+// Row positions that cut a stream, the only one of its partition, every
+// kMergeCap rows (between two different keys), S ranges: laid out as those of
+// k_range_positions.
+template <class T>
+__global__ void k_slice_positions(const T* __restrict__ keys, const StreamDesc* __restrict__ streams, uint32_t nst,
+                                  uint32_t S, uint64_t* __restrict__ pos) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (uint64_t)nst * (S + 1)) return;
+  const StreamDesc sd = streams[i / (S + 1)];
+  const uint64_t end = sd.row_off + sd.rows;
+  uint64_t r = sd.row_off + min((uint64_t)(i % (S + 1)) * kMergeCap, sd.rows);
+  if (i % (S + 1) == S) r = end;
+  while (r > sd.row_off && r < end && keys[r] == keys[r - 1]) ++r;
+  pos[i] = r;
+}
+
+// The tiles of a cut into S ranges per partition, tile p * S + j for range j
+// of partition p, with every stream of the partition in order (some of them
+// empty in the range).  info[0]: tiles above the on-chip capacity, [1] the
+// largest tile, [2] tiles with rows.
+__global__ void k_plan_tiles(const uint64_t* __restrict__ pos, const StreamDesc* __restrict__ streams,
+                             const uint32_t* __restrict__ part_first, uint32_t P, uint32_t S,
+                             MergeTile* __restrict__ tiles, TileStream* __restrict__ ts, TileDesc* __restrict__ tds,
+                             unsigned* __restrict__ info) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= P * S) return;
+  const uint32_t p = t / S, j = t % S, f = part_first[p], n = part_first[p + 1] - f;
+  MergeTile mt;
+  mt.first_ts = f * S + j * n;
+  mt.nts = n;
+  mt.partition = p;
+  uint64_t rows = 0, before = 0;
+  for (uint32_t k = 0; k < n; ++k) {
+    const uint64_t* q = pos + (size_t)(f + k) * (S + 1) + j;
+    const uint64_t lo = q[0], hi = q[1];
+    TileStream x;
+    x.lo = lo;
+    x.hi = hi;
+    x.input = streams[f + k].input;
+    x.pad = 0;
+    ts[mt.first_ts + k] = x;
+    rows += hi - lo;
+    before += lo - streams[f + k].row_off;
+  }
+  // a partition's rows follow those of the partitions before it
+  mt.out_off = (n ? streams[f].row_off : 0) + before;
+  mt.rows_in = rows > kMergeCap ? 0u : (uint32_t)rows;
+  tiles[t] = mt;
+  TileDesc td;
+  td.start = mt.out_off;
+  td.len = 0;
+  td.bucket = p;
+  tds[t] = td;
+  if (rows > kMergeCap) atomicAdd(&info[0], 1u);
+  if (rows) {
+    atomicMax(&info[1], (unsigned)min(rows, (uint64_t)0xffffffffu));
+    atomicAdd(&info[2], 1u);
+  }
+}
+
 // Row position of every splitter in every stream: pos[s * (S + 1) + j] is
 // lower_bound(spl[j - 1]) in stream s's rows for 1 <= j < S, the stream's
 // first row for j = 0 and its end for j = S.
@@ -536,8 +643,7 @@ struct MergeSmem {
 // rest_bytes of a tile = its TSV bytes, lines of k + 2 + digits).
 // kModeHisto: `kite histo` of one input (load_partition_counts' u64 sum,
 // apply_reader_filter_to_rows on it, then the count's frequency; no rows
-// written).  kModeRows: `kite query` (every key with its u64 sum in
-// aux.counts64, no filter).
+// written).
 template <class T, int MODE>
 __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
     const T* __restrict__ keys, const unsigned long long* __restrict__ counts, const MergeTile* __restrict__ tiles,
@@ -724,8 +830,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
           if (cur_in != 0xffffffffu) {
             const InputFilter f = filt[cur_in];
             const unsigned long long eff = DUMP && part > 0xffffffffull ? 0xffffffffull : part;
-            const bool ok = MODE == kModeRows ||
-                            (!(f.has_min && eff < f.min_count) && !(f.has_max && eff > f.max_count));
+            const bool ok = !(f.has_min && eff < f.min_count) && !(f.has_max && eff > f.max_count);
             if (ok) {
               total = (total > ~0ull - part) ? ~0ull : total + part;
               present = true;
@@ -774,7 +879,6 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
         const uint32_t c32 = total > 0xffffffffull ? 0xffffffffu : (uint32_t)total;
         out_keys[mt.out_off + o] = gkey[i];
         out_counts[mt.out_off + o] = c32;
-        if (MODE == kModeRows) aux.counts64[mt.out_off + o] = total;
         if (o == 0) misc[60] = c32;
       }
       outk[o] = gkey[i];
@@ -880,44 +984,43 @@ __global__ void __launch_bounds__(kTsvThreads) k_tsv_tiles(const T* __restrict__
   }
 }
 
-// kite query lookups: key q of partition qp[q] in the merged rows of that
-// partition's non-empty tiles (tile_first / tile_key0 / tile_off / tile_rows,
-// first keys ascending within a partition); its u64 sum, 0 when absent.
-template <class T>
-__global__ void k_query_rows(const T* __restrict__ keys, const unsigned long long* __restrict__ counts64,
-                             const uint32_t* __restrict__ tile_first, const T* __restrict__ tile_key0,
-                             const unsigned long long* __restrict__ tile_off, const uint32_t* __restrict__ tile_rows,
-                             const T* __restrict__ qk, const uint32_t* __restrict__ qp, uint32_t nq,
-                             unsigned long long* __restrict__ out) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nq) return;
-  const T key = qk[q];
-  const uint32_t p = qp[q];
-  uint32_t lo = tile_first[p], hi = tile_first[p + 1];
-  // last tile whose first key is <= key
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (tile_key0[mid] <= key) lo = mid + 1;
-    else hi = mid;
-  }
-  unsigned long long c = 0;
-  if (lo > tile_first[p]) {
-    const uint32_t t = lo - 1;
-    unsigned long long a = tile_off[t], b = a + tile_rows[t];
-    while (a < b) {
-      const unsigned long long mid = a + (b - a) / 2;
-      if (keys[mid] < key) a = mid + 1;
-      else b = mid;
-    }
-    if (a < tile_off[t] + tile_rows[t] && keys[a] == key) c = counts64[a];
-  }
-  out[q] = c;
-}
-
-template <class T>
-struct Key128 {
-  static unsigned __int128 to(T v) { return (unsigned __int128)v; }
+// Dump: a partition's lines, bytes and key range from its tiles' records, one
+// warp per partition; tile byte counts for the scan of their offsets.
+struct PartLines {
+  unsigned long long rows, bytes, kmin_lo, kmin_hi, kmax_lo, kmax_hi;
 };
+template <class T>
+__global__ void k_part_lines(const TileOut<T>* __restrict__ tout, const uint32_t* __restrict__ tile_first, uint32_t P,
+                             unsigned long long* __restrict__ tile_bytes, PartLines* __restrict__ out) {
+  const uint32_t lane = threadIdx.x & 31, p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (p >= P) return;
+  PartLines x{};
+  bool have = false;
+  T kmin = T(0), kmax = T(0);
+  for (uint32_t t0 = tile_first[p]; t0 < tile_first[p + 1]; t0 += 32) {
+    const uint32_t t = t0 + lane;
+    TileOut<T> o{};
+    if (t < tile_first[p + 1]) {
+      o = tout[t];
+      tile_bytes[t] = o.rest_bytes;
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, o.rows > 0);
+    if (!any) continue;
+    x.rows += __reduce_add_sync(0xffffffffu, o.rows);
+    x.bytes += warp_bcast_t(warp_incl_sum((unsigned long long)o.rest_bytes), 31);
+    const T lo = warp_bcast_t(o.first_key, __ffs(any) - 1);
+    kmax = warp_bcast_t(o.last_key, 31 - __clz(any));
+    if (!have) kmin = lo;
+    have = true;
+  }
+  if (lane == 0) {
+    x.kmin_lo = (unsigned long long)kmin;
+    x.kmin_hi = hi64(kmin);
+    x.kmax_lo = (unsigned long long)kmax;
+    x.kmax_hi = hi64(kmax);
+    out[p] = x;
+  }
+}
 
 // ---- host side -----------------------------------------------------------------
 // A device buffer of the call: its own allocation, or a slot of the
@@ -1021,63 +1124,86 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   stat->h2d_bytes += total_bytes;
   MergePool* pool = ex ? ex->pool : nullptr;
   Dev d_bytes(pool, 0), d_streams(pool, 1), d_segs(pool, 2), d_terms(pool, 3), d_vstart(pool, 4), d_dsum(pool, 5),
-      d_sfirst(pool, 7), d_send(pool, 8), d_sids(pool, 9), d_kstart(pool, 10), d_keys(pool, 11),
+      d_qseg(pool, 6), d_pfirst(pool, 7), d_status(pool, 8), d_sids(pool, 9), d_kstart(pool, 10), d_keys(pool, 11),
       d_counts(pool, 12), d_first(pool, 13), d_raw(pool, 14);
   if (!d_bytes.ensure(total_bytes + 64)) return fail(KITE_ERR_OOM, "device bytes");
-  // ---- decode segments, grouped by input: each input's bytes come in on a
-  // side stream and its segments are decoded as soon as they have landed, so
-  // the copies of the later inputs overlap the decode of the earlier ones ----
-  std::vector<SegDesc> segs;
-  std::vector<uint32_t> raw_ids;
-  std::vector<uint32_t> seg_first(streams.size(), 0), seg_end(streams.size(), 0);
-  std::vector<uint32_t> sids;                                   // DVLE streams with rows, input by input
-  std::vector<uint32_t> in_seg(n + 1, 0), in_sid(n + 1, 0);     // per input: its segment and stream-id ranges
+  // ---- pieces: runs of an input's streams in file order, of about a
+  // sixteenth of all bytes (8 MiB at least).  Each piece's bytes come in on a
+  // side stream and its streams are decoded as soon as they have landed, so
+  // the copies of later pieces overlap the decode of earlier ones ----
+  struct Piece {
+    uint64_t lo, hi;        // device byte range copied for it
+    int input;
+    uint32_t q0, q1;        // its streams in sids
+  };
+  std::vector<Piece> pieces;
+  std::vector<uint32_t> raw_ids, sids, qseg;  // RAW streams; DVLE streams with rows; each one's first segment
+  uint64_t nseg64 = 0;
   {
     std::vector<std::vector<uint32_t>> by_input(n);
     for (uint32_t si = 0; si < streams.size(); ++si) by_input[streams[si].input].push_back(si);
+    const uint64_t target = std::max<uint64_t>(8ull << 20, total_bytes / 16);
     for (int i = 0; i < n; ++i) {
-      in_seg[i] = (uint32_t)segs.size();
-      in_sid[i] = (uint32_t)sids.size();
-      for (uint32_t si : by_input[i]) {
-        const StreamDesc& sd = streams[si];
-        seg_first[si] = seg_end[si] = (uint32_t)segs.size();
-        if (sd.rows == 0) continue;
-        if (sd.head == 0) {
-          raw_ids.push_back(si);
-          continue;
+      auto& v = by_input[i];
+      std::sort(v.begin(), v.end(),
+                [&](uint32_t x, uint32_t y) { return streams[x].byte_off < streams[y].byte_off; });
+      const uint64_t in_end = in_base[i] + (in_span[i].second - in_span[i].first);
+      uint64_t at = in_base[i], reach = at;
+      uint32_t q0 = (uint32_t)sids.size();
+      for (size_t j = 0; j < v.size(); ++j) {
+        const StreamDesc& sd = streams[v[j]];
+        if (sd.byte_off > reach + (1u << 20)) {
+          // a query's partitions lie apart: what lies between is not copied
+          if (reach > at) pieces.push_back(Piece{at, reach, i, q0, (uint32_t)sids.size()});
+          at = reach = sd.byte_off;
+          q0 = (uint32_t)sids.size();
         }
-        sids.push_back(si);
-        const uint64_t a = sd.byte_off + sd.head, e = sd.byte_off + sd.byte_len;
-        for (uint64_t o = a; o < e; o += kSeg) segs.push_back(SegDesc{o, std::min(o + kSeg, e), si, o == a ? 1u : 0u});
-        seg_end[si] = (uint32_t)segs.size();
+        if (sd.rows && sd.head) {
+          sids.push_back(v[j]);
+          qseg.push_back((uint32_t)nseg64);
+          nseg64 += (sd.byte_len - sd.head + kSeg - 1) / kSeg;
+        } else if (sd.rows) {
+          raw_ids.push_back(v[j]);
+        }
+        reach = std::max(reach, sd.byte_off + sd.byte_len);
+        if (reach - at >= target && j + 1 < v.size()) {
+          pieces.push_back(Piece{at, reach, i, q0, (uint32_t)sids.size()});
+          at = reach;
+          q0 = (uint32_t)sids.size();
+        }
       }
+      pieces.push_back(Piece{at, mode == kModeQuery ? reach : in_end, i, q0, (uint32_t)sids.size()});
     }
-    in_seg[n] = (uint32_t)segs.size();
-    in_sid[n] = (uint32_t)sids.size();
+    qseg.push_back((uint32_t)nseg64);
   }
-  const uint32_t nseg = (uint32_t)segs.size(), nst = (uint32_t)streams.size(), nsid = (uint32_t)sids.size();
+  const uint32_t nseg = (uint32_t)nseg64, nst = (uint32_t)streams.size(), nsid = (uint32_t)sids.size();
+  std::vector<uint32_t> part_first_stream(P + 1, 0);
+  uint32_t most_streams = 0;   // of a partition
+  uint64_t most_rows = 0;
+  {
+    uint32_t si = 0;
+    for (uint32_t p = 0; p < P; ++p) {
+      part_first_stream[p] = si;
+      uint64_t rows = 0;
+      while (si < nst && streams[si].partition == p) rows += streams[si++].rows;
+      most_streams = std::max(most_streams, si - part_first_stream[p]);
+      most_rows = std::max(most_rows, rows);
+    }
+    part_first_stream[P] = nst;
+  }
   if (!d_streams.ensure(nst * sizeof(StreamDesc) + 8) || !d_segs.ensure(nseg * sizeof(SegDesc) + 8) ||
       !d_terms.ensure(nseg * 4 + 8) || !d_vstart.ensure(nseg * 8 + 8) || !d_dsum.ensure(nseg * sizeof(T) + 16) ||
-      !d_kstart.ensure(nseg * sizeof(T) + 16) ||
-      !d_keys.ensure(total_rows * sizeof(T) + 16) || !d_counts.ensure(total_rows * 8 + 16) ||
-      !d_first.ensure(nst * sizeof(T) + 16) || !d_raw.ensure(raw_ids.size() * 4 + 8) ||
-      !d_sfirst.ensure(nst * 4 + 8) || !d_send.ensure(nst * 4 + 8) || !d_sids.ensure(nsid * 4 + 8))
+      !d_kstart.ensure(nseg * sizeof(T) + 16) || !d_keys.ensure(total_rows * sizeof(T) + 16) ||
+      !d_counts.ensure(total_rows * 8 + 16) || !d_first.ensure(nst * sizeof(T) + 16) ||
+      !d_raw.ensure(raw_ids.size() * 4 + 8) || !d_qseg.ensure(qseg.size() * 4 + 8) ||
+      !d_pfirst.ensure((P + 1) * 4) || !d_sids.ensure(nsid * 4 + 8) || !d_status.ensure(2 * sizeof(DevStatus) + 64))
     return fail(KITE_ERR_OOM, "merge decode buffers");
-  MCU(cudaMemcpyAsync(d_streams.p, streams.data(), nst * sizeof(StreamDesc), cudaMemcpyHostToDevice, s));
-  if (nseg) MCU(cudaMemcpyAsync(d_segs.p, segs.data(), nseg * sizeof(SegDesc), cudaMemcpyHostToDevice, s));
-  if (nst) {
-    MCU(cudaMemcpyAsync(d_sfirst.p, seg_first.data(), nst * 4, cudaMemcpyHostToDevice, s));
-    MCU(cudaMemcpyAsync(d_send.p, seg_end.data(), nst * 4, cudaMemcpyHostToDevice, s));
-  }
-  if (nsid) MCU(cudaMemcpyAsync(d_sids.p, sids.data(), nsid * 4, cudaMemcpyHostToDevice, s));
-  if (!raw_ids.empty())
-    MCU(cudaMemcpyAsync(d_raw.p, raw_ids.data(), raw_ids.size() * 4, cudaMemcpyHostToDevice, s));
-  int launches = 0;
-  DevStatus* dst = nullptr;
-  MCU(cudaMallocAsync(&dst, sizeof(DevStatus), s));
-  MCU(cudaMemsetAsync(dst, 0, sizeof(DevStatus), s));
-  // copy lane: the side stream, one landing event per input, timing events
-  // around the copies ([0], [1]) and around each input's decode ([2 + 2i],
+  DevStatus* dst = d_status.as<DevStatus>();
+  DevStatus* est = dst + 1;                                           // of the encode
+  unsigned* plan_info = reinterpret_cast<unsigned*>(est + 1);         // of the tile plan
+  MCU(cudaMemsetAsync(d_status.p, 0, 2 * sizeof(DevStatus) + 64, s));
+  // copy lane: the side stream, one landing event per piece, timing events
+  // around the copies ([0], [1]) and around each piece's decode ([2 + 2i],
   // [3 + 2i]: recorded after the wait, so they time the kernels only)
   struct CopyLane {
     cudaStream_t cs = nullptr;
@@ -1088,49 +1214,64 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       if (cs) cudaStreamDestroy(cs);
     }
   } cl;
+  const size_t np = pieces.size();
   MCU(cudaStreamCreateWithFlags(&cl.cs, cudaStreamNonBlocking));
-  cl.ev.resize(n, nullptr);
-  for (int i = 0; i < n; ++i) MCU(cudaEventCreateWithFlags(&cl.ev[i], cudaEventDisableTiming));
-  cl.tev.resize(2 + 2 * (size_t)n, nullptr);
+  cl.ev.resize(np, nullptr);
+  for (auto& e : cl.ev) MCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cl.tev.resize(2 + 2 * np, nullptr);
   for (auto& e : cl.tev) MCU(cudaEventCreate(&e));
   MCU(cudaEventRecord(sev[0], s));
   MCU(cudaEventRecord(cl.tev[0], cl.cs));
-  for (int i = 0; i < n; ++i) {
-    if (in_span[i].second > in_span[i].first)
-      MCU(cudaMemcpyAsync(d_bytes.as<uint8_t>() + in_base[i], in[i].base + in_span[i].first,
-                          in_span[i].second - in_span[i].first, cudaMemcpyHostToDevice, cl.cs));
+  for (size_t i = 0; i < np; ++i) {
+    const Piece& pc = pieces[i];
+    if (pc.hi > pc.lo)
+      MCU(cudaMemcpyAsync(d_bytes.as<uint8_t>() + pc.lo,
+                          in[pc.input].base + in_span[pc.input].first + (pc.lo - in_base[pc.input]), pc.hi - pc.lo,
+                          cudaMemcpyHostToDevice, cl.cs));
     MCU(cudaEventRecord(cl.ev[i], cl.cs));
   }
   MCU(cudaEventRecord(cl.tev[1], cl.cs));
+  MCU(cudaMemcpyAsync(d_pfirst.p, part_first_stream.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
+  if (nst) MCU(cudaMemcpyAsync(d_streams.p, streams.data(), nst * sizeof(StreamDesc), cudaMemcpyHostToDevice, s));
+  if (nsid) {
+    MCU(cudaMemcpyAsync(d_sids.p, sids.data(), nsid * 4, cudaMemcpyHostToDevice, s));
+    MCU(cudaMemcpyAsync(d_qseg.p, qseg.data(), qseg.size() * 4, cudaMemcpyHostToDevice, s));
+  }
+  if (!raw_ids.empty())
+    MCU(cudaMemcpyAsync(d_raw.p, raw_ids.data(), raw_ids.size() * 4, cudaMemcpyHostToDevice, s));
+  int launches = 0;
+  if (nseg) {
+    k_make_segs<<<(nseg + 255) / 256, 256, 0, s>>>(d_streams.as<StreamDesc>(), d_sids.as<uint32_t>(),
+                                                   d_qseg.as<uint32_t>(), nsid, nseg, d_segs.as<SegDesc>());
+    launches++;
+  }
   const uint64_t lim_pad = total_bytes + 64;  // every aligned 16-byte block below this is readable
-  for (int i = 0; i < n; ++i) {
+  for (size_t i = 0; i < np; ++i) {
+    const Piece& pc = pieces[i];
     MCU(cudaStreamWaitEvent(s, cl.ev[i], 0));
     MCU(cudaEventRecord(cl.tev[2 + 2 * i], s));
-    const uint32_t s0 = in_seg[i], ns = in_seg[i + 1] - in_seg[i];
-    const uint32_t q0 = in_sid[i], nq = in_sid[i + 1] - in_sid[i];
+    const uint32_t q0 = pc.q0, nq = pc.q1 - pc.q0, s0 = qseg[pc.q0], ns = qseg[pc.q1] - s0;
     if (nq) {
       k_stream_heads<T><<<(nq + 255) / 256, 256, 0, s>>>(d_bytes.as<uint8_t>(), d_streams.as<StreamDesc>(),
                                                          d_sids.as<uint32_t>() + q0, nq, d_keys.as<T>(),
                                                          d_counts.as<unsigned long long>(), d_first.as<T>());
       launches++;
     }
-    if (ns) {
-      // DVLE varints: counts per segment and their scan, relative rows, the
-      // scan of the delta sums, start keys; no host round trip
-      const unsigned gsegs = (ns + kDecWarps - 1) / kDecWarps;
+    const unsigned gsegs = (ns + kDecWarps - 1) / kDecWarps;
+    if (ns)
       k_seg_count<<<gsegs, 32 * kDecWarps, 0, s>>>(d_bytes.as<uint8_t>(), lim_pad, d_segs.as<SegDesc>() + s0, ns,
                                                    d_streams.as<StreamDesc>(), d_terms.as<uint32_t>() + s0);
-      k_stream_seg_scan<<<(nq + 7) / 8, 256, 0, s>>>(d_terms.as<uint32_t>(), d_sfirst.as<uint32_t>(),
-                                                     d_send.as<uint32_t>(), d_streams.as<StreamDesc>(),
-                                                     d_sids.as<uint32_t>() + q0, nq,
+    if (nq)
+      k_stream_seg_scan<<<(nq + 7) / 8, 256, 0, s>>>(d_terms.as<uint32_t>(), d_qseg.as<uint32_t>() + q0,
+                                                     d_streams.as<StreamDesc>(), d_sids.as<uint32_t>() + q0, nq,
                                                      d_vstart.as<unsigned long long>(), dst);
+    if (ns) {
       k_seg_rows<T><<<gsegs, 32 * kDecWarps, 0, s>>>(d_bytes.as<uint8_t>(), lim_pad, d_segs.as<SegDesc>() + s0, ns,
                                                      d_streams.as<StreamDesc>(), d_vstart.as<unsigned long long>() + s0,
                                                      d_keys.as<T>(), d_counts.as<unsigned long long>(),
                                                      d_dsum.as<T>() + s0);
-      k_stream_base_scan<T><<<(nq + 7) / 8, 256, 0, s>>>(d_dsum.as<T>(), d_sfirst.as<uint32_t>(), d_send.as<uint32_t>(),
-                                                         d_first.as<T>(), d_sids.as<uint32_t>() + q0, nq,
-                                                         d_kstart.as<T>());
+      k_stream_base_scan<T><<<(nq + 7) / 8, 256, 0, s>>>(d_dsum.as<T>(), d_qseg.as<uint32_t>() + q0, d_first.as<T>(),
+                                                         d_sids.as<uint32_t>() + q0, nq, d_kstart.as<T>());
       k_seg_base<T><<<gsegs, 32 * kDecWarps, 0, s>>>(d_segs.as<SegDesc>() + s0, ns, d_streams.as<StreamDesc>(),
                                                      d_terms.as<uint32_t>() + s0,
                                                      d_vstart.as<unsigned long long>() + s0, d_kstart.as<T>() + s0,
@@ -1145,9 +1286,59 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
                                                            d_keys.as<T>(), d_counts.as<unsigned long long>());
     launches++;
   }
+  // stage times of the decode ([0], its kernels alone) and the copies in ([5])
+  auto copy_times = [&]() {
+    float ms = 0, dec = 0;
+    for (size_t i = 0; i < np; ++i)
+      if (cudaEventElapsedTime(&ms, cl.tev[2 + 2 * i], cl.tev[3 + 2 * i]) == cudaSuccess) dec += ms;
+    stat->stage_ms[0] = dec;
+    if (cudaEventElapsedTime(&ms, cl.tev[0], cl.tev[1]) == cudaSuccess) stat->stage_ms[5] = ms;
+  };
+  auto bad_delta = [&]() {
+    return fail(KITE_ERR_BAD_INPUT, sizeof(T) == 8 ? "invalid u64 DVLE delta" : "invalid u128 DVLE delta");
+  };
   DevStatus hdec{};
   MCU(cudaMemcpyAsync(&hdec, dst, sizeof hdec, cudaMemcpyDeviceToHost, s));
   MCU(cudaEventRecord(sev[1], s));
+  auto stage_times = [&]() {
+    static const int pairs[5][2] = {{0, 1}, {1, 2}, {2, 3}, {4, 5}, {5, 6}};
+    float ms = 0;
+    for (int i = 0; i < 5; ++i)
+      if (cudaEventElapsedTime(&ms, sev[pairs[i][0]], sev[pairs[i][1]]) == cudaSuccess) stat->stage_ms[i] = ms;
+    // [0] the decode kernels alone (the wait for each piece's bytes left
+    // out), [5] the copies of the inputs in, which the decode overlaps
+    copy_times();
+  };
+  if (mode == kModeQuery) {
+    // ---- query: every key looked up in the streams of its partition ----
+    const uint32_t nq = (uint32_t)ex->nq;
+    std::vector<T> qk(nq);
+    for (uint32_t q = 0; q < nq; ++q) qk[q] = (T)(((unsigned __int128)ex->keys[2 * q + 1] << 64) | ex->keys[2 * q]);
+    Dev d_qk(pool, 28), d_qp(pool, 29), d_qout(pool, 30);
+    if (!d_qk.ensure(nq * sizeof(T) + 16) || !d_qp.ensure(nq * 4 + 8) || !d_qout.ensure(nq * 8 + 8))
+      return fail(KITE_ERR_OOM, "query buffers");
+    for (int i = 2; i < 5; ++i) MCU(cudaEventRecord(sev[i], s));
+    if (nq) {
+      MCU(cudaMemcpyAsync(d_qk.p, qk.data(), nq * sizeof(T), cudaMemcpyHostToDevice, s));
+      MCU(cudaMemcpyAsync(d_qp.p, ex->parts, nq * 4, cudaMemcpyHostToDevice, s));
+      k_query_streams<T><<<(nq + 255) / 256, 256, 0, s>>>(d_keys.as<T>(), d_counts.as<unsigned long long>(),
+                                                          d_streams.as<StreamDesc>(), d_pfirst.as<uint32_t>(),
+                                                          d_qk.as<T>(), d_qp.as<uint32_t>(), nq,
+                                                          d_qout.as<unsigned long long>());
+      launches++;
+    }
+    MCU(cudaEventRecord(sev[5], s));
+    std::vector<uint64_t> found(nq);
+    if (nq) MCU(cudaMemcpyAsync(found.data(), d_qout.p, nq * 8, cudaMemcpyDeviceToHost, s));
+    MCU(cudaEventRecord(sev[6], s));
+    if (sync()) return fail(KITE_ERR_TIMEOUT, "query wait");
+    MCU(cudaGetLastError());
+    if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
+    if (nq) std::memcpy(ex->counts_out, found.data(), nq * 8);
+    stage_times();
+    stat->kernel_launches = launches;
+    return KITE_OK;
+  }
   // planning phases, host wall clock (the decode's kernels run meanwhile until
   // the first wait): [6] splitters, [7] first cut, [8] bisection, [9] tile lists
   auto wall = []() { return std::chrono::steady_clock::now(); };
@@ -1155,30 +1346,23 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - a).count();
   };
   auto tp0 = wall();
-  // ---- tiles: global splitters from a row sample, refined by bisection ----
-  std::vector<uint32_t> part_first_stream(P + 1, 0);
-  {
-    uint32_t si = 0;
-    for (uint32_t p = 0; p < P; ++p) {
-      part_first_stream[p] = si;
-      while (si < nst && streams[si].partition == p) si++;
-    }
-    part_first_stream[P] = nst;
-  }
-  // tiles of three quarters of the on-chip capacity on average (the
-  // refinement below splits the few that the cut leaves above it): the merge
-  // kernel's cost per tile is mostly fixed (stream scan, merge rounds,
-  // barriers), so fuller tiles cost less per row
+  // ---- tiles.  Partitions of one stream each are cut every kMergeCap rows;
+  // others by global splitters from a row sample into tiles of three quarters
+  // of the on-chip capacity on average (the merge kernel's cost per tile is
+  // mostly fixed, so fuller tiles cost less per row).  The cut, the tiles and
+  // their stream ranges are made on the device; only when one of its ranges is
+  // above the capacity (skewed keys) does the host cut again, with bisection.
+  // (The host's lists and the copies of the position matrix and the tiles took
+  // 3.0 - 4.7 ms of each call at 50 - 100M rows, 0.1 - 0.2 ms now.)
   uint32_t S = 1;
-  {
+  auto want_ranges = [&]() {
     const double want = (double)total_rows / ((double)P * 0.75 * kMergeCap);
-    if (want > 1.0) S = (uint32_t)std::min(4096.0, std::ceil(want));
-  }
-  std::vector<T> spl;
-  Dev d_spl;
-  if (S > 1 && total_rows) {
+    return want > 1.0 ? (uint32_t)std::min(4096.0, std::ceil(want)) : 1u;
+  };
+  Dev d_spl(pool, 28), d_pos(pool, 31);
+  auto make_splitters = [&]() -> int {  // S - 1 of them
     const uint32_t ns = (uint32_t)std::min<uint64_t>(total_rows, 1u << 20);
-    Dev d_sample, d_hist;
+    Dev d_sample(pool, 29), d_hist(pool, 30);
     if (!d_sample.ensure(ns * sizeof(T)) || !d_spl.ensure(S * sizeof(T)) || !d_hist.ensure(65536 * 4))
       return fail(KITE_ERR_OOM, "merge splitters");
     k_sample_rows<T><<<(ns + 255) / 256, 256, 0, s>>>(d_keys.as<T>(), total_rows, ns, d_sample.as<T>());
@@ -1187,9 +1371,10 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     launches += 1 + compute_hist_splitters<T>(d_sample.as<T>(), ns, key_bits, S, d_spl.as<T>(),
                                               d_hist.as<unsigned>(), s);
     stat->splitter_used = KITE_SPLIT_SAMPLED;
-    if (ex && ex->mlp && ex->splitter_mode != KITE_SPLIT_SAMPLED) {
-      // the learned CDF of the row sample cuts the merged key range; kept
-      // when its predicted max/mean tile load is the lower one (LEARNED: always)
+    if (ex && ex->mlp && ex->splitter_mode == KITE_SPLIT_LEARNED) {
+      // the learned CDF of the row sample, on request: its training (650 ms)
+      // is longer than most merges, and ranges that the histogram cuts badly
+      // are bisected
       double hist_imb = 0.0;
       if (predict_imbalance<T>(ex->mlp, d_sample.as<T>(), ns, d_spl.as<T>(), S, s, timeout_ms, &hist_imb))
         return fail(KITE_ERR_TIMEOUT, "merge splitter evaluation did not finish");
@@ -1203,31 +1388,84 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       stat->mlp_pred_imbalance = rep.pred_imbalance;
       stat->mlp_loss = rep.loss;
       stat->mlp_reused = rep.reused ? 1u : 0u;
-      if (rep.pred_imbalance < 1e29 && (ex->splitter_mode == KITE_SPLIT_LEARNED || rep.pred_imbalance < hist_imb)) {
+      if (rep.pred_imbalance < 1e29) {
         MCU(cudaMemcpyAsync(d_spl.p, d_spl2.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToDevice, s));
         stat->splitter_used = KITE_SPLIT_LEARNED;
       }
       if (sync()) return fail(KITE_ERR_TIMEOUT, "merge splitter wait");
     }
-    spl.resize(S - 1);
-    MCU(cudaMemcpyAsync(spl.data(), d_spl.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToHost, s));
-  } else {
-    S = 1;
+    return KITE_OK;
+  };
+  auto range_positions = [&]() -> int {
+    const uint64_t nq = (uint64_t)nst * (S + 1);
+    if (!d_pos.ensure(nq * 8)) return fail(KITE_ERR_OOM, "merge range positions");
+    k_range_positions<T><<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(d_keys.as<T>(), d_streams.as<StreamDesc>(), nst,
+                                                                     d_spl.as<T>(), S, d_pos.as<uint64_t>());
+    launches++;
+    return KITE_OK;
+  };
+  std::vector<MergeTile> mts;  // the host's cut; empty when the device made the tiles
+  std::vector<TileDesc> tds;
+  std::vector<uint32_t> tile_first(P + 1, 0);
+  const uint64_t out_off = total_rows;  // rows reserved for the output
+  uint32_t ntiles = 0;
+  TileStream* tss = nullptr;
+  std::vector<TileStream> tss_own;
+  size_t nts_all = 0;
+  Dev d_mt(pool, 15), d_ts(pool, 16), d_tds(pool, 22);
+  bool planned = false;  // the tiles are on the device
+  unsigned info[3] = {0, 0, 0};
+  if (total_rows && most_streams <= kMaxTileStreams) {
+    const bool slices = most_streams <= 1;
+    S = slices ? (uint32_t)((most_rows + kMergeCap - 1) / kMergeCap) : want_ranges();
+    if ((uint64_t)P * S <= 4 * (total_rows / kMergeCap + P)) {
+      const uint64_t nt = (uint64_t)P * S, npos = (uint64_t)nst * (S + 1);
+      if (!slices && S > 1) {
+        if (const int rc = make_splitters()) return rc;
+        if (const int rc = range_positions()) return rc;
+      } else {
+        if (!d_pos.ensure(npos * 8)) return fail(KITE_ERR_OOM, "merge range positions");
+        k_slice_positions<T><<<(unsigned)((npos + 255) / 256), 256, 0, s>>>(
+            d_keys.as<T>(), d_streams.as<StreamDesc>(), nst, S, d_pos.as<uint64_t>());
+        launches++;
+        stat->splitter_used = KITE_SPLIT_SAMPLED;
+      }
+      if (!d_mt.ensure(nt * sizeof(MergeTile) + 8) || !d_ts.ensure((size_t)nst * S * sizeof(TileStream) + 8) ||
+          !d_tds.ensure(nt * sizeof(TileDesc) + 8))
+        return fail(KITE_ERR_OOM, "merge tile buffers");
+      k_plan_tiles<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(
+          d_pos.as<uint64_t>(), d_streams.as<StreamDesc>(), d_pfirst.as<uint32_t>(), P, S, d_mt.as<MergeTile>(),
+          d_ts.as<TileStream>(), d_tds.as<TileDesc>(), plan_info);
+      launches++;
+      MCU(cudaMemcpyAsync(info, plan_info, sizeof info, cudaMemcpyDeviceToHost, s));
+      if (sync()) return fail(KITE_ERR_TIMEOUT, "merge tile wait");
+      if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
+      planned = info[0] == 0;
+      if (planned) {
+        ntiles = (uint32_t)nt;
+        nts_all = (size_t)nst * S;
+        for (uint32_t p = 0; p <= P; ++p) tile_first[p] = p * S;
+      }
+    }
   }
   stat->stage_ms[6] = ms_since(tp0);
+  if (!planned) {
+  // ---- the host's cut ----
+  S = total_rows ? want_ranges() : 1;
+  std::vector<T> spl;
+  if (S > 1) {
+    if (const int rc = make_splitters()) return rc;
+    spl.resize(S - 1);
+    MCU(cudaMemcpyAsync(spl.data(), d_spl.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToHost, s));
+  }
   auto tp1 = wall();
   // ---- first cut on the device: the row position of every splitter in every
   // stream (one binary search each), read back as one matrix
   const size_t SP = (size_t)S + 1;
   std::vector<uint64_t> pos((size_t)nst * SP);
   if (nst && S > 1) {
-    Dev d_pos;
-    if (!d_pos.ensure(pos.size() * 8)) return fail(KITE_ERR_OOM, "merge range positions");
-    const uint64_t nq = pos.size();
-    k_range_positions<T><<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(d_keys.as<T>(), d_streams.as<StreamDesc>(), nst,
-                                                                     d_spl.as<T>(), S, d_pos.as<uint64_t>());
-    launches++;
-    MCU(cudaMemcpyAsync(pos.data(), d_pos.p, nq * 8, cudaMemcpyDeviceToHost, s));
+    if (const int rc = range_positions()) return rc;
+    MCU(cudaMemcpyAsync(pos.data(), d_pos.p, pos.size() * 8, cudaMemcpyDeviceToHost, s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge range wait");
   } else {
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge splitter wait");
@@ -1298,8 +1536,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   for (uint32_t p = 0; p < P; ++p) work.insert(work.end(), cut[p].work.begin(), cut[p].work.end());
   std::vector<uint64_t>().swap(pos);
   // the decode's status arrived with the sync above
-  if (hdec.code == KITE_DEV_SHORT_VARINTS)
-    return fail(KITE_ERR_BAD_INPUT, sizeof(T) == 8 ? "invalid u64 DVLE delta" : "invalid u128 DVLE delta");
+  if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
   Dev d_qlo, d_qhi, d_qkey, d_qout;
   std::vector<uint64_t> lp, hp;
   for (int round = 0; !work.empty() && round < 200; ++round) {
@@ -1411,21 +1648,15 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   // the partitions' offsets, then every partition's tiles and stream ranges
   // written in place in parallel, the stream ranges straight into pinned
   // memory for their copy to the device
-  std::vector<MergeTile> mts;
-  std::vector<TileDesc> tds;
-  std::vector<uint32_t> tile_first(P + 1, 0);
   std::vector<uint64_t> ts_first(P + 1, 0), row_first(P + 1, 0);
   for (uint32_t p = 0; p < P; ++p) {
     tile_first[p + 1] = tile_first[p] + (uint32_t)pt[p].mts.size();
     ts_first[p + 1] = ts_first[p] + pt[p].tss.size();
     row_first[p + 1] = row_first[p] + pt[p].rows;
   }
-  const uint64_t out_off = row_first[P];
-  const size_t nts_all = (size_t)ts_first[P];
+  nts_all = (size_t)ts_first[P];
   mts.resize(tile_first[P]);
   tds.resize(tile_first[P]);
-  std::vector<TileStream> tss_own;
-  TileStream* tss = nullptr;
   if (pool) {
     MergePoolSlot& hs = pool->host;
     const size_t need = nts_all * sizeof(TileStream) + 64;
@@ -1456,45 +1687,53 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     PartTiles().tss.swap(o.tss);
   });
   stat->stage_ms[9] = ms_since(tp3);
-  const uint32_t ntiles = (uint32_t)mts.size();
+  ntiles = (uint32_t)mts.size();
+  }  // the host's cut
   std::vector<InputFilter> filt(n);
   for (int i = 0; i < n; ++i)
     filt[i] = InputFilter{(uint32_t)in[i].has_min, (uint32_t)in[i].has_max, in[i].min_count, in[i].max_count};
-  Dev d_mt(pool, 15), d_ts(pool, 16), d_filt(pool, 17), d_okeys(pool, 18), d_ocounts(pool, 19), d_tout(pool, 20),
-      d_over(pool, 21), d_tds(pool, 22), d_tf(pool, 23), d_boff(pool, 24), d_prev(pool, 25), d_meta(pool, 26),
-      d_out(pool, 27);
+  Dev d_filt(pool, 17), d_okeys(pool, 18), d_ocounts(pool, 19), d_tout(pool, 20), d_over(pool, 21), d_tf(pool, 23),
+      d_boff(pool, 24), d_prev(pool, 25), d_meta(pool, 26), d_out(pool, 27);
   if (!d_mt.ensure(ntiles * sizeof(MergeTile) + 8) || !d_ts.ensure(nts_all * sizeof(TileStream) + 8) ||
       !d_filt.ensure(n * sizeof(InputFilter)) || !d_okeys.ensure(out_off * sizeof(T) + 16) ||
       !d_ocounts.ensure(out_off * 4 + 16) || !d_tout.ensure(ntiles * sizeof(TileOut<T>) + 16) ||
       !d_over.ensure(8) || !d_tds.ensure(ntiles * sizeof(TileDesc) + 8) || !d_tf.ensure((P + 1) * 4) ||
       !d_boff.ensure(ntiles * 8 + 8) || !d_prev.ensure(ntiles * sizeof(T) + 16) || !d_meta.ensure(P * sizeof(BucketMeta)))
     return fail(KITE_ERR_OOM, "merge tile buffers");
-  if (ntiles) {
+  if (!mts.empty()) {
     MCU(cudaMemcpyAsync(d_mt.p, mts.data(), ntiles * sizeof(MergeTile), cudaMemcpyHostToDevice, s));
     MCU(cudaMemcpyAsync(d_ts.p, tss, nts_all * sizeof(TileStream), cudaMemcpyHostToDevice, s));
+    MCU(cudaMemcpyAsync(d_tds.p, tds.data(), ntiles * sizeof(TileDesc), cudaMemcpyHostToDevice, s));
   }
+  MCU(cudaMemcpyAsync(d_tf.p, tile_first.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
   MCU(cudaMemcpyAsync(d_filt.p, filt.data(), n * sizeof(InputFilter), cudaMemcpyHostToDevice, s));
   MCU(cudaMemsetAsync(d_over.p, 0xff, 8, s));
+  auto tile_imbalance = [&]() {
+    uint64_t tmax = info[1], tne = info[2];
+    if (!planned) {
+      tmax = tne = 0;
+      for (auto& m : mts) {
+        tmax = std::max<uint64_t>(tmax, m.rows_in);
+        tne += m.rows_in != 0;
+      }
+    }
+    return tne ? (double)tmax / ((double)out_off / (double)tne) : 0.0;
+  };
   const size_t smem = MergeSmem<T>::total;
   auto kmerge = mode == kModeDump    ? k_merge_tiles<T, kModeDump>
                 : mode == kModeHisto ? k_merge_tiles<T, kModeHisto>
-                : mode == kModeRows  ? k_merge_tiles<T, kModeRows>
                                      : k_merge_tiles<T, kModeMerge>;
   cudaFuncSetAttribute(kmerge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   MergeAux aux{};
   aux.line_k = key_bits / 2;
-  Dev d_hist, d_spill, d_c64;
+  Dev d_hist(pool, 30);
   if (mode == kModeHisto) {
-    if (!d_hist.ensure((kHistBins + 1) * 8) || !d_spill.ensure(out_off * 8 + 8)) return fail(KITE_ERR_OOM, "histo buffers");
+    if (!d_hist.ensure((kHistBins + 1) * 8)) return fail(KITE_ERR_OOM, "histo buffers");
     MCU(cudaMemsetAsync(d_hist.p, 0, (kHistBins + 1) * 8, s));
     aux.hist = d_hist.as<unsigned long long>();
     aux.spill_n = aux.hist + kHistBins;
-    aux.spill = d_spill.as<unsigned long long>();
+    aux.spill = d_okeys.as<unsigned long long>();  // no rows are written in this mode
     aux.spill_cap = out_off;
-  }
-  if (mode == kModeRows) {
-    if (!d_c64.ensure(out_off * 8 + 8)) return fail(KITE_ERR_OOM, "query buffers");
-    aux.counts64 = d_c64.as<unsigned long long>();
   }
   if (mode == kModeMerge && ntiles) {
     // ---- merge, encode and copy-out pipelined over partition groups: group
@@ -1511,18 +1750,25 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       static const uint32_t cw[9] = {0, 6, 12, 18, 24, 30, 35, 38, 40};
       for (uint32_t g = 0; g <= NG; ++g) pb[g] = (uint32_t)((uint64_t)P * cw[g] / 40);
     }
-    MCU(cudaMemcpyAsync(d_tds.p, tds.data(), ntiles * sizeof(TileDesc), cudaMemcpyHostToDevice, s));
-    MCU(cudaMemcpyAsync(d_tf.p, tile_first.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
     if (!d_over.ensure((size_t)NG * 8)) return fail(KITE_ERR_OOM, "merge tile buffers");
     MCU(cudaMemsetAsync(d_over.p, 0xff, (size_t)NG * 8, s));  // per group: its first overflowing row
+    // pinned partition records (kept by the pool)
+    MergePoolSlot hm_own;
+    MergePoolSlot& hms = pool ? pool->records : hm_own;
     struct HostMem {
-      void* p = nullptr;
+      MergePoolSlot& own;
       ~HostMem() {
-        if (p) cudaFreeHost(p);
+        if (own.p) cudaFreeHost(own.p);
       }
-    } hmm;
-    MCU(cudaMallocHost(&hmm.p, (size_t)P * sizeof(BucketMeta)));
-    BucketMeta* hm = static_cast<BucketMeta*>(hmm.p);
+    } hmm{hm_own};
+    if (hms.cap < (size_t)P * sizeof(BucketMeta)) {
+      if (hms.p) cudaFreeHost(hms.p);
+      hms.p = nullptr;
+      hms.cap = 0;
+      MCU(cudaMallocHost(&hms.p, (size_t)P * sizeof(BucketMeta)));
+      hms.cap = (size_t)P * sizeof(BucketMeta);
+    }
+    BucketMeta* hm = static_cast<BucketMeta*>(hms.p);
     BucketMeta* hm_dev = nullptr;
     MCU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hm_dev), hm, 0));
     // output buffers: the inputs' payload size to start with (a merged
@@ -1537,9 +1783,6 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       if (!hown) return fail(KITE_ERR_OOM, "merge output host buffer");
       hout = hown.get();
     }
-    DevStatus* est = nullptr;
-    MCU(cudaMallocAsync(&est, sizeof(DevStatus), s));
-    MCU(cudaMemsetAsync(est, 0, sizeof(DevStatus), s));
     struct Evs {
       std::vector<cudaEvent_t> e;
       ~Evs() {
@@ -1618,8 +1861,6 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     MCU(cudaMemcpyAsync(&hest, est, sizeof hest, cudaMemcpyDeviceToHost, s));
     MCU(cudaMemcpyAsync(overs.data(), d_over.p, (size_t)NG * 8, cudaMemcpyDeviceToHost, s));
     if (bounded_sync(s, timeout_ms) || bounded_sync(cl.cs, timeout_ms)) return fail(KITE_ERR_TIMEOUT, "merge wait");
-    cudaFreeAsync(dst, s);
-    cudaFreeAsync(est, s);
     if (hst.code) {
       char b[160];
       snprintf(b, sizeof b, "merge: device status %u (%u, %u, %u)", hst.code, hst.a, hst.b, hst.c);
@@ -1630,7 +1871,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       // first overflowing row in (partition, key) order: name its key like the reference
       const uint32_t t = tile_first[pb[g]] + (uint32_t)(overs[g] >> 32), r = (uint32_t)(overs[g] & 0xffffffffu);
       T key{};
-      MCU(cudaMemcpy(&key, d_okeys.as<T>() + mts[t].out_off + r, sizeof(T), cudaMemcpyDeviceToHost));
+      MergeTile mt{};
+      MCU(cudaMemcpy(&mt, d_mt.as<MergeTile>() + t, sizeof mt, cudaMemcpyDeviceToHost));
+      MCU(cudaMemcpy(&key, d_okeys.as<T>() + mt.out_off + r, sizeof(T), cudaMemcpyDeviceToHost));
       unsigned __int128 v = (unsigned __int128)key;
       std::string ks;
       if (v == 0) ks = "0";
@@ -1648,11 +1891,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       float ms = 0;
       for (int i = 0; i < 2; ++i)
         if (cudaEventElapsedTime(&ms, sev[pairs[i][0]], sev[pairs[i][1]]) == cudaSuccess) stat->stage_ms[i] = ms;
-      float dec = 0;
-      for (int i = 0; i < n; ++i)
-        if (cudaEventElapsedTime(&ms, cl.tev[2 + 2 * i], cl.tev[3 + 2 * i]) == cudaSuccess) dec += ms;
-      stat->stage_ms[0] = dec;
-      if (cudaEventElapsedTime(&ms, cl.tev[0], cl.tev[1]) == cudaSuccess) stat->stage_ms[5] = ms;
+      copy_times();
       double mg = 0, en = 0, cp = 0;
       for (uint32_t g = 0; g < NG; ++g) {
         if (cudaEventElapsedTime(&ms, ge[7 * g], ge[7 * g + 1]) == cudaSuccess) mg += ms;
@@ -1669,14 +1908,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     stat->payload_bytes = total_out;
     stat->tiles = ntiles;
     stat->kernel_launches = launches;
-    uint64_t tmax = 0, tsum = 0, tne = 0;
-    for (auto& m : mts)
-      if (m.rows_in) {
-        tmax = std::max<uint64_t>(tmax, m.rows_in);
-        tsum += m.rows_in;
-        tne++;
-      }
-    stat->tile_imbalance = tne ? (double)tmax / ((double)tsum / tne) : 0.0;
+    stat->tile_imbalance = tile_imbalance();
     if (!emit) return KITE_OK;
     for (uint32_t g = 0; g < NG; ++g)
       for (uint32_t p = pb[g]; p < pb[g + 1]; ++p) {
@@ -1705,43 +1937,25 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     launches++;
   }
   MCU(cudaEventRecord(sev[3], s));
+  stat->tiles = ntiles;
   DevStatus hst{};
-  unsigned long long over = 0;
-  std::vector<TileOut<T>> htout(ntiles);
   MCU(cudaMemcpyAsync(&hst, dst, sizeof hst, cudaMemcpyDeviceToHost, s));
-  MCU(cudaMemcpyAsync(&over, d_over.p, 8, cudaMemcpyDeviceToHost, s));
-  if (ntiles) MCU(cudaMemcpyAsync(htout.data(), d_tout.p, ntiles * sizeof(TileOut<T>), cudaMemcpyDeviceToHost, s));
-  if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
-  cudaFreeAsync(dst, s);
-  if (hst.code) {
+  auto bad_status = [&]() {
     char b[160];
     snprintf(b, sizeof b, "%s: device status %u (%u, %u, %u)", dump ? "dump" : "merge", hst.code, hst.a, hst.b,
              hst.c);
     return fail(hst.code == KITE_DEV_BAD_INPUT ? KITE_ERR_BAD_INPUT : KITE_ERR_DEVICE, b);
-  }
-  auto stage_times = [&]() {
-    static const int pairs[5][2] = {{0, 1}, {1, 2}, {2, 3}, {4, 5}, {5, 6}};
-    float ms = 0;
-    for (int i = 0; i < 5; ++i)
-      if (cudaEventElapsedTime(&ms, sev[pairs[i][0]], sev[pairs[i][1]]) == cudaSuccess) stat->stage_ms[i] = ms;
-    // [0] the decode kernels alone (the wait for each input's bytes left
-    // out), [5] the copies of the inputs in, which the decode overlaps
-    float dec = 0;
-    for (int i = 0; i < n; ++i)
-      if (cudaEventElapsedTime(&ms, cl.tev[2 + 2 * i], cl.tev[3 + 2 * i]) == cudaSuccess) dec += ms;
-    stat->stage_ms[0] = dec;
-    if (cudaEventElapsedTime(&ms, cl.tev[0], cl.tev[1]) == cudaSuccess) stat->stage_ms[5] = ms;
   };
-  stat->tiles = ntiles;
   if (mode == kModeHisto) {
     // ---- count -> frequency: the small bins, then the listed large counts ----
     std::vector<unsigned long long> hb(kHistBins + 1);
     MCU(cudaMemcpyAsync(hb.data(), d_hist.p, (kHistBins + 1) * 8, cudaMemcpyDeviceToHost, s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "histo wait");
+    if (hst.code) return bad_status();
     const unsigned long long ns = std::min<unsigned long long>(hb[kHistBins], out_off);
     std::vector<unsigned long long> big(ns);
     MCU(cudaEventRecord(sev[4], s));
-    if (ns) MCU(cudaMemcpyAsync(big.data(), d_spill.p, ns * 8, cudaMemcpyDeviceToHost, s));
+    if (ns) MCU(cudaMemcpyAsync(big.data(), d_okeys.p, ns * 8, cudaMemcpyDeviceToHost, s));
     MCU(cudaEventRecord(sev[5], s));
     MCU(cudaEventRecord(sev[6], s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "histo wait");
@@ -1762,75 +1976,30 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     }
     return KITE_OK;
   }
-  if (mode == kModeRows) {
-    // ---- query lookups over the non-empty tiles of each partition ----
-    std::vector<uint32_t> qtf(P + 1, 0), qrows;
-    std::vector<T> qkey0;
-    std::vector<unsigned long long> qoff;
-    for (uint32_t p = 0; p < P; ++p) {
-      qtf[p] = (uint32_t)qrows.size();
-      for (uint32_t t = tile_first[p]; t < tile_first[p + 1]; ++t)
-        if (htout[t].rows) {
-          qkey0.push_back(htout[t].first_key);
-          qoff.push_back(mts[t].out_off);
-          qrows.push_back(htout[t].rows);
-        }
-    }
-    qtf[P] = (uint32_t)qrows.size();
-    const uint32_t nq = (uint32_t)ex->nq, nt = (uint32_t)qrows.size();
-    std::vector<T> qk(nq);
-    std::vector<uint32_t> qp(nq);
-    for (uint32_t q = 0; q < nq; ++q) {
-      qk[q] = (T)(((unsigned __int128)ex->keys[2 * q + 1] << 64) | ex->keys[2 * q]);
-      qp[q] = ex->parts[q];
-    }
-    Dev d_qtf, d_qk0, d_qoff, d_qrows, d_qk, d_qp, d_qout;
-    if (!d_qtf.ensure((P + 1) * 4) || !d_qk0.ensure(nt * sizeof(T) + 16) || !d_qoff.ensure(nt * 8 + 8) ||
-        !d_qrows.ensure(nt * 4 + 8) || !d_qk.ensure(nq * sizeof(T) + 16) || !d_qp.ensure(nq * 4 + 8) ||
-        !d_qout.ensure(nq * 8 + 8))
-      return fail(KITE_ERR_OOM, "query buffers");
-    MCU(cudaMemcpyAsync(d_qtf.p, qtf.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
-    if (nt) {
-      MCU(cudaMemcpyAsync(d_qk0.p, qkey0.data(), nt * sizeof(T), cudaMemcpyHostToDevice, s));
-      MCU(cudaMemcpyAsync(d_qoff.p, qoff.data(), nt * 8, cudaMemcpyHostToDevice, s));
-      MCU(cudaMemcpyAsync(d_qrows.p, qrows.data(), nt * 4, cudaMemcpyHostToDevice, s));
-    }
-    MCU(cudaEventRecord(sev[4], s));
-    if (nq) {
-      MCU(cudaMemcpyAsync(d_qk.p, qk.data(), nq * sizeof(T), cudaMemcpyHostToDevice, s));
-      MCU(cudaMemcpyAsync(d_qp.p, qp.data(), nq * 4, cudaMemcpyHostToDevice, s));
-      k_query_rows<T><<<(nq + 255) / 256, 256, 0, s>>>(d_okeys.as<T>(), d_c64.as<unsigned long long>(),
-                                                       d_qtf.as<uint32_t>(), d_qk0.as<T>(),
-                                                       d_qoff.as<unsigned long long>(), d_qrows.as<uint32_t>(),
-                                                       d_qk.as<T>(), d_qp.as<uint32_t>(), nq,
-                                                       d_qout.as<unsigned long long>());
-      launches++;
-    }
-    MCU(cudaEventRecord(sev[5], s));
-    if (nq) MCU(cudaMemcpyAsync(ex->counts_out, d_qout.p, nq * 8, cudaMemcpyDeviceToHost, s));
-    MCU(cudaEventRecord(sev[6], s));
-    if (sync()) return fail(KITE_ERR_TIMEOUT, "query wait");
-    MCU(cudaGetLastError());
-    stage_times();
-    stat->kernel_launches = launches;
-    return KITE_OK;
-  }
   if (dump) {
-    // ---- TSV: tile byte offsets in (partition, key) order, then formatting ----
-    std::vector<unsigned long long> tboff(ntiles + 1);
-    std::vector<uint64_t> prow(P, 0), pbytes(P, 0);
+    // ---- TSV: tile byte offsets in (partition, key) order on the device, the
+    // partitions' records back to the host, then formatting ----
+    Dev d_lines(pool, 32), d_scan(pool, 33);
+    if (!d_boff.ensure((ntiles + 1) * 8) || !d_lines.ensure(P * sizeof(PartLines)) ||
+        !d_scan.ensure(scan_tmp_elems(ntiles + 1) * 8 + 64))
+      return fail(KITE_ERR_OOM, "dump output");
+    std::vector<PartLines> lines(P);
+    if (ntiles) {
+      k_part_lines<T><<<(P + 7) / 8, 256, 0, s>>>(d_tout.as<TileOut<T>>(), d_tf.as<uint32_t>(), P,
+                                                  d_boff.as<unsigned long long>(), d_lines.as<PartLines>());
+      launches += 1 + exclusive_scan_u64(d_boff.as<unsigned long long>(), d_boff.as<unsigned long long>(), ntiles,
+                                         d_scan.as<unsigned long long>(), s);
+      MCU(cudaMemcpyAsync(lines.data(), d_lines.p, P * sizeof(PartLines), cudaMemcpyDeviceToHost, s));
+    }
+    if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
+    if (hst.code) return bad_status();
     unsigned long long acc = 0;
     uint64_t out_rows = 0;
-    for (uint32_t t = 0; t < ntiles; ++t) {
-      tboff[t] = acc;
-      acc += htout[t].rest_bytes;
-      prow[mts[t].partition] += htout[t].rows;
-      pbytes[mts[t].partition] += htout[t].rest_bytes;
-      out_rows += htout[t].rows;
+    for (const PartLines& l : lines) {
+      acc += l.bytes;
+      out_rows += l.rows;
     }
-    tboff[ntiles] = acc;
-    if (!d_boff.ensure((ntiles + 1) * 8) || !d_out.ensure(acc + 16)) return fail(KITE_ERR_OOM, "dump output");
-    if (ntiles && acc) MCU(cudaMemcpyAsync(d_boff.p, tboff.data(), (ntiles + 1) * 8, cudaMemcpyHostToDevice, s));
+    if (!d_out.ensure(acc + 16)) return fail(KITE_ERR_OOM, "dump output");
     MCU(cudaEventRecord(sev[4], s));
     if (ntiles && acc) {
       const size_t tsm = 256 + (size_t)kTsvThreads * (key_bits / 2 + 12);
@@ -1843,7 +2012,6 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     stat->d2h_bytes += emit ? acc : 0;
     stat->rows = out_rows;
     stat->payload_bytes = acc;
-    stat->tiles = ntiles;
     stat->kernel_launches = launches;
     if (!emit || acc == 0) {
       MCU(cudaEventRecord(sev[6], s));
@@ -1856,20 +2024,20 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     // group i+2 is queued once group i has been emitted, so the copy of the
     // next group overlaps the callback's work on this one
     uint64_t maxpart = 0;
-    for (uint32_t p = 0; p < P; ++p) maxpart = std::max(maxpart, pbytes[p]);
+    for (uint32_t p = 0; p < P; ++p) maxpart = std::max<uint64_t>(maxpart, lines[p].bytes);
     const uint64_t half = std::max<uint64_t>(std::min<uint64_t>(acc, 256ull << 20), maxpart);
     std::vector<uint32_t> gfirst{0};  // first partition of every group
     std::vector<uint64_t> goff{0};
     {
       uint64_t g = 0, off = 0;
       for (uint32_t p = 0; p < P; ++p) {
-        if (g + pbytes[p] > half) {
+        if (g + lines[p].bytes > half) {
           gfirst.push_back(p);
           goff.push_back(off);
           g = 0;
         }
-        g += pbytes[p];
-        off += pbytes[p];
+        g += lines[p].bytes;
+        off += lines[p].bytes;
       }
       gfirst.push_back(P);
       goff.push_back(off);
@@ -1908,28 +2076,19 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       const uint8_t* src = group_dst(g);
       uint64_t off = 0;
       for (uint32_t p = gfirst[g]; p < gfirst[g + 1]; ++p) {
-        if (!prow[p]) continue;
-        // key range of the partition's lines: first row of its first non-empty
-        // tile, last row of its last one
+        const PartLines& l = lines[p];
+        if (!l.rows) continue;
         kite_chunk_meta cm{};
         cm.partition_id = p;
         cm.codec = 0;
-        cm.row_count = prow[p];
-        cm.raw_bytes = pbytes[p];
-        bool first = true;
-        for (uint32_t t = tile_first[p]; t < tile_first[p + 1]; ++t) {
-          if (!htout[t].rows) continue;
-          const unsigned __int128 a = (unsigned __int128)htout[t].first_key, b = (unsigned __int128)htout[t].last_key;
-          if (first) {
-            cm.key_min_lo[0] = (uint64_t)a;
-            cm.key_min_lo[1] = (uint64_t)(a >> 64);
-            first = false;
-          }
-          cm.key_max_lo[0] = (uint64_t)b;
-          cm.key_max_lo[1] = (uint64_t)(b >> 64);
-        }
-        if (emit(user, &cm, src + off, (size_t)pbytes[p])) return fail(KITE_ERR_CALLBACK, "emit callback aborted");
-        off += pbytes[p];
+        cm.row_count = l.rows;
+        cm.raw_bytes = l.bytes;
+        cm.key_min_lo[0] = l.kmin_lo;
+        cm.key_min_lo[1] = l.kmin_hi;
+        cm.key_max_lo[0] = l.kmax_lo;
+        cm.key_max_lo[1] = l.kmax_hi;
+        if (emit(user, &cm, src + off, (size_t)l.bytes)) return fail(KITE_ERR_CALLBACK, "emit callback aborted");
+        off += l.bytes;
       }
       if (g + 2 < ngroups) MCU(queue_copy(g + 2));
     }
@@ -1939,91 +2098,14 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     stage_times();
     return KITE_OK;
   }
-  if (over != ~0ull) {
-    // first overflowing row in (partition, key) order: name its key like the reference
-    const uint32_t t = (uint32_t)(over >> 32), r = (uint32_t)(over & 0xffffffffu);
-    T key{};
-    MCU(cudaMemcpyAsync(&key, d_okeys.as<T>() + mts[t].out_off + r, sizeof(T), cudaMemcpyDeviceToHost, s));
-    if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
-    unsigned __int128 v = (unsigned __int128)key;
-    std::string ks;
-    if (v == 0) ks = "0";
-    while (v) {
-      ks.insert(ks.begin(), (char)('0' + (int)(v % 10)));
-      v /= 10;
-    }
-    return fail(KITE_ERR_COUNT_OVERFLOW, "merged count exceeds u32 for key " + ks);
-  }
-  // ---- encode: per partition, tiles in key order ----
-  for (uint32_t t = 0; t < ntiles; ++t) tds[t].len = htout[t].rows;
-  if (ntiles) MCU(cudaMemcpyAsync(d_tds.p, tds.data(), ntiles * sizeof(TileDesc), cudaMemcpyHostToDevice, s));
-  MCU(cudaMemcpyAsync(d_tf.p, tile_first.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
-  launch_tile_link_ranges<T>(d_tout.as<TileOut<T>>(), P, d_tf.as<uint32_t>(), d_boff.as<unsigned long long>(),
-                             d_prev.as<T>(), d_meta.as<BucketMeta>(), s);
-  launch_bucket_offsets(d_meta.as<BucketMeta>(), P, nullptr, s);
-  launches += 2;
-  std::vector<BucketMeta> meta(P);
-  MCU(cudaMemcpyAsync(meta.data(), d_meta.p, P * sizeof(BucketMeta), cudaMemcpyDeviceToHost, s));
+  // a merge of inputs without rows
   if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
-  uint64_t out_bytes = 0, out_rows = 0;
-  for (auto& m : meta) {
-    out_bytes += m.bytes;
-    out_rows += m.rows;
-  }
-  if (!d_out.ensure(out_bytes + 16)) return fail(KITE_ERR_OOM, "merge output");
-  DevStatus* est = nullptr;
-  MCU(cudaMallocAsync(&est, sizeof(DevStatus), s));
-  MCU(cudaMemsetAsync(est, 0, sizeof(DevStatus), s));
-  MCU(cudaEventRecord(sev[4], s));
-  launch_encode<T>(d_okeys.as<T>(), d_ocounts.as<uint32_t>(), d_tds.as<TileDesc>(), d_tout.as<TileOut<T>>(),
-                   d_boff.as<unsigned long long>(), d_prev.as<T>(), d_meta.as<BucketMeta>(), ntiles,
-                   d_out.as<uint8_t>(), out_bytes, est, s);
-  launches++;
-  MCU(cudaEventRecord(sev[5], s));
-  // the output to the host: through the caller's pinned staging when given
-  // (a copy at full link speed), else into ordinary host memory
-  uint8_t* hout = staging ? staging(out_bytes + 16) : nullptr;
-  std::unique_ptr<uint8_t[]> hown;
-  if (!hout) {
-    hown.reset(new (std::nothrow) uint8_t[out_bytes + 16]);
-    if (!hown) return fail(KITE_ERR_OOM, "merge output host buffer");
-    hout = hown.get();
-  }
-  if (out_bytes) MCU(cudaMemcpyAsync(hout, d_out.p, out_bytes, cudaMemcpyDeviceToHost, s));
-  MCU(cudaEventRecord(sev[6], s));
-  MCU(cudaMemcpyAsync(&hst, est, sizeof hst, cudaMemcpyDeviceToHost, s));
-  if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
+  if (hst.code) return bad_status();
   stage_times();
-  cudaFreeAsync(est, s);
-  if (hst.code) return fail(KITE_ERR_DEVICE, "merge encode failed");
-  stat->d2h_bytes += out_bytes;
-  stat->rows = out_rows;
-  stat->payload_bytes = out_bytes;
-  stat->tiles = ntiles;
+  stat->rows = 0;
+  stat->payload_bytes = 0;
   stat->kernel_launches = launches;
-  uint64_t tmax = 0, tsum = 0, tne = 0;
-  for (auto& m : mts)
-    if (m.rows_in) {
-      tmax = std::max<uint64_t>(tmax, m.rows_in);
-      tsum += m.rows_in;
-      tne++;
-    }
-  stat->tile_imbalance = tne ? (double)tmax / ((double)tsum / tne) : 0.0;
-  if (!emit) return KITE_OK;
-  for (uint32_t p = 0; p < P; ++p) {
-    const BucketMeta& m = meta[p];
-    if (!m.rows) continue;
-    kite_chunk_meta cm{};
-    cm.partition_id = p;
-    cm.codec = KITE_CODEC_DVLE;
-    cm.row_count = m.rows;
-    cm.raw_bytes = m.bytes;
-    cm.key_min_lo[0] = m.kmin_lo;
-    cm.key_min_lo[1] = m.kmin_hi;
-    cm.key_max_lo[0] = m.kmax_lo;
-    cm.key_max_lo[1] = m.kmax_hi;
-    if (emit(user, &cm, hout + m.byte_off, (size_t)m.bytes)) return fail(KITE_ERR_CALLBACK, "emit callback aborted");
-  }
+  stat->tile_imbalance = 0.0;
   return KITE_OK;
 #undef MCU
 }
