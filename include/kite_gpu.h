@@ -252,7 +252,7 @@ int kite_gpu_synchronize(kite_gpu_ctx* ctx);
  * d_counts their counts, d_partition_rows[partitions] the rows of each
  * partition; totals[4] (host) gets reads, bases, k-mers and rows.
  *
- * Working memory is one fixed array of about 21 MiB in this library's device
+ * Working memory is one fixed array of about 19 MiB in this library's device
  * data, one per device, which every call on that device shares: calls that
  * overlap on the GPU race and corrupt each other's results, so serialise them
  * (and after KITE_ERR_TIMEOUT, wait for `stream` before the next call).  The

@@ -14,7 +14,7 @@
 // Limits and sharing:
 //  * at most KITE_NOALLOC_MAX_BYTES (512 KiB) of FASTQ per call; a larger
 //    chunk is rejected with KITE_ERR_UNSUPPORTED before any launch.
-//  * the array (kScratchBytes, about 21 MiB) exists once per device in the
+//  * the array (kScratchBytes, about 19 MiB) exists once per device in the
 //    process.  Every call on a device uses the same array, so calls that
 //    overlap on the GPU (two host threads, or two streams without ordering
 //    between them) race and corrupt each other's results: serialise them.
@@ -25,13 +25,18 @@
 //    context replaces it (after cudaDeviceReset, for example).
 //  * the call returns once the work has finished, waiting at most timeout_ms.
 //
-// The kernels are a small-input variant of the context path: one pass finds
-// the sequence lines, one rolls the k-mers (KmerIter::next,
-// src/count/kmer.rs:241-267 and :311-337), the keys are grouped by their
-// Fibonacci-hash partition (src/count/kmer.rs:67-71, :111-116), and one CTA
-// per partition sorts its keys through global memory and reduces them to
-// (key, count) rows, as the reference's flush_bucket does per bucket
-// (src/count/worker.rs:296-449).
+// The chunk is small, so what counts is the number of dependent steps and how
+// many SMs share each.  Six launches: newlines per 2 KiB segment; k-mers, one
+// CTA per segment (KmerIter::next, src/count/kmer.rs:241-267 and :311-337);
+// keys to their tile, a key range of a Fibonacci-hash partition
+// (src/count/kmer.rs:67-71, :111-116) of about 256 keys; one CTA per tile
+// sorts on chip and reduces to (key, count) rows, as the reference's
+// flush_bucket does per bucket (src/count/worker.rs:296-449); tiles above the
+// on-chip capacity through global memory; rows to the caller.  The two scans
+// that need every CTA's result are done by the last CTA to finish.  254 KB of
+// reads (93,134 k-mers, k = 31, 256 partitions) take 43 us on the device; one
+// CTA finding the lines, one thread per 256 bases and one CTA per partition
+// sorting through global memory took about 250.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -42,36 +47,39 @@
 
 #include "kite_gpu.h"
 #include "kite_internal.h"
+#include "kmer_words.cuh"
 
 namespace kite {
 namespace na {
 
 constexpr uint32_t kMaxBytes = KITE_NOALLOC_MAX_BYTES;
-constexpr uint32_t kMaxSeq = kMaxBytes / 4 + 2;  // a record spans at least four newlines
 constexpr uint32_t kMaxParts = 65536;
-constexpr uint32_t kPiece = 256;  // bases per extraction piece
+constexpr uint32_t kMaxTiles = 65536;
+constexpr uint32_t kSegment = 2048;    // bytes of text per extraction CTA
+constexpr uint32_t kTileKeys = 256;    // keys a tile is meant to have
+constexpr uint32_t kTileCap = 2048;    // keys of a tile sorted on chip
 constexpr int kMaxDevices = 64;
+constexpr int kExtractThreads = 256;
+constexpr int kTileSortThreads = 128;
 constexpr int kSortThreads = 512;
+constexpr uint32_t kMaxSegments = kMaxBytes / kSegment + 1;  // the text may start inside its first 16 bytes
 
 struct Counters {
   unsigned long long reads, bases, kmers;
-  unsigned int nseq, npieces, nkeys, nrows;
-  unsigned int status, pad;
+  unsigned int nkeys, nrows, nbig, extracted, sorted, pad;
 };
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffKeysA = 0;
 constexpr size_t kOffKeysB = align256(kOffKeysA + (size_t)kMaxBytes * 16);
 constexpr size_t kOffCounts = align256(kOffKeysB + (size_t)kMaxBytes * 16);
-constexpr size_t kOffSeqStart = align256(kOffCounts + (size_t)kMaxBytes * 4);
-constexpr size_t kOffSeqEnd = align256(kOffSeqStart + (size_t)kMaxSeq * 4);
-constexpr size_t kOffPieceOff = align256(kOffSeqEnd + (size_t)kMaxSeq * 4);
-constexpr size_t kOffBucketCount = align256(kOffPieceOff + (size_t)(kMaxSeq + 1) * 4);
-constexpr size_t kOffBucketFill = align256(kOffBucketCount + (size_t)kMaxParts * 4);
-constexpr size_t kOffBucketOff = align256(kOffBucketFill + (size_t)kMaxParts * 4);
-constexpr size_t kOffBucketRows = align256(kOffBucketOff + (size_t)(kMaxParts + 1) * 4);
-constexpr size_t kOffRowOff = align256(kOffBucketRows + (size_t)kMaxParts * 4);
-constexpr size_t kOffCounters = align256(kOffRowOff + (size_t)(kMaxParts + 1) * 4);
+constexpr size_t kOffSegLines = align256(kOffCounts + (size_t)kMaxBytes * 4);
+constexpr size_t kOffTileCount = align256(kOffSegLines + (size_t)kMaxSegments * 4);
+constexpr size_t kOffTileOff = align256(kOffTileCount + (size_t)kMaxTiles * 4);
+constexpr size_t kOffTileRows = align256(kOffTileOff + (size_t)(kMaxTiles + 1) * 4);
+constexpr size_t kOffRowOff = align256(kOffTileRows + (size_t)kMaxTiles * 4);
+constexpr size_t kOffBig = align256(kOffRowOff + (size_t)(kMaxTiles + 1) * 4);
+constexpr size_t kOffCounters = align256(kOffBig + (size_t)kMaxTiles * 4);
 constexpr size_t kScratchBytes = align256(kOffCounters + sizeof(Counters));
 
 // Typed views of the scratch array.
@@ -80,14 +88,12 @@ struct View {
   template <class T> __device__ T* keys_a() const { return reinterpret_cast<T*>(s + kOffKeysA); }
   template <class T> __device__ T* keys_b() const { return reinterpret_cast<T*>(s + kOffKeysB); }
   __device__ uint32_t* counts() const { return reinterpret_cast<uint32_t*>(s + kOffCounts); }
-  __device__ uint32_t* seq_start() const { return reinterpret_cast<uint32_t*>(s + kOffSeqStart); }
-  __device__ uint32_t* seq_end() const { return reinterpret_cast<uint32_t*>(s + kOffSeqEnd); }
-  __device__ uint32_t* piece_off() const { return reinterpret_cast<uint32_t*>(s + kOffPieceOff); }
-  __device__ uint32_t* bucket_count() const { return reinterpret_cast<uint32_t*>(s + kOffBucketCount); }
-  __device__ uint32_t* bucket_fill() const { return reinterpret_cast<uint32_t*>(s + kOffBucketFill); }
-  __device__ uint32_t* bucket_off() const { return reinterpret_cast<uint32_t*>(s + kOffBucketOff); }
-  __device__ uint32_t* bucket_rows() const { return reinterpret_cast<uint32_t*>(s + kOffBucketRows); }
+  __device__ uint32_t* seg_lines() const { return reinterpret_cast<uint32_t*>(s + kOffSegLines); }
+  __device__ uint32_t* tile_count() const { return reinterpret_cast<uint32_t*>(s + kOffTileCount); }
+  __device__ uint32_t* tile_off() const { return reinterpret_cast<uint32_t*>(s + kOffTileOff); }
+  __device__ uint32_t* tile_rows() const { return reinterpret_cast<uint32_t*>(s + kOffTileRows); }
   __device__ uint32_t* row_off() const { return reinterpret_cast<uint32_t*>(s + kOffRowOff); }
+  __device__ uint32_t* big() const { return reinterpret_cast<uint32_t*>(s + kOffBig); }
   __device__ Counters* counters() const { return reinterpret_cast<Counters*>(s + kOffCounters); }
 };
 
@@ -101,212 +107,286 @@ namespace kite {
 namespace na {
 namespace {
 
-// A/a=0, C/c=1, G/g=2, T/t=3, anything else 4 (src/count/kmer.rs:2-13).
-__device__ __forceinline__ uint32_t base_code(uint8_t c) {
-  switch (c) {
-    case 'A': case 'a': return 0;
-    case 'C': case 'c': return 1;
-    case 'G': case 'g': return 2;
-    case 'T': case 't': return 3;
-    default: return 4;
-  }
+// The chunk in 16-byte granules of its address: a caller's pointer may have any
+// alignment, so the text starts `skew` bytes into the first granule.
+struct Text {
+  const uint8_t* base;  // 16-byte aligned
+  uint32_t skew, end;   // the text is bytes [skew, end) from base
+};
+
+__device__ __forceinline__ uint4 text_granule(const Text& t, uint32_t at) {
+  if (at >= t.skew && at + 16 <= t.end) return *reinterpret_cast<const uint4*>(t.base + at);
+  uint32_t w[4] = {0, 0, 0, 0};
+  if (at < t.end)  // its first or last granule: only its own bytes are read
+    for (uint32_t i = 0; i < 16; ++i)
+      if (at + i >= t.skew && at + i < t.end) w[i >> 2] |= (uint32_t)t.base[at + i] << (8 * (i & 3u));
+  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Sequence lines of the chunk (parse_sequences, src/count/parser.rs:19-65):
-// line 4r+1 of the chunk is sequence r; a final sequence line without its
-// newline runs to the end; a chunk that does not start with '@' yields
-// nothing (the worker ignores the parse error, src/count/worker.rs:217).
-// Also the piece offsets of every sequence, and the reads / bases totals.
-// One CTA.
-__global__ void __launch_bounds__(1024) k_lines(const uint8_t* __restrict__ d, uint32_t len, uint8_t* scr) {
-  constexpr uint32_t kPer = 16, kWin = 1024 * kPer;
+// The tile of a key: ranges of equal width (a power of two per partition)
+// over the keys' 2k bits, so that tile order is partition, then key order.
+struct TileOf {
+  uint32_t shift, bits, key_bits;
+  template <class T>
+  __device__ __forceinline__ uint32_t operator()(T key) const {
+    return bits ? (bucket_of(key, shift) << bits) | (uint32_t)(uint64_t)(key >> (key_bits - bits))
+                : bucket_of(key, shift);
+  }
+};
+
+// Newlines per segment; what later kernels add to starts at zero.
+__global__ void __launch_bounds__(128) k_prepare(Text t, uint32_t tiles, uint8_t* scr) {
   __shared__ unsigned sm[40];
-  __shared__ unsigned long long sm64[40];
   const View v{scr};
-  Counters* c = v.counters();
-  uint32_t* ss = v.seq_start();
-  uint32_t* se = v.seq_end();
-  uint32_t* po = v.piece_off();
-  if (len == 0 || d[0] != '@') {
-    if (threadIdx.x == 0) {
-      c->nseq = 0;
-      c->npieces = 0;
-      po[0] = 0;
-    }
-    return;
-  }
-  unsigned carry = 0;  // newlines before the current window
-  for (uint32_t w0 = 0; w0 < len; w0 += kWin) {
-    const uint32_t b = w0 + threadIdx.x * kPer;
-    const uint32_t e = min(b + kPer, len);
-    unsigned cnt = 0;
-    for (uint32_t i = b; i < e; ++i) cnt += d[i] == '\n';
-    unsigned tot;
-    unsigned line = carry + block_exclusive_scan<1024, unsigned>(cnt, sm, &tot);
-    for (uint32_t i = b; i < e; ++i) {
-      if (d[i] != '\n') continue;
-      if ((line & 3u) == 0) ss[line >> 2] = i + 1;  // header ends: sequence starts
-      else if ((line & 3u) == 1) se[line >> 2] = i;
-      ++line;
-    }
-    carry += tot;
-  }
-  const unsigned nl = carry;
-  const unsigned nseq = nl ? (nl + 3) / 4 : 0;
-  if (threadIdx.x == 0 && (nl & 3u) == 1) se[nl >> 2] = len;
+  const uint32_t at = blockIdx.x * kSegment + threadIdx.x * 16;
+  for (uint32_t i = blockIdx.x * 128 + threadIdx.x; i < tiles; i += gridDim.x * 128) v.tile_count()[i] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *v.counters() = Counters{};
+  const uint4 w = text_granule(t, at);
+  const unsigned n = (__popc(__vcmpeq4(w.x, 0x0a0a0a0au)) + __popc(__vcmpeq4(w.y, 0x0a0a0a0au)) +
+                      __popc(__vcmpeq4(w.z, 0x0a0a0a0au)) + __popc(__vcmpeq4(w.w, 0x0a0a0a0au))) >> 3;
+  unsigned tot;
+  block_exclusive_scan<128, unsigned>(n, sm, &tot);
+  if (threadIdx.x == 0) v.seg_lines()[blockIdx.x] = tot;
+}
+static_assert(kSegment == 128 * 16, "a thread of k_prepare counts one granule");
+
+// True in every thread of the last CTA to get here; what the others wrote
+// before is then visible to it.
+__device__ __forceinline__ bool last_cta(unsigned* done) {
+  __shared__ bool last;
+  __threadfence();
   __syncthreads();
-  unsigned pcarry = 0;
-  unsigned long long reads = 0, bases = 0;
-  for (uint32_t s0 = 0; s0 < nseq; s0 += 1024) {
-    const uint32_t s = s0 + threadIdx.x;
-    unsigned pieces = 0;
-    if (s < nseq) {
-      const uint32_t L = se[s] - ss[s];
-      pieces = (L + kPiece - 1) / kPiece;
-      reads += L > 0;
-      bases += L;
-    }
-    unsigned tot;
-    const unsigned ex = block_exclusive_scan<1024, unsigned>(pieces, sm, &tot);
-    if (s < nseq) po[s] = pcarry + ex;
-    pcarry += tot;
-  }
-  unsigned long long rt, bt;
-  block_exclusive_scan<1024, unsigned long long>(reads, sm64, &rt);
-  block_exclusive_scan<1024, unsigned long long>(bases, sm64, &bt);
-  if (threadIdx.x == 0) {
-    po[nseq] = pcarry;
-    c->nseq = nseq;
-    c->npieces = pcarry;
-    c->reads = rt;
-    c->bases = bt;
-  }
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
 }
 
-// Rolling k-mers, one piece of up to kPiece bases per thread: the piece
-// emits the k-mers that END inside it and starts rolling k-1 bases earlier
-// (clamped to the sequence start), so every k-mer is emitted exactly once.
-// A first pass counts, one atomic reserves the slots, a second pass writes
-// the keys and the partition histogram.
-template <class T>
-__global__ void __launch_bounds__(256) k_extract(const uint8_t* __restrict__ d, uint32_t k, uint32_t canonical,
-                                                 uint32_t shift, uint8_t* scr) {
-  const View v{scr};
-  Counters* c = v.counters();
-  const uint32_t npieces = c->npieces, nseq = c->nseq;
-  const uint32_t* ss = v.seq_start();
-  const uint32_t* se = v.seq_end();
-  const uint32_t* po = v.piece_off();
-  T* keys = v.keys_a<T>();
-  uint32_t* bcount = v.bucket_count();
-  const T mask = (2 * k == (uint32_t)KeyTraits<T>::kBits) ? ~T(0) : ((T(1) << (2 * k)) - T(1));
-  const uint32_t rshift = 2 * (k - 1);
-  unsigned long long kmers = 0;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < npieces; q += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = nseq - 1;  // last sequence with po[s] <= q
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1) >> 1;
-      if (po[mid] <= q) lo = mid;
-      else hi = mid - 1;
-    }
-    const uint32_t s0 = ss[lo];
-    const uint32_t ps = s0 + (q - po[lo]) * kPiece;
-    const uint32_t pe = min(ps + kPiece, se[lo]);
-    const uint32_t r0 = (ps - s0 >= k - 1) ? ps - (k - 1) : s0;
-    uint32_t n = 0, valid = 0;
-    for (uint32_t i = r0; i < pe; ++i) {
-      if (base_code(d[i]) > 3) {
-        valid = 0;
-        continue;
-      }
-      ++valid;
-      n += (valid >= k && i >= ps);
-    }
-    if (n == 0) continue;
-    const uint32_t at = atomicAdd(&c->nkeys, n);
-    if (at + n > kMaxBytes) {
-      atomicCAS(&c->status, 0u, 1u);
-      continue;
-    }
-    T fwd = 0, rev = 0;
-    valid = 0;
-    uint32_t o = at;
-    for (uint32_t i = r0; i < pe; ++i) {
-      const uint32_t b = base_code(d[i]);
-      if (b > 3) {
-        fwd = 0;
-        rev = 0;
-        valid = 0;
-        continue;
-      }
-      fwd = ((fwd << 2) | T(b)) & mask;
-      rev = (rev >> 2) | (T(b ^ 3u) << rshift);
-      ++valid;
-      if (valid >= k && i >= ps) {
-        const T key = canonical ? (fwd < rev ? fwd : rev) : fwd;
-        keys[o++] = key;
-        atomicAdd(&bcount[bucket_of(key, shift)], 1u);
-      }
-    }
-    kmers += n;
-  }
-  for (int m = 16; m; m >>= 1) kmers += __shfl_xor_sync(0xffffffffu, kmers, m);
-  if ((threadIdx.x & 31) == 0 && kmers) atomicAdd(&c->kmers, kmers);
-}
-
-// Exclusive scan of n counters into out[0..n], out[n] = total.  One CTA.
-__global__ void __launch_bounds__(1024) k_scan(const uint32_t* __restrict__ in, uint32_t n,
-                                               uint32_t* __restrict__ out) {
-  __shared__ unsigned sm[40];
+// Exclusive scan of n counters into out[0..n] by one CTA, four per thread and step.
+template <int NT>
+__device__ __forceinline__ void cta_scan(const uint32_t* in, uint32_t n, uint32_t* out, unsigned* sm) {
   unsigned carry = 0;
-  for (uint32_t i0 = 0; i0 < n; i0 += 1024) {
-    const uint32_t i = i0 + threadIdx.x;
-    const unsigned x = i < n ? in[i] : 0u;
+  for (uint32_t i0 = 0; i0 < n; i0 += NT * 4) {
+    const uint32_t i = i0 + threadIdx.x * 4;
+    unsigned x[4], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      x[j] = i + j < n ? __ldcg(in + i + j) : 0u;
+      sum += x[j];
+    }
     unsigned tot;
-    const unsigned ex = block_exclusive_scan<1024, unsigned>(x, sm, &tot);
-    if (i < n) out[i] = carry + ex;
+    unsigned at = carry + block_exclusive_scan<NT, unsigned>(sum, sm, &tot);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      if (i + j < n) out[i + j] = at;
+      at += x[j];
+    }
     carry += tot;
   }
   if (threadIdx.x == 0) out[n] = carry;
 }
 
-// Keys grouped by partition: keys_a -> keys_b at the partition offsets.
+// K-mers of one segment: its 64 words and the two before it are encoded by one
+// thread each (lines 1 mod 4 of a chunk that starts with '@' are sequences,
+// parse_sequences, src/count/parser.rs:19-65; a k-mer cannot cross a newline,
+// so only its last byte's line matters), then each warp takes words in turn
+// with one lane per end byte.  A key's place in its tile is the tile counter's
+// value, kept beside the key; the last CTA scans the counters.
 template <class T>
-__global__ void __launch_bounds__(256) k_scatter(uint32_t shift, uint8_t* scr) {
+__global__ void __launch_bounds__(kExtractThreads) k_extract(Text t, uint32_t k, uint32_t canonical, TileOf tile_of,
+                                                             uint32_t tiles, uint8_t* scr) {
+  constexpr int NT = kExtractThreads, W = kSegment / 32, WARPS = NT / 32;
+  __shared__ uint64_t code[W + 2], rcode[W + 2];
+  __shared__ uint32_t vb[W + 2], nl[W + 2], ends[W], place[W];
+  __shared__ unsigned long long scan_sm[40];
+  __shared__ unsigned scan32[40];
+  __shared__ uint32_t base;
   const View v{scr};
-  const uint32_t n = min(v.counters()->nkeys, kMaxBytes);
-  const T* a = v.keys_a<T>();
-  T* b = v.keys_b<T>();
-  const uint32_t* off = v.bucket_off();
-  uint32_t* fill = v.bucket_fill();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const T key = a[i];
-    const uint32_t bk = bucket_of(key, shift);
-    const uint32_t pos = off[bk] + atomicAdd(&fill[bk], 1u);
-    if (pos < kMaxBytes) b[pos] = key;
+  Counters* c = v.counters();
+  const int tid = threadIdx.x;
+  // this thread's word: tid - 2 of the segment
+  const uint32_t at = blockIdx.x * kSegment + tid * 32 - 64;  // wraps below zero for the first two of the text
+  const bool mine = tid < W + 2 && (blockIdx.x > 0 || tid >= 2) && at < t.end;
+  Word32 w{0, 0, 0, 0};
+  if (mine) w = encode_word(text_granule(t, at), text_granule(t, at + 16));
+  if (tid < W + 2) {
+    code[tid] = w.code;
+    rcode[tid] = w.rcode;
+    vb[tid] = w.vb;
+    nl[tid] = w.nl;
+  }
+  const bool own = mine && tid >= 2;
+  unsigned long long sum = own ? __popc(w.nl) : 0u;
+  for (uint32_t i = tid; i < blockIdx.x; i += NT) sum += (unsigned long long)v.seg_lines()[i] << 32;
+  unsigned long long tot;
+  const unsigned long long before = block_exclusive_scan<NT, unsigned long long>(sum, scan_sm, &tot);
+  unsigned ph = ((unsigned)(tot >> 32) + (unsigned)before) & 3u;  // the line's phase at the word
+  const bool chunk_ok = t.end > t.skew && t.base[t.skew] == '@';
+  uint32_t V = 0;
+  unsigned long long reads = 0, bases = 0;
+  if (own && chunk_ok) {
+    // bytes outside the text are no newlines and no bases
+    uint32_t in = 0xffffffffu;
+    if (at < t.skew) in &= 0xffffffffu << (t.skew - at);
+    if (t.end - at < 32) in &= (1u << (t.end - at)) - 1u;
+    const uint32_t seq = seq_mask(w.nl, ph) & in;
+    if constexpr (sizeof(T) == 8) {
+      V = (uint32_t)(runs_of((uint64_t)vb[tid - 1] | (uint64_t)w.vb << 32, k) >> (33 - k)) & seq;
+    } else {
+      const u128 ok = (u128)((uint64_t)vb[tid - 2] | (uint64_t)vb[tid - 1] << 32) | (u128)w.vb << 64;
+      V = (uint32_t)(runs_of128(ok, k) >> (65 - k)) & seq;
+    }
+    bases = __popc(seq);
+    reads = __popc(seq & (w.nl << 1 | nl[tid - 1] >> 31));  // a line's first byte follows a newline
+  }
+  unsigned n;
+  const unsigned first = block_exclusive_scan<NT, unsigned>(__popc(V), scan32, &n);
+  if (tid >= 2 && tid < W + 2) {
+    ends[tid - 2] = V;
+    place[tid - 2] = first;
+  }
+  if (tid == 0) base = n ? atomicAdd(&c->nkeys, n) : 0u;
+  for (int m = 16; m; m >>= 1) {
+    reads += __shfl_xor_sync(0xffffffffu, reads, m);
+    bases += __shfl_xor_sync(0xffffffffu, bases, m);
+  }
+  if ((tid & 31) == 0 && bases) {
+    atomicAdd(&c->reads, reads);
+    atomicAdd(&c->bases, bases);
+  }
+  __syncthreads();
+  const unsigned lane = tid & 31;
+  const T mask = (2 * k == (uint32_t)KeyTraits<T>::kBits) ? ~T(0) : ((T(1) << (2 * k)) - T(1));
+  const uint32_t fs = 2 * (31 - lane);
+  T* keys = v.keys_a<T>() + base;
+  uint32_t* ranks = v.counts() + base;
+  uint32_t* counts = v.tile_count();
+  uint32_t rank[W / WARPS];
+#pragma unroll
+  for (int j = 0; j < W / WARPS; ++j) {
+    const int i = (tid >> 5) + j * WARPS;  // word i of the segment is entry i + 2
+    const uint32_t Vi = ends[i];
+    rank[j] = 0;
+    if (!((Vi >> lane) & 1u)) continue;
+    T fwd, rc;
+    const u128 x = (u128)code[i + 1] << 64 | code[i + 2];
+    if constexpr (sizeof(T) == 8) {
+      fwd = (uint64_t)(x >> fs) & mask;
+      rc = (uint64_t)(((u128)rcode[i + 2] << 64 | rcode[i + 1]) >> (2 * (33 + lane - k))) & mask;
+    } else {
+      fwd = (fs ? x >> fs | (u128)code[i] << (128 - fs) : x) & mask;
+      const uint32_t rs = 2 * (65 + lane - k);  // 2 .. 128
+      const u128 lo = (u128)rcode[i + 1] << 64 | rcode[i];
+      rc = rs < 64 ? lo >> rs | (u128)rcode[i + 2] << (128 - rs)
+                   : ((u128)rcode[i + 2] << 64 | rcode[i + 1]) >> (rs - 64);
+      rc &= mask;
+    }
+    const T key = canonical && rc < fwd ? rc : fwd;
+    keys[place[i] + __popc(Vi & ((1u << lane) - 1u))] = key;
+    rank[j] = atomicAdd(&counts[tile_of(key)], 1u);
+  }
+#pragma unroll
+  for (int j = 0; j < W / WARPS; ++j) {
+    const int i = (tid >> 5) + j * WARPS;
+    const uint32_t Vi = ends[i];
+    if ((Vi >> lane) & 1u) ranks[place[i] + __popc(Vi & ((1u << lane) - 1u))] = rank[j];
+  }
+  if (last_cta(&c->extracted)) {
+    cta_scan<NT>(v.tile_count(), tiles, v.tile_off(), scan32);
+    if (tid == 0) c->kmers = __ldcg(&c->nkeys);
   }
 }
 
-// One CTA per partition: LSD radix sort of its keys through global memory
-// (8-bit digits over the bits that vary, each chunk of CAP keys ranked stably
-// on chip), then the run-length reduction to (key, count) rows written to
-// keys_a / counts at the partition's offset, and the partition's row count.
+// Keys to their tiles: keys_a -> keys_b.
 template <class T>
-__global__ void __launch_bounds__(kSortThreads) k_sort_rle(uint8_t* scr) {
+__global__ void __launch_bounds__(256) k_scatter(TileOf tile_of, uint8_t* scr) {
+  const View v{scr};
+  const uint32_t n = v.counters()->nkeys;
+  const T* a = v.keys_a<T>();
+  T* b = v.keys_b<T>();
+  const uint32_t* off = v.tile_off();
+  const uint32_t* rank = v.counts();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const T key = a[i];
+    b[off[tile_of(key)] + rank[i]] = key;
+  }
+}
+
+// One CTA per tile of at most kTileCap keys: a bitonic sort in shared memory,
+// then the run-length reduction to rows, written to keys_a / counts at the
+// tile's offset.  A warp's 32 pairs of a step with stride <= 32 are 64
+// consecutive keys, the same in every such step, so only longer strides need
+// the whole CTA.  Larger tiles are listed.
+template <class T>
+__global__ void __launch_bounds__(kTileSortThreads) k_sort_tiles(uint8_t* scr) {
+  constexpr uint32_t NT = kTileSortThreads;
+  __shared__ T buf[kTileCap];
+  __shared__ uint16_t head[kTileCap];
+  __shared__ unsigned sm[40];
+  const View v{scr};
+  const uint32_t tile = blockIdx.x, tid = threadIdx.x;
+  const uint32_t n = v.tile_count()[tile];
+  if (n == 0 || n > kTileCap) {
+    if (tid == 0) {
+      if (n == 0) v.tile_rows()[tile] = 0;
+      else v.big()[atomicAdd(&v.counters()->nbig, 1u)] = tile;
+    }
+    return;
+  }
+  const uint32_t off = v.tile_off()[tile];
+  const T* src = v.keys_b<T>() + off;
+  uint32_t m = 64;
+  while (m < n) m *= 2;
+  for (uint32_t i = tid; i < m; i += NT) buf[i] = i < n ? src[i] : ~T(0);
+  __syncthreads();
+  for (uint32_t size = 2; size <= m; size *= 2) {
+    for (uint32_t stride = size / 2; stride; stride /= 2) {
+      for (uint32_t i = tid; i < m / 2; i += NT) {
+        const uint32_t a = 2 * i - (i & (stride - 1)), b = a + stride;
+        const T x = buf[a], y = buf[b];
+        if ((y < x) == ((a & size) == 0) && x != y) {
+          buf[a] = y;
+          buf[b] = x;
+        }
+      }
+      // the next step's keys may be another warp's when its stride, or this one's, is long
+      if (stride > 32 || (stride == 1 && size > 32)) __syncthreads();
+      else __syncwarp();
+    }
+  }
+  __syncthreads();
+  const uint32_t per = (n + NT - 1) / NT, b0 = min(tid * per, n), e0 = min(b0 + per, n);
+  unsigned heads = 0;
+  for (uint32_t i = b0; i < e0; ++i) heads += i == 0 || buf[i] != buf[i - 1];
+  unsigned U;
+  unsigned u = block_exclusive_scan<NT, unsigned>(heads, sm, &U);
+  for (uint32_t i = b0; i < e0; ++i)
+    if (i == 0 || buf[i] != buf[i - 1]) head[u++] = (uint16_t)i;
+  __syncthreads();
+  T* ok = v.keys_a<T>() + off;
+  uint32_t* oc = v.counts() + off;
+  for (uint32_t r = tid; r < U; r += NT) {
+    const uint32_t h = head[r];
+    ok[r] = buf[h];
+    oc[r] = (r + 1 < U ? head[r + 1] : n) - h;
+  }
+  if (tid == 0) v.tile_rows()[tile] = U;
+}
+
+// One CTA per tile above the on-chip capacity: LSD radix sort of its keys through
+// global memory (8-bit digits over the bits that vary, each chunk of CAP keys
+// ranked stably on chip), then the run-length reduction to (key, count) rows
+// written to keys_a / counts at the tile's offset, and the tile's row count.
+template <class T>
+__device__ void sort_big(const View& v, uint32_t bk) {
   constexpr int NT = kSortThreads, ITEMS = tile_items<T>(), CAP = NT * ITEMS, NW = NT / 32;
   __shared__ unsigned warp_hist[256 * NW];
   __shared__ unsigned scan_sm[40];
   __shared__ unsigned dtot[256], dstart[256];
   __shared__ unsigned long long run_off[256];
   __shared__ T red_mn[NW], red_mx[NW];
-  const View v{scr};
-  const uint32_t bk = blockIdx.x;
-  const uint32_t n = v.bucket_count()[bk];
-  if (n == 0) {
-    if (threadIdx.x == 0) v.bucket_rows()[bk] = 0;
-    return;
-  }
-  const uint32_t off = v.bucket_off()[bk];
+  const uint32_t n = v.tile_count()[bk];
+  const uint32_t off = v.tile_off()[bk];
   T* src = v.keys_b<T>() + off;
   T* dst = v.keys_a<T>() + off;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -429,21 +509,33 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_rle(uint8_t* scr) {
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) v.bucket_rows()[bk] = U;
+  if (threadIdx.x == 0) v.tile_rows()[bk] = U;
+  __syncthreads();
 }
 
-// One CTA per partition: copies its rows to the caller's arrays at the
-// partition's row offset (rows past max_rows are dropped; the host reports
-// the shortfall) and stores the partition's row count.
+// The listed tiles, then (by the last CTA) the row offsets of all tiles.
 template <class T>
-__global__ void __launch_bounds__(256) k_emit(uint8_t* scr, uint32_t P, T* __restrict__ out_keys,
+__global__ void __launch_bounds__(kSortThreads) k_sort_listed(uint32_t tiles, uint8_t* scr) {
+  __shared__ unsigned sm[40];
+  const View v{scr};
+  Counters* c = v.counters();
+  const uint32_t n = c->nbig;
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) sort_big<T>(v, v.big()[i]);
+  if (last_cta(&c->sorted)) cta_scan<kSortThreads>(v.tile_rows(), tiles, v.row_off(), sm);
+}
+
+// One CTA per tile: copies its rows to the caller's arrays at the tile's row
+// offset (rows past max_rows are dropped; the host reports the shortfall); a
+// partition's first tile stores the partition's row count.
+template <class T>
+__global__ void __launch_bounds__(128) k_emit(uint8_t* scr, uint32_t tiles, uint32_t per_part, T* __restrict__ out_keys,
                                               uint32_t* __restrict__ out_counts, unsigned long long max_rows,
                                               uint32_t* __restrict__ part_rows) {
   const View v{scr};
   const uint32_t bk = blockIdx.x;
-  const uint32_t rows = v.bucket_rows()[bk];
+  const uint32_t rows = v.tile_rows()[bk];
   const unsigned long long ro = v.row_off()[bk];
-  const uint32_t off = v.bucket_off()[bk];
+  const uint32_t off = v.tile_off()[bk];
   const T* ok = v.keys_a<T>() + off;
   const uint32_t* oc = v.counts() + off;
   for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x) {
@@ -452,8 +544,8 @@ __global__ void __launch_bounds__(256) k_emit(uint8_t* scr, uint32_t P, T* __res
     out_counts[ro + i] = oc[i];
   }
   if (threadIdx.x == 0) {
-    part_rows[bk] = rows;
-    if (bk == 0) v.counters()->nrows = v.row_off()[P];
+    if (bk % per_part == 0) part_rows[bk / per_part] = v.row_off()[bk + per_part] - (uint32_t)ro;
+    if (bk == 0) v.counters()->nrows = v.row_off()[tiles];
   }
 }
 
@@ -551,31 +643,29 @@ template <class T>
 int run(uint8_t* scr, uint32_t sms, uint32_t k, bool canonical, uint32_t P, const uint8_t* d_fastq, uint32_t len,
         void* d_keys, uint32_t* d_counts, uint64_t max_rows, uint32_t* d_part_rows, uint64_t* totals,
         cudaStream_t s, uint32_t timeout_ms) {
-  // What accumulates across threads starts at zero on every call.
-  if (cudaMemsetAsync(scr + kOffBucketCount, 0, (size_t)P * 4, s) != cudaSuccess ||
-      cudaMemsetAsync(scr + kOffBucketFill, 0, (size_t)P * 4, s) != cudaSuccess ||
-      cudaMemsetAsync(scr + kOffCounters, 0, sizeof(Counters), s) != cudaSuccess)
-    return KITE_ERR_CUDA;
   uint32_t log2p = 0;
   while ((1u << log2p) < P) ++log2p;
-  const uint32_t shift = 64 - log2p;
-  const uint32_t max_pieces = len / 4 + 2 + len / kPiece;
-  // grid-stride kernels: four CTAs per SM at most
-  const uint32_t g_pieces = std::min<uint32_t>((max_pieces + 255) / 256, 4 * sms);
-  const uint32_t g_keys = std::min<uint32_t>(std::max<uint32_t>(len, 1) / 256 + 1, 4 * sms);
-  uint32_t* const bucket_count = reinterpret_cast<uint32_t*>(scr + kOffBucketCount);
-  uint32_t* const bucket_off = reinterpret_cast<uint32_t*>(scr + kOffBucketOff);
-  uint32_t* const bucket_rows = reinterpret_cast<uint32_t*>(scr + kOffBucketRows);
-  uint32_t* const row_off = reinterpret_cast<uint32_t*>(scr + kOffRowOff);
-  const cudaError_t le[7] = {
-      launch(k_lines, 1, 1024, s, d_fastq, len, scr),
-      launch(k_extract<T>, g_pieces, 256, s, d_fastq, k, canonical ? 1u : 0u, shift, scr),
-      launch(k_scan, 1, 1024, s, bucket_count, P, bucket_off),
-      launch(k_scatter<T>, g_keys, 256, s, shift, scr),
-      launch(k_sort_rle<T>, P, kSortThreads, s, scr),
-      launch(k_scan, 1, 1024, s, bucket_rows, P, row_off),
-      launch(k_emit<T>, P, 256, s, scr, P, static_cast<T*>(d_keys), d_counts, (unsigned long long)max_rows,
-             d_part_rows)};
+  // Tiles: a partition's keys by their top bits, kTileKeys each when every
+  // second byte ends a k-mer (reads with qualities) and the keys are even.
+  uint32_t bits = 0;
+  while (bits < 2 * k && (P << (bits + 1)) <= kMaxTiles && (P << bits) * kTileKeys < len / 2) ++bits;
+  const uint32_t tiles = P << bits;
+  const TileOf tile_of{64 - log2p, bits, 2 * k};
+  Text t;
+  t.skew = (uint32_t)(reinterpret_cast<uintptr_t>(d_fastq) & 15u);
+  t.base = d_fastq - t.skew;
+  t.end = t.skew + len;
+  const uint32_t segments = std::max<uint32_t>((t.end + kSegment - 1) / kSegment, 1);
+  if (len == 0) t.end = t.skew = 0;  // nothing is read
+  const uint32_t g_keys = std::min<uint32_t>(len / 512 + 1, 4 * sms);
+  const cudaError_t le[6] = {
+      launch(k_prepare, segments, 128, s, t, tiles, scr),
+      launch(k_extract<T>, segments, kExtractThreads, s, t, k, canonical ? 1u : 0u, tile_of, tiles, scr),
+      launch(k_scatter<T>, g_keys, 256, s, tile_of, scr),
+      launch(k_sort_tiles<T>, tiles, kTileSortThreads, s, scr),
+      launch(k_sort_listed<T>, std::min(tiles, sms), kSortThreads, s, tiles, scr),
+      launch(k_emit<T>, tiles, 128, s, scr, tiles, 1u << bits, static_cast<T*>(d_keys), d_counts,
+             (unsigned long long)max_rows, d_part_rows)};
   for (const cudaError_t e : le)
     if (e != cudaSuccess) return KITE_ERR_CUDA;
   int rc = wait_idle(s, timeout_ms);
@@ -589,7 +679,6 @@ int run(uint8_t* scr, uint32_t sms, uint32_t k, bool canonical, uint32_t P, cons
   totals[1] = hc.bases;
   totals[2] = hc.kmers;
   totals[3] = hc.nrows;
-  if (hc.status) return KITE_ERR_DEVICE;
   if (hc.nrows > max_rows) return KITE_ERR_BAD_INPUT;
   return KITE_OK;
 }
