@@ -151,15 +151,12 @@ int fail(kite_gpu_ctx* c, int code, const std::string& msg) {
 // Bounded wait for all work queued on `s`.
 // Waits (bounded by cfg.timeout_ms) for a recorded event.
 int wait_event(kite_gpu_ctx* ctx, cudaEvent_t e) {
-  const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(ctx->cfg.timeout_ms);
-  int spins = 0;
+  PollPause pause(ctx->cfg.timeout_ms);
   for (;;) {
     cudaError_t q = cudaEventQuery(e);
     if (q == cudaSuccess) return KITE_OK;
     if (q != cudaErrorNotReady) return fail(ctx, KITE_ERR_CUDA, std::string("stream wait: ") + cudaGetErrorString(q));
-    if (std::chrono::steady_clock::now() > deadline)
-      return fail(ctx, KITE_ERR_TIMEOUT, "device work did not finish within timeout_ms");
-    if (++spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(50));
+    if (!pause()) return fail(ctx, KITE_ERR_TIMEOUT, "device work did not finish within timeout_ms");
   }
 }
 

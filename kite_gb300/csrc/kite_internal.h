@@ -2,9 +2,11 @@
 // the kernel translation units.  Not part of the public ABI.
 #pragma once
 
+#include <chrono>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <thread>
 
 #include "kite_common.cuh"
 
@@ -176,6 +178,28 @@ int count_matrix_offsets(unsigned* m, uint32_t rows, uint32_t cols, unsigned lon
 int bounded_sync(cudaStream_t s, uint32_t timeout_ms);
 // Waits for one recorded event: 0, -1 (CUDA error) or -3 (timeout).
 int bounded_event_wait(cudaEvent_t e, uint32_t timeout_ms);
+
+// The pause between two polls of a bounded host wait.  A sleep of 50 us takes
+// 100 and more, as long as a small call's whole device work: a wait polls for
+// its first millisecond and sleeps between polls after that.  (Sleeping after
+// 64 polls, 2,000 reads counted on the device took 770 us with 99 us of device
+// work, 594 us without the sleeps.)
+class PollPause {
+ public:
+  explicit PollPause(uint32_t timeout_ms)
+      : start_(std::chrono::steady_clock::now()), limit_(std::chrono::milliseconds(timeout_ms)) {}
+  // False when the wait has run out.
+  bool operator()() {
+    const auto waited = std::chrono::steady_clock::now() - start_;
+    if (waited > limit_) return false;
+    if (waited > std::chrono::milliseconds(1)) std::this_thread::sleep_for(std::chrono::microseconds(50));
+    return true;
+  }
+
+ private:
+  std::chrono::steady_clock::time_point start_;
+  std::chrono::steady_clock::duration limit_;
+};
 
 // ---- sort_kernels.cu ----
 constexpr int kTileThreads = 512;

@@ -38,10 +38,8 @@
 // CTA finding the lines, one thread per 256 bases and one CTA per partition
 // sorting through global memory took about 250.
 #include <algorithm>
-#include <chrono>
 #include <cstring>
 #include <mutex>
-#include <thread>
 #include <tuple>
 #include <utility>
 
@@ -629,13 +627,12 @@ cudaError_t launch(void (*f)(KArgs...), dim3 g, dim3 b, cudaStream_t s, Args... 
 
 // Polls the stream until its work is done; no event or other object is made.
 int wait_idle(cudaStream_t s, uint32_t timeout_ms) {
-  const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms);
-  for (int spins = 0;; ++spins) {
+  PollPause pause(timeout_ms);
+  for (;;) {
     const cudaError_t q = cudaStreamQuery(s);
     if (q == cudaSuccess) return KITE_OK;
     if (q != cudaErrorNotReady) return KITE_ERR_CUDA;
-    if (std::chrono::steady_clock::now() > deadline) return KITE_ERR_TIMEOUT;
-    if (spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(50));
+    if (!pause()) return KITE_ERR_TIMEOUT;
   }
 }
 

@@ -1,7 +1,5 @@
 // Device-wide exclusive prefix sum over u64 (reduce-then-scan, no inter-CTA
 // waiting).  Used for bucket/tile region offsets and newline prefixes.
-#include <chrono>
-#include <thread>
 
 #include "kite_internal.h"
 
@@ -152,22 +150,13 @@ int bounded_sync(cudaStream_t s, uint32_t timeout_ms) {
 }
 
 int bounded_event_wait(cudaEvent_t e, uint32_t timeout_ms) {
-  const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms);
-  int rc = 0;
-  for (int spins = 0;; ++spins) {
+  PollPause pause(timeout_ms);
+  for (;;) {
     const cudaError_t q = cudaEventQuery(e);
-    if (q == cudaSuccess) break;
-    if (q != cudaErrorNotReady) {
-      rc = -1;
-      break;
-    }
-    if (std::chrono::steady_clock::now() > deadline) {
-      rc = -3;
-      break;
-    }
-    if (spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(50));
+    if (q == cudaSuccess) return 0;
+    if (q != cudaErrorNotReady) return -1;
+    if (!pause()) return -3;
   }
-  return rc;
 }
 
 }  // namespace kite
