@@ -14,7 +14,7 @@ namespace kite {
 // Pinned host staging of at least the given bytes (nullptr if it cannot be had).
 using StagingFn = std::function<uint8_t*(size_t)>;
 
-// Modes of merge_run (the merge kernel's kModeMerge / kModeDump / kModeHisto / kModeRows).
+// Modes of merge_run (the merge kernel's kModeMerge / kModeDump / kModeHisto / kModeQuery).
 enum : int { kMergeModeMerge = 0, kMergeModeDump = 1, kMergeModeHisto = 2, kMergeModeQuery = 3 };
 
 // Device buffers of the merge path kept by a context across calls (grown,
@@ -25,7 +25,7 @@ struct MergePoolSlot {
   size_t cap = 0;
 };
 struct MergePool {
-  static constexpr int kSlots = 34;
+  static constexpr int kSlots = 35;
   MergePoolSlot slot[kSlots];
   MergePoolSlot host;     // pinned host memory: the tile stream lists on their way to the device
   MergePoolSlot records;  // pinned host memory: a merge's partition records

@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "merge.h"
+#include "key_table.cuh"
 #include "kite_internal.h"
 #include "splitters.h"
 
@@ -645,11 +646,11 @@ struct MergeSmem {
 // apply_reader_filter_to_rows on it, then the count's frequency; no rows
 // written).
 template <class T, int MODE>
-__global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
-    const T* __restrict__ keys, const unsigned long long* __restrict__ counts, const MergeTile* __restrict__ tiles,
-    const TileStream* __restrict__ ts, const InputFilter* __restrict__ filt, T* __restrict__ out_keys,
-    uint32_t* __restrict__ out_counts, TileOut<T>* __restrict__ tout, unsigned long long* __restrict__ overflow,
-    DevStatus* st, MergeAux aux) {
+__device__ __forceinline__ void merge_tile(
+    const uint32_t tile, const T* __restrict__ keys, const unsigned long long* __restrict__ counts,
+    const MergeTile* __restrict__ tiles, const TileStream* __restrict__ ts, const InputFilter* __restrict__ filt,
+    T* __restrict__ out_keys, uint32_t* __restrict__ out_counts, TileOut<T>* __restrict__ tout,
+    unsigned long long* __restrict__ overflow, DevStatus* st, const MergeAux& aux) {
   constexpr bool DUMP = MODE == kModeDump;
   using L = MergeSmem<T>;
   constexpr int NT = kMergeThreads;
@@ -666,17 +667,17 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
   unsigned long long* misc = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(sstart) + L::seg);
   unsigned* hbin = reinterpret_cast<unsigned*>(reinterpret_cast<uint8_t*>(misc) + L::misc);
 
-  const MergeTile mt = tiles[blockIdx.x];
+  const MergeTile mt = tiles[tile];
   const uint32_t nts = mt.nts, n = mt.rows_in;
   if (n == 0 || nts == 0) {
     if (threadIdx.x == 0) {
       TileOut<T> o{};
-      tout[blockIdx.x] = o;
+      tout[tile] = o;
     }
     return;
   }
   if (n > kMergeCap || nts > kMaxTileStreams) {
-    dev_fail(st, KITE_DEV_TILE_OVERFLOW, blockIdx.x, n, nts);
+    dev_fail(st, KITE_DEV_TILE_OVERFLOW, tile, n, nts);
     return;
   }
   if (threadIdx.x < 32) {
@@ -875,7 +876,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
         }
       } else {
         if (MODE == kModeMerge && total > 0xffffffffull)
-          atomicMin(overflow, ((unsigned long long)blockIdx.x << 32) | (unsigned long long)o);
+          atomicMin(overflow, ((unsigned long long)tile << 32) | (unsigned long long)o);
         const uint32_t c32 = total > 0xffffffffull ? 0xffffffffu : (uint32_t)total;
         out_keys[mt.out_off + o] = gkey[i];
         out_counts[mt.out_off + o] = c32;
@@ -918,7 +919,330 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
     o.rows = (uint32_t)out_base;
     o.first_count = first_count;
     o.rest_bytes = rest_total;
-    tout[blockIdx.x] = o;
+    tout[tile] = o;
+  }
+}
+
+// One tile per CTA, or (list) the listed ones in turn.
+template <class T, int MODE>
+__global__ void __launch_bounds__(kMergeThreads) k_merge_tiles(
+    const T* __restrict__ keys, const unsigned long long* __restrict__ counts, const MergeTile* __restrict__ tiles,
+    const TileStream* __restrict__ ts, const InputFilter* __restrict__ filt, T* __restrict__ out_keys,
+    uint32_t* __restrict__ out_counts, TileOut<T>* __restrict__ tout, unsigned long long* __restrict__ overflow,
+    DevStatus* st, MergeAux aux, const uint32_t* __restrict__ list, const unsigned* __restrict__ nlist) {
+  const uint32_t n = list ? *nlist : gridDim.x;
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    merge_tile<T, MODE>(list ? list[i] : i, keys, counts, tiles, ts, filt, out_keys, out_counts, tout, overflow, st, aux);
+    __syncthreads();
+  }
+}
+
+// ---- u64 tiles by a table -------------------------------------------------------
+// What bounds a tile's merge is the work per row in shared memory: the merge
+// rounds above read 13 keys per row and move row indices through three rounds
+// for eight streams.  Here a row goes once into a table of keys and u32 sums
+// whose homes are in key order, as in the tile sort, and the slots, their
+// clusters put in order, are the merged rows.  A tile of one stream needs no
+// table: its rows lie in the slots in order.  A tile goes to the kernel above,
+// through a list, when a row's count is 0 or 2^19 and more (4,096 of them could
+// pass 32 bits), when a key lands kProbeLimit slots from home, and when a chunk
+// repeats a key that a filter or the one-stream path would meet.
+// k = 31: 8 databases, 96M rows 3.85 -> 1.85 ms; histo of 64.6M rows in four chunks per
+// partition 2.6 -> 1.1 ms; dump of 36.2M rows in one 1.4 -> 0.6 ms.  An AT-rich
+// genome, where a third of the tiles fail, is the case against: 31M rows of four
+// databases 1.5 -> 1.9 ms (with 16 probes instead of 32 1.8, and the first merge
+// 2.1).
+struct MergeTable {
+  static constexpr int NT = 512, NW = NT / 32, SLOTS = 7168, UNROLL = 4;
+  static constexpr size_t o_tab = 0;
+  static constexpr size_t o_cnt = o_tab + (size_t)SLOTS * 8;
+  static constexpr size_t o_ord = o_cnt + (size_t)SLOTS * 4;       // occupied slots in order (u16); histo: the bins
+  static constexpr size_t o_queue = o_ord + (size_t)kMergeCap * 2;  // per warp: 64 keys and counts that probe on
+  static constexpr size_t o_base = o_queue + (size_t)NW * 64 * 12;  // per stream: its first row less its place
+  static constexpr size_t o_start = o_base + (size_t)kMaxTileStreams * 8;
+  static constexpr size_t o_misc = o_start + (size_t)(kMaxTileStreams + 4) * 4;  // u64 range (2), then u32
+  static constexpr size_t o_edge = o_misc + 64;
+  static constexpr size_t total = o_edge + NW * 4;
+  static_assert(kHistBins * 4 <= kMergeCap * 2, "the bins fit the order list");
+  static_assert(total <= 115712, "two CTAs per SM");
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(MergeTable::NT, 2)
+    k_merge_table(const uint64_t* __restrict__ keys, const unsigned long long* __restrict__ counts,
+                  const MergeTile* __restrict__ tiles, uint32_t ntiles, const TileStream* __restrict__ ts,
+                  const InputFilter* __restrict__ filt, uint32_t filtered, uint64_t* __restrict__ out_keys,
+                  uint32_t* __restrict__ out_counts, TileOut<uint64_t>* __restrict__ tout, uint32_t* __restrict__ list,
+                  unsigned* __restrict__ nlist, unsigned* __restrict__ met, MergeAux aux) {
+  using L = MergeTable;
+  constexpr int NT = L::NT, NW = L::NW, UN = L::UNROLL;
+  constexpr unsigned long long kFree = ~0ull;
+  extern __shared__ __align__(16) uint8_t sm[];
+  unsigned long long* tab = reinterpret_cast<unsigned long long*>(sm + L::o_tab);
+  unsigned* cnt = reinterpret_cast<unsigned*>(sm + L::o_cnt);
+  uint16_t* ord = reinterpret_cast<uint16_t*>(sm + L::o_ord);
+  unsigned* hbin = reinterpret_cast<unsigned*>(sm + L::o_ord);
+  unsigned long long* sbase = reinterpret_cast<unsigned long long*>(sm + L::o_base);
+  uint32_t* sstart = reinterpret_cast<uint32_t*>(sm + L::o_start);
+  unsigned long long* range = reinterpret_cast<unsigned long long*>(sm + L::o_misc);
+  unsigned* misc = reinterpret_cast<unsigned*>(sm + L::o_misc) + 4;  // [0] failed, [1] bytes, [2 + parity] listed
+  unsigned* edge = reinterpret_cast<unsigned*>(sm + L::o_edge);
+  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  unsigned long long* qkey = reinterpret_cast<unsigned long long*>(sm + L::o_queue) + wid * 64;
+  unsigned* qcnt = reinterpret_cast<unsigned*>(sm + L::o_queue + (size_t)NW * 64 * 8) + wid * 64;
+  const InputFilter f0 = filt[0];
+  // dump and histo filter a key's sum, merge a row (a chunk has a key once)
+  auto passes = [](const InputFilter& f, uint32_t c) {
+    return !(f.has_min && c < f.min_count) && !(f.has_max && c > f.max_count);
+  };
+  unsigned ones = 0;  // histo: sums of 1, most of them
+  if (MODE == kModeHisto)
+    for (uint32_t b = threadIdx.x; b < kHistBins; b += NT) hbin[b] = 0;
+  if (threadIdx.x < 2) misc[threadIdx.x] = 0;
+  for (uint32_t tile = blockIdx.x, par = 0; tile < ntiles; tile += gridDim.x, par ^= 1) {
+    const MergeTile mt = tiles[tile];
+    const uint32_t n = mt.rows_in, nts = mt.nts;
+    if (n == 0 || nts == 0) {
+      if (MODE != kModeHisto && threadIdx.x == 0) tout[tile] = TileOut<uint64_t>{};
+      continue;
+    }
+    // data whose tiles often fail (met[1] of met[0] so far) is listed without
+    // the try; one tile in 16 still tries
+    if (threadIdx.x == 0) {
+      const unsigned tried = *(volatile unsigned*)&met[0], failed = *(volatile unsigned*)&met[1];
+      misc[2 + par] = n > kMergeCap || nts > kMaxTileStreams || (tried >= 32 && 3 * failed > tried && (tile & 15u));
+    }
+    __syncthreads();
+    if (misc[2 + par]) {
+      if (threadIdx.x == 0) list[atomicAdd(nlist, 1u)] = tile;
+      continue;
+    }
+    const bool single = nts == 1;
+    // slots: twice the rows, in whole threads' shares
+    const uint32_t slots = single ? (n + 15) & ~15u
+                           : n < (uint32_t)L::SLOTS / 2 - 288 ? (2 * n + 64 + 511) & ~511u : (uint32_t)L::SLOTS;
+    // ---- the streams (warp 0); the others clear the slots ----
+    if (wid == 0) {
+      uint32_t carry = 0;
+      unsigned long long mn = ~0ull, mx = 0;
+      for (uint32_t i0 = 0; i0 < nts; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        TileStream t{};
+        if (i < nts) t = ts[mt.first_ts + i];
+        const uint32_t len = (uint32_t)(t.hi - t.lo);
+        if (len) {
+          mn = min(mn, (unsigned long long)keys[t.lo]);
+          mx = max(mx, (unsigned long long)keys[t.hi - 1]);
+        }
+        const uint32_t incl = warp_inclusive(len, lane);
+        if (i < nts) {
+          sstart[i] = carry + incl - len;
+          // the stream's input rides in the top bits: rows are far below 2^40
+          sbase[i] = (t.lo - (carry + incl - len)) & ((1ull << 40) - 1) | (unsigned long long)t.input << 40;
+        }
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      }
+      if (lane == 0) {
+        range[0] = mn;
+        range[1] = mx;
+      }
+    } else {
+      const uint32_t j0 = threadIdx.x - 32;
+      if (!single)
+        for (uint32_t j = j0; j < slots / 2; j += NT - 32) reinterpret_cast<uint4*>(tab)[j] = make_uint4(~0u, ~0u, ~0u, ~0u);
+      for (uint32_t j = j0; j < slots / 4; j += NT - 32) reinterpret_cast<uint4*>(cnt)[j] = make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+    // ---- the rows, UN at a time per thread so that their loads overlap ----
+    {
+      const RangeMap<uint64_t> map(range[0], range[1]);
+      const HomeLinear<uint64_t> home(map, range[1], single ? 1u : slots - 2 * kProbeLimit);
+      bool bad = false;
+      uint32_t nq = 0;
+      auto probe = [&](uint32_t m) {  // the last m queued rows
+        __syncwarp();
+        nq -= m;
+        if (lane < m) {
+          const unsigned long long v = qkey[nq + lane];
+          uint32_t s = home(v);
+          const uint32_t end = s + kProbeLimit;
+          for (;;) {
+            if (++s == end) {
+              bad = true;
+              break;
+            }
+            const unsigned long long x = atomicCAS(&tab[s], kFree, v);
+            if (x == kFree || x == v) {
+              atomicAdd(&cnt[s], qcnt[nq + lane]);
+              break;
+            }
+          }
+        }
+        __syncwarp();
+      };
+      uint32_t si = 0;  // the stream of the thread's row
+      for (uint32_t r0 = threadIdx.x; r0 - threadIdx.x < n; r0 += NT * UN) {
+        unsigned long long v[UN], old[UN];
+        uint32_t c[UN], h[UN];
+        bool in[UN];
+#pragma unroll
+        for (int q = 0; q < UN; ++q) {
+          const uint32_t r = r0 + q * NT;
+          in[q] = r < n;
+          v[q] = kFree;
+          c[q] = 0;
+          if (in[q]) {
+            if (!single) {  // the last stream that starts at or before the row
+              uint32_t hi = nts - 1;
+              while (si < hi) {
+                const uint32_t mid = (si + hi + 1) >> 1;
+                if (sstart[mid] <= r) si = mid;
+                else hi = mid - 1;
+              }
+            }
+            const unsigned long long sb = sbase[si];
+            const uint64_t src = (sb + r) & ((1ull << 40) - 1);
+            v[q] = keys[src];
+            const unsigned long long w = counts[src];
+            bad |= w - 1 >= (1u << 19) - 1 || v[q] == kFree;
+            c[q] = (uint32_t)w;
+            // the row before it in its stream must have another key
+            if ((single || (MODE == kModeMerge && filtered)) && r > sstart[si]) bad |= keys[src - 1] >= v[q];
+            if (MODE == kModeMerge && filtered) in[q] = passes(filt[sb >> 40], c[q]);
+          }
+        }
+        if (single) {
+#pragma unroll
+          for (int q = 0; q < UN; ++q)
+            if (r0 + q * NT < n) {
+              tab[r0 + q * NT] = v[q];
+              cnt[r0 + q * NT] = in[q] ? c[q] : 0u;
+            }
+          continue;
+        }
+#pragma unroll
+        for (int q = 0; q < UN; ++q) {
+          h[q] = home(v[q]);
+          old[q] = in[q] ? atomicCAS(&tab[h[q]], kFree, v[q]) : kFree;
+        }
+#pragma unroll
+        for (int q = 0; q < UN; ++q) {
+          const bool hit = old[q] == kFree || old[q] == v[q];
+          if (hit && in[q]) atomicAdd(&cnt[h[q]], c[q]);
+          const unsigned miss = __ballot_sync(0xffffffffu, !hit);
+          if (miss) {
+            if (!hit) {
+              const uint32_t j = nq + __popc(miss & lt);
+              qkey[j] = v[q];
+              qcnt[j] = c[q];
+            }
+            nq += __popc(miss);
+            if (nq >= 32) probe(32);
+          }
+        }
+        if (__any_sync(0xffffffffu, bad)) break;
+      }
+      if (nq) probe(nq);
+      if (bad) misc[0] = 1;
+    }
+    __syncthreads();
+    if (misc[0]) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        list[atomicAdd(nlist, 1u)] = tile;
+        misc[0] = 0;
+        atomicAdd(&met[1], 1u);
+        atomicAdd(&met[0], 1u);
+      }
+      continue;
+    }
+    if (threadIdx.x == 0) atomicAdd(&met[0], 1u);
+    if (MODE == kModeHisto) {
+      for (uint32_t j = threadIdx.x; j < slots; j += NT) {
+        const uint32_t c = cnt[j];
+        if (c == 0 || !passes(f0, c)) continue;
+        if (c == 1) {
+          ++ones;
+        } else if (c < kHistBins) {
+          atomicAdd(&hbin[c], 1u);
+        } else {
+          const unsigned long long at = atomicAdd(aux.spill_n, 1ull);
+          if (at < aux.spill_cap) aux.spill[at] = c;
+        }
+      }
+      __syncthreads();
+      continue;
+    }
+    // ---- clusters in order (one lane each), then the thread's 16 slots listed ----
+    const uint32_t a = threadIdx.x * 16;
+    auto used = [&](auto&& ok) {
+      uint32_t m = 0;
+      if (a < slots) {
+        const uint4* c4 = reinterpret_cast<const uint4*>(cnt + a);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 x = c4[j];
+          m |= (ok(x.x) ? 1u << (4 * j) : 0u) | (ok(x.y) ? 2u << (4 * j) : 0u) | (ok(x.z) ? 4u << (4 * j) : 0u) |
+               (ok(x.w) ? 8u << (4 * j) : 0u);
+        }
+      }
+      return m;
+    };
+    uint32_t mine = used([](uint32_t c) { return c != 0; });
+    if (!single) {
+      const uint32_t before = a && a < slots && cnt[a - 1], after = a + 16 < slots && cnt[a + 16];
+      const uint32_t multi = mine & ~((mine << 1) | before) & ((mine >> 1) | (after << 15));
+      const unsigned inc = warp_inclusive(__popc(multi), lane);
+      uint16_t* first = reinterpret_cast<uint16_t*>(qkey);
+      unsigned p = inc - __popc(multi);
+      for (uint32_t m = multi; m; m &= m - 1) first[p++] = (uint16_t)(a + __ffs(m) - 1);
+      const unsigned nc = __shfl_sync(0xffffffffu, inc, 31);
+      __syncthreads();  // every warp has read the counts
+      for (unsigned j = lane; j < nc; j += 32) order_cluster(tab, cnt, first[j], slots);
+      __syncthreads();
+    }
+    if (MODE == kModeDump && filtered) mine = used([&](uint32_t c) { return c != 0 && passes(f0, c); });
+    unsigned U;
+    {
+      const unsigned inc = warp_inclusive(__popc(mine), lane);
+      if (lane == 31) edge[wid] = inc;
+      __syncthreads();
+      const unsigned wt = lane < (unsigned)NW ? edge[lane] : 0u;
+      const unsigned wi = warp_inclusive(wt, lane);
+      U = __shfl_sync(0xffffffffu, wi, NW - 1);
+      unsigned u = __shfl_sync(0xffffffffu, wi - wt, wid) + inc - __popc(mine);
+      for (uint32_t m = mine; m; m &= m - 1) ord[u++] = (uint16_t)(a + __ffs(m) - 1);
+    }
+    __syncthreads();
+    if (U == 0) {
+      if (threadIdx.x == 0) tout[tile] = TileOut<uint64_t>{};
+      continue;
+    }
+    const uint32_t line = aux.line_k + 2;
+    write_rows<NT>(
+        U, out_keys + mt.out_off, out_counts + mt.out_off, &misc[1], &tout[tile],
+        [&](unsigned u, uint64_t* key, uint32_t* c) {
+          const uint32_t s = ord[u];
+          *key = tab[s];
+          *c = cnt[s];
+        },
+        [&](unsigned u, uint64_t delta, uint32_t c) {
+          return MODE == kModeDump ? line + dec_digits(c) : dvle_size<uint64_t>(u, delta, c);
+        });
+  }
+  if (MODE == kModeHisto) {
+    __syncthreads();
+    ones = __reduce_add_sync(0xffffffffu, ones);
+    if (lane == 0 && ones) atomicAdd(&hbin[1], ones);
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < kHistBins; b += NT)
+      if (hbin[b]) atomicAdd(&aux.hist[b], (unsigned long long)hbin[b]);
   }
 }
 
@@ -1724,7 +2048,50 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
                 : mode == kModeHisto ? k_merge_tiles<T, kModeHisto>
                                      : k_merge_tiles<T, kModeMerge>;
   cudaFuncSetAttribute(kmerge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // u64 tiles go through the table, those that it lists through kmerge: always
+  // for dump and histo, for merge unless an input with a filter has several
+  // chunks in a partition (their sum is what is filtered)
+  bool by_table = sizeof(T) == 8, filtered = false;
+  for (int i = 0; i < n; ++i) {
+    if (!in[i].has_min && !in[i].has_max) continue;
+    filtered = true;
+    for (uint32_t p = 0; mode == kModeMerge && p < P; ++p) by_table &= in[i].part_count[p] <= 1;
+  }
+  Dev d_list(pool, 34);  // listed tiles, behind the groups' counters and the tiles met
+  if (!d_list.ensure(((size_t)ntiles + 16) * 4)) return fail(KITE_ERR_OOM, "merge tile buffers");
+  if (by_table) MCU(cudaMemsetAsync(d_list.p, 0, 16 * 4, s));
+  int dev = 0, sms = 0;
+  MCU(cudaGetDevice(&dev));
+  MCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   MergeAux aux{};
+  // The merge of tiles [ta, tb), group g of at most 8.
+  auto merge_tiles = [&](uint32_t ta, uint32_t tb, uint32_t g) {
+    if (tb <= ta) return;
+    const uint32_t nt = tb - ta;
+    uint32_t* list = nullptr;
+    unsigned* nlist = nullptr;
+    if constexpr (sizeof(T) == 8) {
+      if (by_table) {
+        nlist = d_list.as<unsigned>() + g;
+        list = d_list.as<uint32_t>() + 16 + ta;
+        auto ktable = mode == kModeDump    ? k_merge_table<kModeDump>
+                      : mode == kModeHisto ? k_merge_table<kModeHisto>
+                                           : k_merge_table<kModeMerge>;
+        cudaFuncSetAttribute(ktable, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MergeTable::total);
+        // histo's CTAs keep their bins over all their tiles
+        const uint32_t grid = mode == kModeHisto ? std::min<uint32_t>(nt, 2 * sms) : nt;
+        ktable<<<grid, MergeTable::NT, MergeTable::total, s>>>(
+            d_keys.as<T>(), d_counts.as<unsigned long long>(), d_mt.as<MergeTile>() + ta, nt, d_ts.as<TileStream>(),
+            d_filt.as<InputFilter>(), filtered ? 1u : 0u, d_okeys.as<T>(), d_ocounts.as<uint32_t>(),
+            d_tout.as<TileOut<T>>() + ta, list, nlist, d_list.as<unsigned>() + 8, aux);
+        launches++;
+      }
+    }
+    kmerge<<<list ? std::min<uint32_t>(nt, 2 * sms) : nt, kMergeThreads, smem, s>>>(
+        d_keys.as<T>(), d_counts.as<unsigned long long>(), d_mt.as<MergeTile>() + ta, d_ts.as<TileStream>(),
+        d_filt.as<InputFilter>(), d_okeys.as<T>(), d_ocounts.as<uint32_t>(), d_tout.as<TileOut<T>>() + ta,
+        d_over.as<unsigned long long>() + g, dst, aux, list, nlist);
+  };
   aux.line_k = key_bits / 2;
   Dev d_hist(pool, 30);
   if (mode == kModeHisto) {
@@ -1796,12 +2163,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     auto queue_merge = [&](uint32_t g) -> cudaError_t {
       const uint32_t pa = pb[g], pe = pb[g + 1], ta = tile_first[pa], tb = tile_first[pe];
       cudaEventRecord(ge[7 * g], s);
-      if (tb > ta)
-        kmerge<<<tb - ta, kMergeThreads, smem, s>>>(d_keys.as<T>(), d_counts.as<unsigned long long>(),
-                                                    d_mt.as<MergeTile>() + ta, d_ts.as<TileStream>(),
-                                                    d_filt.as<InputFilter>(), d_okeys.as<T>(), d_ocounts.as<uint32_t>(),
-                                                    d_tout.as<TileOut<T>>() + ta, d_over.as<unsigned long long>() + g,
-                                                    dst, aux);
+      merge_tiles(ta, tb, g);
       cudaEventRecord(ge[7 * g + 1], s);
       if (pe > pa) {
         launch_tile_link_ranges<T>(d_tout.as<TileOut<T>>(), pe - pa, d_tf.as<uint32_t>() + pa,
@@ -1930,10 +2292,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   }
   MCU(cudaEventRecord(sev[2], s));
   if (ntiles) {
-    kmerge<<<ntiles, kMergeThreads, smem, s>>>(d_keys.as<T>(), d_counts.as<unsigned long long>(),
-                                               d_mt.as<MergeTile>(), d_ts.as<TileStream>(), d_filt.as<InputFilter>(),
-                                               d_okeys.as<T>(), d_ocounts.as<uint32_t>(), d_tout.as<TileOut<T>>(),
-                                               d_over.as<unsigned long long>(), dst, aux);
+    merge_tiles(0, ntiles, 0);
     launches++;
   }
   MCU(cudaEventRecord(sev[3], s));

@@ -10,6 +10,7 @@
 // out in place, with the tile's DVLE size for every row but the first.
 #include <algorithm>
 
+#include "key_table.cuh"
 #include "kite_internal.h"
 
 namespace kite {
@@ -607,7 +608,6 @@ __device__ __forceinline__ void sort_tile(uint32_t tid, T* __restrict__ keys, ui
 // compare-and-swap on an all-ones slot, which no key of at most 62 bits is;
 // they stream through registers, so a tile may hold any number of keys.
 // ---------------------------------------------------------------------------
-constexpr unsigned kProbeLimit = 32;
 constexpr unsigned kHashProbes = 96;   // with hashed homes
 constexpr unsigned kMaxRanked = 512;   // distinct keys of a bin ranked by counting
 constexpr unsigned kHashAny = 1024;  // u128 tiles of at most so many keys always suit the table
@@ -627,56 +627,6 @@ struct TableSmem {
   static constexpr size_t o_misc = o_edge + (size_t)NW * 4;
   static constexpr size_t total = o_misc + 32;
 };
-
-// A key's place in the tile's key range [lo, hi]: the 32 bits of its distance
-// from lo that start at hi's top bit (a monotone map of the range).
-template <class T>
-struct RangeMap {
-  T lo;
-  int lz;
-  __device__ __forceinline__ RangeMap(T mn, T mx) : lo(mn), lz(mx == mn ? 0 : clz_key(T(mx - mn))) {}
-  __device__ __forceinline__ uint32_t at(T key) const {
-    const T v = key - lo;
-    if constexpr (sizeof(T) == 8) {
-      return (uint32_t)((v << lz) >> 32);
-    } else {
-      const uint64_t vh = hi64(v), vl = (uint64_t)v;
-      const uint64_t h = lz < 64 ? vh : vl, l = lz < 64 ? vl : 0ull;
-      const uint32_t a = (lz & 32) ? (uint32_t)h : (uint32_t)(h >> 32), b = (lz & 32) ? (uint32_t)(l >> 32) : (uint32_t)h;
-      return __funnelshift_l(b, a, lz & 31);
-    }
-  }
-};
-
-// width * 2^32 / gap, rounded down a little, so that the places x < gap of an
-// interval are spread over `width` slots by __umulhi(x, scale).
-__device__ __forceinline__ uint32_t home_scale(uint32_t width, uint32_t gap) {
-  const float f = __fdividef((float)width * 4294967296.f, (float)gap) * 0.999999f;
-  return gap == 0 ? 0u : f < 4294960000.f ? (uint32_t)f : 0xffffffffu;
-}
-
-// Home slot of a key: its place in the range scaled to the homes.
-template <class T>
-struct HomeLinear {
-  RangeMap<T> map;
-  uint32_t scale, last;
-  __device__ __forceinline__ HomeLinear(const RangeMap<T>& m, T mx, uint32_t homes)
-      : map(m), scale(home_scale(homes, m.at(mx))), last(homes - 1) {}
-  __device__ __forceinline__ uint32_t operator()(T key) const {
-    const uint32_t b = __umulhi(map.at(key), scale);
-    return b < last ? b : last;  // a key outside the range cannot leave the table
-  }
-};
-
-template <class T>
-__device__ __forceinline__ void empty_tile(TileOut<T>* out) {
-  TileOut<T> o;
-  o.first_key = o.last_key = T(0);
-  o.rows = 0;
-  o.first_count = 0;
-  o.rest_bytes = 0;
-  *out = o;
-}
 
 // A tile as the sort meets it: its keys and its key range.
 template <class T>
@@ -728,62 +678,6 @@ __device__ __forceinline__ void list_others(const TileRetry& r, const unsigned* 
   const uint32_t i = next[0] + threadIdx.x, n = tiles[i].len;
   if (n) r.add(i, n);
   else empty_tile(&tout[i]);
-}
-
-__device__ __forceinline__ unsigned warp_inclusive(unsigned v, unsigned lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= (unsigned)o) v += y;
-  }
-  return v;
-}
-
-// The U rows of a sorted tile (row(u, &key, &count)) to global memory, and the
-// tile's record.  Each warp takes consecutive rows; a lane's previous key comes
-// from the lane below, and from the round before for the first lane.  `rest`
-// is a zeroed counter, zeroed again; one barrier inside, after the last row has
-// been read.
-template <int NT, class T, class F>
-__device__ __forceinline__ void write_rows(unsigned U, T* g, uint32_t* gc, unsigned* rest_sum, TileOut<T>* out, F&& row) {
-  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned per = (U + NT - 1) / NT * 32;  // rows per warp
-  const unsigned ub = wid * per, ue = min(U, ub + per);
-  unsigned rest = 0;
-  if (ub < ue) {
-    T below = T(0);  // the key before the round's first row
-    uint32_t x;
-    if (ub) row(ub - 1, &below, &x);
-    for (unsigned u0 = ub; u0 < ue; u0 += 32) {
-      const unsigned u = u0 + lane;
-      T key = T(0);
-      uint32_t c = 0;
-      if (u < ue) row(u, &key, &c);
-      T prev = shfl_up_key(key, 1);
-      if (lane == 0) prev = below;
-      below = shfl_key(key, 31);
-      if (u < ue) {
-        g[u] = key;
-        gc[u] = c;
-        if (u) rest += varint_len(T(key - prev)) + varint_len32(c);
-      }
-    }
-  }
-  rest = __reduce_add_sync(0xffffffffu, rest);
-  if (lane == 0 && rest) atomicAdd(rest_sum, rest);
-  TileOut<T> o;
-  if (threadIdx.x == 0) {
-    uint32_t x;
-    row(0, &o.first_key, &o.first_count);
-    row(U - 1, &o.last_key, &x);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    o.rows = U;
-    o.rest_bytes = *rest_sum;
-    *out = o;
-    *rest_sum = 0;
-  }
 }
 
 __global__ void __launch_bounds__(TableSmem::NT, 2)
@@ -976,24 +870,7 @@ __global__ void __launch_bounds__(TableSmem::NT, 2)
       for (uint32_t m = mine; m; m &= m - 1) ord[u++] = (uint16_t)(a + __ffs(m) - 1);
       for (unsigned j = lane; j < nc; j += 32) {
         const uint32_t first = list[j];
-        unsigned long long last = tab[first];
-        for (uint32_t e = first + 1; e < slots; ++e) {
-          const unsigned long long v = tab[e];
-          if (v == kFree) break;
-          if (v > last) {
-            last = v;
-            continue;
-          }
-          const unsigned c = cnt[e];
-          uint32_t q = e;
-          do {
-            tab[q] = tab[q - 1];
-            cnt[q] = cnt[q - 1];
-            --q;
-          } while (q > first && tab[q - 1] > v);
-          tab[q] = v;
-          cnt[q] = c;
-        }
+        order_cluster(tab, cnt, first, slots);
       }
     }
     __syncthreads();
@@ -1069,7 +946,8 @@ __global__ void __launch_bounds__(TableSmem::NT, 2)
           const uint32_t s = ord[u];
           *key = tab[s];
           *c = cnt[s];
-        });
+        },
+        dvle_size<uint64_t>);
     if (threadIdx.x == 0) {
       retry.met_tile(hashed && 2 * U > n);  // mostly distinct keys: the binning sort is the faster one
       if (n > tile_capacity<uint64_t>() && fallbacks) atomicAdd(&fallbacks[1], (unsigned long long)U);
@@ -1270,7 +1148,8 @@ __global__ void __launch_bounds__(HashSmem::NT, 2)
                      const unsigned e = list[u];
                      *key = buf[e & 0xffffu];
                      *c = e >> 16;
-                   });
+                   },
+                   dvle_size<u128>);
     // mostly distinct keys: the binning sort is the faster one
     if (threadIdx.x == 0) retry.met_tile(n > kHashAny && 4 * U > 3 * n);
     load(next);
