@@ -58,6 +58,12 @@ enum {
   KITE_ERR_STATE = -9           /* call out of order */
 };
 
+/* How the key-range tiles are cut.  SAMPLED: by a histogram of sampled keys.
+ * LEARNED: by a CDF trained on them (650 ms once per context), unless it
+ * predicts a worse balance than imbalance_bound and the histogram.  AUTO: by the
+ * histogram, or, when it predicts a largest tile above imbalance_bound times the
+ * mean, by the sample's quantiles (reported as SAMPLED); merge, dump and histo
+ * use the histogram. */
 enum { KITE_SPLIT_AUTO = 0, KITE_SPLIT_SAMPLED = 1, KITE_SPLIT_LEARNED = 2 };
 
 /* Codec bits of a chunk (src/format/run_block.rs:1-3). */
@@ -71,7 +77,7 @@ typedef struct {
   int canonical;             /* 0 or 1 */
   uint32_t partitions;       /* power of two >= 2: hash buckets of the .kite file */
   int splitter_mode;         /* KITE_SPLIT_* : how key-range tiles are cut */
-  double imbalance_bound;    /* learned splitters fall back above this max/mean (0 = 1.10) */
+  double imbalance_bound;    /* AUTO and LEARNED look for other splitters above this max/mean (0 = 1.10) */
   uint64_t arena_bytes;      /* FASTQ bytes held on device before a flush (0 = auto) */
   uint32_t timeout_ms;       /* bound on every host-side wait (0 = 600000) */
   void* stream;              /* optional cudaStream_t to run on (NULL = own stream) */

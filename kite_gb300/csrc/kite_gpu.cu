@@ -116,7 +116,7 @@ struct kite_gpu_ctx {
 
   // scratch
   DevBuf blocks, nl, scan_tmp, bucket_count, bucket_off, bucket_fill, totals, status;
-  DevBuf keys_a, keys_b, counts, sample, sample_count, splitters, splitters2, hist16;
+  DevBuf keys_a, keys_b, counts, sample, sample_count, splitters, splitters2, hist16, quant_keys;
   DevBuf tile_count, tile_off, tile_fill, tiles, big_ids, tile_out, tile_boff, tile_prev, meta, out;
   DevBuf lvl_count, lvl_off, reg_off, reg_cnt, sort_stats, blk_mat, blk_gsum, blk_keys, stage_ctr;
   DevBuf col_total, sample_first, spans, digits, tile_lists, piece_off, piece_cnt, piece_base;
@@ -575,14 +575,15 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     // Splitters: SAMPLED = histogram only; LEARNED = train the CDF and keep
     // it unless its predicted max/mean tile load exceeds imbalance_bound AND
     // the histogram's prediction is lower (then the histogram); AUTO =
-    // histogram unless its own prediction exceeds the bound, then as LEARNED.
+    // histogram unless its own prediction exceeds the bound, then the sample's
+    // quantiles if they predict less.
     KCU(ctx->splitters.ensure((size_t)S * sizeof(T)));
     KCU(ctx->splitters2.ensure((size_t)S * sizeof(T)));
     KCU(ctx->hist16.ensure((size_t)65536 * 4));
     const int mode = ctx->cfg.splitter_mode;
     const double bound = ctx->cfg.imbalance_bound;
     T* hist_spl = ctx->splitters.as<T>();
-    T* mlp_spl = ctx->splitters2.as<T>();
+    T* mlp_spl = ctx->splitters2.as<T>();  // or the quantiles
     double hist_imb = -1.0;
     // The splitters depend only on the key sample, complete since the bucket
     // counts were read back: they are made on the side stream, so their
@@ -599,8 +600,17 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
         st.kernel_launches += 1;
       }
     }
-    bool learned = false;
-    if (mode == KITE_SPLIT_LEARNED || (mode == KITE_SPLIT_AUTO && hist_imb > bound)) {
+    bool learned = false, quantiles = false;
+    if (mode == KITE_SPLIT_AUTO && hist_imb > bound && nsample >= S) {
+      KCU(ctx->quant_keys.ensure((size_t)quantile_keys() * sizeof(T)));
+      double imb = 0.0;
+      st.kernel_launches += 1 + compute_quantile_splitters<T>(ctx->sample.as<T>(), nsample, S, mlp_spl,
+                                                              ctx->quant_keys.as<T>(), ss);
+      if (predict_imbalance<T>(ctx->mlp, ctx->sample.as<T>(), nsample, mlp_spl, S, ss, ctx->cfg.timeout_ms, &imb))
+        return fail(ctx, KITE_ERR_TIMEOUT, "splitter evaluation did not finish");
+      quantiles = imb < hist_imb;
+    }
+    if (mode == KITE_SPLIT_LEARNED) {
       MlpReport rep;
       if (mlp_splitters<T>(ctx->mlp, ctx->sample.as<T>(), nsample, 2 * k, S, mlp_spl, ss, ctx->cfg.timeout_ms, &rep))
         return fail(ctx, KITE_ERR_CUDA, "learned splitter training failed");
@@ -609,7 +619,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
       st.mlp_pred_imbalance = rep.pred_imbalance;
       st.mlp_reused = rep.reused ? 1u : 0u;
       learned = rep.pred_imbalance <= bound;
-      if (!learned && mode == KITE_SPLIT_LEARNED) {
+      if (!learned) {
         st.kernel_launches += compute_hist_splitters<T>(ctx->sample.as<T>(), nsample, 2 * k, S, hist_spl,
                                                         ctx->hist16.as<unsigned>(), ss);
         if (predict_imbalance<T>(ctx->mlp, ctx->sample.as<T>(), nsample, hist_spl, S, ss, ctx->cfg.timeout_ms,
@@ -622,7 +632,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     }
     st.hist_pred_imbalance = hist_imb;
     st.splitter_used = learned ? KITE_SPLIT_LEARNED : KITE_SPLIT_SAMPLED;
-    const T* chosen = learned ? mlp_spl : hist_spl;
+    const T* chosen = learned || quantiles ? mlp_spl : hist_spl;
     tile_spl = chosen;
     KCU(cudaEventRecord(ctx->spl_ready, ss));
     KCU(cudaStreamWaitEvent(s, ctx->spl_ready, 0));
@@ -1082,7 +1092,7 @@ void kite_gpu_close(kite_gpu_ctx* ctx) {
   for (auto e : ctx->gev) cudaEventDestroy(e);
   DevBuf* bufs[] = {&ctx->arena, &ctx->blocks, &ctx->nl, &ctx->scan_tmp, &ctx->bucket_count, &ctx->bucket_off,
                     &ctx->bucket_fill, &ctx->totals, &ctx->status, &ctx->keys_a, &ctx->keys_b, &ctx->counts,
-                    &ctx->sample, &ctx->sample_count, &ctx->splitters, &ctx->splitters2, &ctx->hist16,
+                    &ctx->sample, &ctx->sample_count, &ctx->splitters, &ctx->splitters2, &ctx->hist16, &ctx->quant_keys,
                     &ctx->tile_count, &ctx->tile_off, &ctx->tile_fill, &ctx->tiles, &ctx->big_ids,
                     &ctx->tile_out, &ctx->tile_boff, &ctx->tile_prev, &ctx->meta, &ctx->out,
                     &ctx->lvl_count, &ctx->lvl_off, &ctx->reg_off, &ctx->reg_cnt, &ctx->sort_stats,
