@@ -150,16 +150,19 @@ __device__ __forceinline__ void reserve_ranges(const ExtractParams<T>& p, unsign
 
 __host__ __device__ size_t extract64_smem_bytes(uint32_t partitions, bool scatter);
 
-// A word's forward and reverse-complement code streams, shared with the warp.
-struct CodeWords {
-  uint64_t code, rcode;
+// The warp's 64 words and the one before them as 32-bit words, codes in reverse
+// word order and complement codes in word order: a lane's windows are three
+// consecutive words each, at fixed offsets.  (A window past the complement
+// codes' end is masked off.)
+struct WarpCodes {
+  uint64_t code[65], rcode[67];
 };
 
 size_t extract_smem_bytes(int key_bytes, uint32_t blk_bytes, uint32_t partitions, bool scatter) {
   (void)blk_bytes;
   const size_t b = extract64_smem_bytes(partitions, scatter);
-  // the u64 histogram pass also shares every thread's three encoded words with its warp
-  return key_bytes == 8 && !scatter ? ((b + 15) & ~(size_t)15) + (size_t)kExtractThreads * 3 * sizeof(CodeWords) : b;
+  // the u64 histogram pass also shares every thread's encoded words with its warp
+  return key_bytes == 8 && !scatter ? ((b + 15) & ~(size_t)15) + (size_t)(kExtractThreads / 32) * sizeof(WarpCodes) : b;
 }
 
 // ---------------------------------------------------------------------------
@@ -301,11 +304,17 @@ __global__ void __launch_bounds__(kExtractThreads, 6) k_extract64(ExtractParams<
     // lanes share every sequence word's k-mers (a thread's own bytes may be
     // a quality line) and a word's keys go out as one coalesced run.
     const unsigned lane = threadIdx.x & 31;
-    CodeWords* ws = reinterpret_cast<CodeWords*>(sm + ((extract64_smem_bytes(P, false) + 15) & ~(size_t)15)) +
-                    (size_t)(threadIdx.x & ~31u) * 3;
-    ws[3 * lane] = CodeWords{wp.code, wp.rcode};
-    ws[3 * lane + 1] = CodeWords{w0.code, w0.rcode};
-    ws[3 * lane + 2] = CodeWords{w1.code, w1.rcode};
+    WarpCodes& wc = reinterpret_cast<WarpCodes*>(
+        sm + ((extract64_smem_bytes(P, false) + 15) & ~(size_t)15))[threadIdx.x >> 5];
+    // word i of the warp (0: the one before it) is code[64 - i], rcode[i]
+    if (lane == 0) {
+      wc.code[64] = wp.code;
+      wc.rcode[0] = wp.rcode;
+    }
+    wc.code[63 - 2 * lane] = w0.code;
+    wc.code[62 - 2 * lane] = w1.code;
+    wc.rcode[2 * lane + 1] = w0.rcode;
+    wc.rcode[2 * lane + 2] = w1.rcode;
     __syncwarp();
     const unsigned lt = (1u << lane) - 1u;
     const uint64_t wts = ts - (uint64_t)lane * 64;  // the warp's first byte
@@ -317,14 +326,15 @@ __global__ void __launch_bounds__(kExtractThreads, 6) k_extract64(ExtractParams<
     }
     // A lane's windows are fixed shifts of the (previous, current) word pair:
     // the forward k-mer is the low 64 bits of (pw.code:cw.code) >> sft and the
-    // reverse complement the low 64 bits of (cw.rcode:pw.rcode) >> t, both
-    // per-lane constants.  Each is two 32-bit funnel shifts of the 32-bit
-    // words that the shift's word offset selects (chosen once per lane).
-    const uint32_t sft = 2 * (31 - lane);     // 0 .. 62: word offset 0 or 1
-    const bool f_hi = sft >= 32;
-    const uint32_t fsh = sft & 31u;
-    const uint32_t tr = 2 * (33 + lane - k);  // 4 .. 126: word offset 0 .. 3
-    const uint32_t tq = tr >> 5, tsh = tr & 31u;
+    // reverse complement the low 64 bits of (cw.rcode:pw.rcode) >> t: two
+    // 32-bit funnel shifts each, of words loaded at the shift's word offset.
+    // (1.16G keys 6.5 -> 5.5 ms: loading both words whole and selecting by the
+    // offset took ten more instructions per word.)
+    const uint32_t sft = 2 * (31 - lane);     // 0 .. 62
+    const uint32_t tr = 2 * (33 + lane - k);  // 4 .. 126
+    const uint32_t* fw = reinterpret_cast<const uint32_t*>(wc.code) + 126 + (sft >> 5);  // word 1's
+    const uint32_t* rw = reinterpret_cast<const uint32_t*>(wc.rcode) + (tr >> 5);
+    const uint32_t mlo = (uint32_t)mask, mhi = (uint32_t)(mask >> 32);
     unsigned run = 0;
     for (unsigned ls = __ballot_sync(0xffffffffu, (V0 | V1) != 0u); ls; ls &= ls - 1) {
       const int l = __ffs(ls) - 1;
@@ -336,21 +346,14 @@ __global__ void __launch_bounds__(kExtractThreads, 6) k_extract64(ExtractParams<
         const bool act = (V >> lane) & 1u;
         uint64_t key = 0;
         if (act) {
-          const CodeWords pw = ws[3 * l + h], cw = ws[3 * l + h + 1];
-          const uint32_t c0 = (uint32_t)cw.code, c1 = (uint32_t)(cw.code >> 32);
-          const uint32_t p0 = (uint32_t)pw.code, p1 = (uint32_t)(pw.code >> 32);
-          const uint32_t a0 = f_hi ? c1 : c0, a1 = f_hi ? p0 : c1, a2 = f_hi ? p1 : p0;
-          const uint64_t fwd =
-              (((uint64_t)__funnelshift_r(a1, a2, fsh) << 32) | __funnelshift_r(a0, a1, fsh)) & mask;
+          const uint32_t* f = fw - 2 * (2 * l + h);
+          const uint32_t* r = rw + 2 * (2 * l + h);
+          const uint32_t f1 = f[1];
+          const uint64_t fwd = (uint64_t)(__funnelshift_r(f1, f[2], sft) & mhi) << 32 | (__funnelshift_r(f[0], f1, sft) & mlo);
           key = fwd;
           if (canon) {
-            const uint32_t r0 = (uint32_t)pw.rcode, r1 = (uint32_t)(pw.rcode >> 32);
-            const uint32_t r2 = (uint32_t)cw.rcode, r3 = (uint32_t)(cw.rcode >> 32);
-            const uint32_t b0 = tq == 0 ? r0 : tq == 1 ? r1 : tq == 2 ? r2 : r3;
-            const uint32_t b1 = tq == 0 ? r1 : tq == 1 ? r2 : tq == 2 ? r3 : 0u;
-            const uint32_t b2 = tq == 0 ? r2 : tq == 1 ? r3 : 0u;
-            const uint64_t rc =
-                (((uint64_t)__funnelshift_r(b1, b2, tsh) << 32) | __funnelshift_r(b0, b1, tsh)) & mask;
+            const uint32_t r1 = r[1];
+            const uint64_t rc = (uint64_t)(__funnelshift_r(r1, r[2], tr) & mhi) << 32 | (__funnelshift_r(r[0], r1, tr) & mlo);
             key = rc < fwd ? rc : fwd;
           }
           atomicAdd(&hist[bucket_of(key, shift)], 1u);
@@ -1184,34 +1187,36 @@ __global__ void __launch_bounds__(NT, (IT * sizeof(T) > 64 ? 512 : 1024) / NT)
 // BATCH keys ranked on chip by partition (shared-memory atomics; order inside a
 // partition does not matter), staged in partition order and written as runs at
 // the block's offsets.
-constexpr int kBsThreads = 256, kBsItems = 8, kBsBatch = kBsThreads * kBsItems;
+// Each thread keeps its bucket's output position in a register, and a staged
+// key's bucket is computed again rather than kept (a byte store and two loads
+// per key).  1.16G u64 keys (10M reads): 5.3 -> 4.4 ms, with 256 threads 5.2, with
+// 512 and eight keys each 5.2: an extraction block of reads yields some 6,000
+// keys, two batches of 3,072.  u128 keys in 384 threads: 1.6 ms against 1.4.
 template <class T>
 struct BsSmem {
-  static constexpr int NW = kBsThreads / 32;
+  static constexpr int NT = sizeof(T) == 8 ? 384 : 256, IT = 8, BATCH = NT * IT, PER_SM = sizeof(T) == 8 ? 3 : 4;
   static constexpr size_t o_stage = 0;
-  static constexpr size_t o_dig = o_stage + (size_t)kBsBatch * sizeof(T);
-  static constexpr size_t o_whist = (o_dig + (size_t)kBsBatch + 15) & ~(size_t)15;
-  static constexpr size_t o_cur = o_whist + (size_t)256 * NW * 4;
-  static constexpr size_t o_dtot = o_cur + (size_t)256 * 8;
+  static constexpr size_t o_gpos = o_stage + (size_t)BATCH * sizeof(T);
+  static constexpr size_t o_whist = o_gpos + (size_t)256 * 8;
+  static constexpr size_t o_dtot = o_whist + (size_t)256 * 4;
   static constexpr size_t o_dstart = o_dtot + (size_t)256 * 4;
   static constexpr size_t o_scan = o_dstart + (size_t)256 * 4;
   static constexpr size_t total = o_scan + 64 * 4;
 };
 
 template <class T>
-__global__ void __launch_bounds__(kBsThreads, 4)
+__global__ void __launch_bounds__(BsSmem<T>::NT, BsSmem<T>::PER_SM)
     k_bucket_scatter(const T* __restrict__ keys_stage, const unsigned long long* __restrict__ blk_keys,
                      const unsigned* __restrict__ blk_offs, const BlockDesc* __restrict__ blocks,
                      const unsigned long long* __restrict__ bucket_off, uint32_t P, uint32_t shift,
                      T* __restrict__ keys_out, const unsigned long long* __restrict__ stage_counter,
                      unsigned long long stage_cap) {
   using L = BsSmem<T>;
-  constexpr int NT = kBsThreads, IT = kBsItems;
+  constexpr int NT = L::NT, IT = L::IT;
   extern __shared__ __align__(16) uint8_t sm[];
   T* stage = reinterpret_cast<T*>(sm + L::o_stage);
-  uint8_t* dig8 = sm + L::o_dig;
+  unsigned long long* gpos = reinterpret_cast<unsigned long long*>(sm + L::o_gpos);  // a bucket's output less its stage start
   unsigned* whist = reinterpret_cast<unsigned*>(sm + L::o_whist);
-  unsigned long long* cur = reinterpret_cast<unsigned long long*>(sm + L::o_cur);
   unsigned* dtot = reinterpret_cast<unsigned*>(sm + L::o_dtot);
   unsigned* dstart = reinterpret_cast<unsigned*>(sm + L::o_dstart);
   unsigned* scan_sm = reinterpret_cast<unsigned*>(sm + L::o_scan);
@@ -1220,17 +1225,19 @@ __global__ void __launch_bounds__(kBsThreads, 4)
   // an unstaged block (a == ~0), or staging over capacity anywhere so far:
   // the host scatters from the FASTQ instead
   if (n == 0 || a == ~0ull || (stage_counter && *stage_counter > stage_cap)) return;
-  const BlockDesc d = blocks[blockIdx.x];
-  const unsigned* row = blk_offs + (size_t)blockIdx.x * P;
-  const unsigned* first = blk_offs + (size_t)d.sample_first * P;  // the sample's first block
-  const unsigned long long* boff = bucket_off + (size_t)d.sample * P;
-  for (uint32_t b = threadIdx.x; b < P; b += NT) cur[b] = boff[b] + (row[b] - first[b]);
-  for (int b = threadIdx.x; b < 256; b += NT) whist[b] = 0;  // rank counters
+  const uint32_t b = threadIdx.x;  // this thread's bucket
+  unsigned long long cur = 0;      // where its next key goes
+  if (b < P) {
+    const BlockDesc d = blocks[blockIdx.x];
+    cur = bucket_off[(size_t)d.sample * P + b] +
+          (blk_offs[(size_t)blockIdx.x * P + b] - blk_offs[(size_t)d.sample_first * P + b]);
+  }
+  if (b < 256) whist[b] = 0;  // rank counters
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned pos0 = (unsigned)wid * 32u * IT + lane;
-  for (uint64_t c0 = 0; c0 < n; c0 += kBsBatch) {
-    const unsigned cn = (unsigned)((n - c0) < (uint64_t)kBsBatch ? (n - c0) : (uint64_t)kBsBatch);
+  for (uint64_t c0 = 0; c0 < n; c0 += L::BATCH) {
+    const unsigned cn = (unsigned)((n - c0) < (uint64_t)L::BATCH ? (n - c0) : (uint64_t)L::BATCH);
     T key[IT];
     unsigned dg[IT], dest[IT];
     bool valid[IT];
@@ -1239,23 +1246,24 @@ __global__ void __launch_bounds__(kBsThreads, 4)
       const unsigned pos = pos0 + q * 32u;
       valid[q] = pos < cn;
       key[q] = valid[q] ? keys_stage[a + c0 + pos] : T(0);
-      dg[q] = valid[q] ? bucket_of(key[q], shift) : 0u;
     }
+#pragma unroll
+    for (int q = 0; q < IT; ++q) dg[q] = valid[q] ? bucket_of(key[q], shift) : 0u;
     atomic_rank<NT, IT, 256>(dg, valid, dest, whist, scan_sm, dtot, dstart);
+    if (b < 256) {
+      gpos[b] = cur - dstart[b];
+      cur += dtot[b];
+    }
 #pragma unroll
     for (int q = 0; q < IT; ++q)
-      if (valid[q]) {
-        stage[dest[q]] = key[q];
-        dig8[dest[q]] = (uint8_t)dg[q];
-      }
+      if (valid[q]) stage[dest[q]] = key[q];
     __syncthreads();
     for (unsigned i = threadIdx.x; i < cn; i += NT) {
-      const unsigned d = dig8[i];
-      keys_out[cur[d] + (i - dstart[d])] = stage[i];
+      const T x = stage[i];
+      keys_out[gpos[bucket_of(x, shift)] + i] = x;
     }
-    __syncthreads();
-    for (uint32_t b = threadIdx.x; b < P; b += NT) cur[b] += dtot[b];
-    __syncthreads();
+    // no barrier: the next batch changes the stage and the positions only
+    // after the ranking's first barrier, which every thread reaches after this loop
   }
 }
 
@@ -1267,7 +1275,7 @@ void launch_bucket_scatter(const T* keys_stage, const unsigned long long* blk_ke
   const size_t smem = BsSmem<T>::total;
   cudaFuncSetAttribute(k_bucket_scatter<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (nblocks)
-    k_bucket_scatter<T><<<nblocks, kBsThreads, smem, s>>>(keys_stage, blk_keys, blk_offs, blocks, bucket_off,
+    k_bucket_scatter<T><<<nblocks, BsSmem<T>::NT, smem, s>>>(keys_stage, blk_keys, blk_offs, blocks, bucket_off,
                                                           partitions, shift, keys_out, stage_counter, stage_cap);
 }
 template void launch_bucket_scatter<uint64_t>(const uint64_t*, const unsigned long long*, const unsigned*,

@@ -55,8 +55,10 @@ template <> struct KeyTraits<u128> {
 
 // Fibonacci hash partition (src/count/kmer.rs:67-71, :111-116).
 // `shift` = 64 - log2(partitions), always < 64 because partitions >= 2.
+// (At most 2^32 partitions: the product's upper word is enough.)
 __device__ __forceinline__ uint32_t bucket_of(uint64_t key, uint32_t shift) {
-  return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> shift);
+  const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+  return (__umulhi(lo, 0x7F4A7C15u) + lo * 0x9E3779B9u + hi * 0x7F4A7C15u) >> (shift - 32);
 }
 __device__ __forceinline__ uint32_t bucket_of(u128 key, uint32_t shift) {
   return bucket_of((uint64_t)key ^ (uint64_t)(key >> 64), shift);
