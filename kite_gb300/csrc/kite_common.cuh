@@ -72,15 +72,10 @@ __device__ __forceinline__ int clz_key(u128 v) {
 
 // LEB128 length of an unsigned value (write_varint_u64/u128,
 // src/format/run_block.rs:9-35): max(1, ceil(bits/7)).
-__device__ __forceinline__ int varint_len(uint64_t v) {
-  int bits = 64 - __clzll((long long)v);
-  return bits == 0 ? 1 : (bits + 6) / 7;
-}
-__device__ __forceinline__ int varint_len32(uint32_t v) { return (38 - __clz((int)(v | 1u))) / 7; }
-__device__ __forceinline__ int varint_len(u128 v) {
-  int bits = 128 - clz_key(v);
-  return bits == 0 ? 1 : (bits + 6) / 7;
-}
+__device__ __forceinline__ int seventh(unsigned x) { return (int)(x * 293u >> 11); }  // x / 7 for x < 680
+__device__ __forceinline__ int varint_len(uint64_t v) { return seventh(70 - (unsigned)__clzll((long long)(v | 1))); }
+__device__ __forceinline__ int varint_len32(uint32_t v) { return seventh(38 - (unsigned)__clz((int)(v | 1u))); }
+__device__ __forceinline__ int varint_len(u128 v) { return seventh(134 - (unsigned)clz_key(v | u128(1))); }
 
 __host__ __device__ __forceinline__ uint64_t hi64(uint64_t) { return 0; }
 __host__ __device__ __forceinline__ uint64_t hi64(u128 v) { return (uint64_t)(v >> 64); }
