@@ -83,7 +83,7 @@ typedef struct {
   void* stream;              /* optional cudaStream_t to run on (NULL = own stream) */
   uint32_t samples;          /* batched count: samples per segment (0 = 1); see kite_gpu_count_submit_sample */
   double tile_fill;          /* target tile load as a fraction of on-chip capacity (0 = 0.85) */
-  int scatter_shape;         /* key-range split scatter launch shape 0..3 (0 = 256 threads x 8 keys) */
+  int scatter_shape;         /* key-range split scatter launch shape 0..3 (0 = by the number of ranges) */
   uint32_t tile_wait_polls;  /* bound of the tile sort's first wait for a tile's bulk load (0 = 2^18 polls);
                                 1 gives up unless the copy has already landed (tests of the timeout path:
                                 the count then returns KITE_ERR_TIMEOUT) */
@@ -121,7 +121,8 @@ typedef struct {
   uint64_t kernel_launches;          /* kernels this library launched in the last finish */
   double mlp_loss, mlp_pred_imbalance, hist_pred_imbalance; /* learned-splitter diagnostics */
   double range_imbalance;            /* max / mean keys per key range (summed over partitions) */
-  uint64_t sort_fallbacks;           /* tiles whose on-chip sort fell back to LSD passes (a large bin of distinct keys) */
+  uint64_t sort_fallbacks;           /* tiles whose keys were too clustered for the sort's first form: counted with
+                                        hashed homes, or LSD passes for a large bin of distinct keys */
   uint32_t split_levels;             /* key-range split passes over the keys (0, 1 or 2) */
   uint32_t staged_scatter;           /* 1: keys staged by the histogram pass, then a ranked bucket scatter */
   uint32_t mlp_reused;               /* 1: the learned CDF of an earlier segment was kept (no training) */

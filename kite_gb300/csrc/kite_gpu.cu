@@ -8,7 +8,8 @@
 //       reads/bases/kmers, key sample from the segment's first chunk
 //   K3  extract (scatter pass): k-mers into their hash-bucket regions
 //   K3b tile split: each bucket cut into key-range tiles by splitters
-//   K4  tile sort + run-length reduction on chip (oversized tiles: K4b)
+//   K4  tile sort + run-length reduction on chip: distinct keys counted in
+//       tables, or binned (listed tiles); oversized tiles: K4b
 //   K7  DVLE encode of every bucket's rows into one payload per partition
 #include <algorithm>
 #include <chrono>
@@ -148,7 +149,6 @@ int fail(kite_gpu_ctx* c, int code, const std::string& msg) {
                   std::string(#call) + ": " + cudaGetErrorString(_e));                  \
   } while (0)
 
-// Bounded wait for all work queued on `s`.
 // Waits (bounded by cfg.timeout_ms) for a recorded event.
 int wait_event(kite_gpu_ctx* ctx, cudaEvent_t e) {
   PollPause pause(ctx->cfg.timeout_ms);

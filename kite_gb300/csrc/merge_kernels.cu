@@ -11,17 +11,17 @@
 //                           otherwise one DVLE chunk per non-empty partition.
 //
 // GPU structure:
-//   decode    payload bytes cut into 8 KiB segments, one warp each;
-//             per-segment varint terminator counts and parity sums,
-//             per-stream scans on the device, then a pass that writes
-//             (key, u64 count) rows.  A
-//             "stream" is one chunk.
-//   tiles     key-range tiles per partition from global splitters, refined by
-//             bisection until every tile fits on chip; each stream is
-//             binary-searched for the tile edges.
-//   merge     one CTA per tile: rows of all its streams into shared memory,
-//             merged ranks by binary search (ties broken by stream order),
-//             per-input sums, filter, cross-input sums, overflow check.
+//   decode    payload bytes cut into 8 KiB segments, one warp each, as their
+//             piece of the input lands: varints per segment, per-stream scans,
+//             then rows with a lane each, keys relative to the segment until
+//             the start keys are added.  A "stream" is one chunk.
+//   tiles     key-range tiles per partition from global splitters (or slices of
+//             a partition's only stream), planned on the device; ranges above
+//             the on-chip capacity are cut by bisection on the host.
+//   merge     one CTA per tile: u64 rows summed in a shared-memory table, or
+//             (u128, and tiles that a table does not suit) rows merged by merge
+//             paths, with per-input sums, filter, cross-input sums, overflow
+//             check.
 //   encode    the count path's DVLE link + encode kernels.
 //
 // The same decode / tile / merge stages serve `kite dump` (one input):
