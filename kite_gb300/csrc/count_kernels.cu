@@ -918,8 +918,7 @@ __global__ void __launch_bounds__(NT, (IT * sizeof(T) > 64 ? 512 : 1024) / NT) k
   }
   T lo = T(0);
   uint32_t sh = 0;
-  if (p.dig) __syncthreads();  // the histogram pass left every digit
-  else load_digits(p, r, spl, lut, &lo, &sh);  // ends with a barrier
+  load_digits(p, r, spl, lut, &lo, &sh);  // ends with a barrier
   uint64_t a, e;
   part_range(p, r, g, &a, &e);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -936,13 +935,8 @@ __global__ void __launch_bounds__(NT, (IT * sizeof(T) > 64 ? 512 : 1024) / NT) k
       valid[q] = pos < cn;
       key[q] = valid[q] ? p.keys_in[c0 + pos] : T(0);
     }
-    if (p.dig) {
 #pragma unroll
-      for (int q = 0; q < IT; ++q) dg[q] = valid[q] ? (unsigned)p.dig[c0 + pos0 + q * 32u] : 0u;
-    } else {
-#pragma unroll
-      for (int q = 0; q < IT; ++q) dg[q] = valid[q] ? digit_of_key(spl, lut, lo, sh, key[q]) : 0u;
-    }
+    for (int q = 0; q < IT; ++q) dg[q] = valid[q] ? digit_of_key(spl, lut, lo, sh, key[q]) : 0u;
 #pragma unroll
     for (int q = 0; q < IT; ++q) rank[q] = valid[q] ? atomicAdd(&whist[dg[q]], 1u) : 0u;
     __syncthreads();
@@ -1513,10 +1507,12 @@ void launch_split_scatter(const TileSplitParams<T>& p, int shape, cudaStream_t s
       if (p.R * p.G) kern<<<p.R * p.G, C::NT, smem, s>>>(p);
       return;
     }
-    auto kern = k_split_scatter<T, C::NT, C::IT, C::RADIX>;
-    const size_t smem = ScatterSmem<T, C::NT, C::IT, C::RADIX>::total;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (p.R * p.G) kern<<<p.R * p.G, C::NT, smem, s>>>(p);
+    if constexpr (C::RADIX == 16) {  // the first of two levels: at most four coarse ranges
+      auto kern = k_split_scatter<T, C::NT, C::IT, C::RADIX>;
+      const size_t smem = ScatterSmem<T, C::NT, C::IT, C::RADIX>::total;
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (p.R * p.G) kern<<<p.R * p.G, C::NT, smem, s>>>(p);
+    }
   });
 }
 
@@ -1527,10 +1523,15 @@ uint32_t split_scatter_slots(uint32_t D, int shape) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   with_scatter_cfg<T>(D, shape, [&](auto cfg) {
     using C = decltype(cfg);
-    auto kern = k_split_scatter<T, C::NT, C::IT, C::RADIX>;
-    const size_t smem = ScatterSmem<T, C::NT, C::IT, C::RADIX>::total;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
+    auto slots = [&](auto kern, size_t smem) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
+    };
+    // more than 16 digits: a last level, whose digits the histogram pass left
+    if constexpr (C::RADIX > 16)
+      slots(k_split_scatter_bulk<T, C::NT, C::IT, C::RADIX>, BulkScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
+    else
+      slots(k_split_scatter<T, C::NT, C::IT, C::RADIX>, ScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
   });
   return (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per_sm);
 }
