@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(MergeTable::NT, 2)
   if (MODE == kModeHisto)
     for (uint32_t b = threadIdx.x; b < kHistBins; b += NT) hbin[b] = 0;
   if (threadIdx.x < 2) misc[threadIdx.x] = 0;
-  for (uint32_t tile = blockIdx.x, par = 0; tile < ntiles; tile += gridDim.x, par ^= 1) {
+  for (uint32_t tile = blockIdx.x, par = 0; tile < ntiles; tile += gridDim.x) {
     const MergeTile mt = tiles[tile];
     const uint32_t n = mt.rows_in, nts = mt.nts;
     if (n == 0 || nts == 0) {
@@ -1014,7 +1014,12 @@ __global__ void __launch_bounds__(MergeTable::NT, 2)
       misc[2 + par] = n > kMergeCap || nts > kMaxTileStreams || (tried >= 32 && 3 * failed > tried && (tile & 15u));
     }
     __syncthreads();
-    if (misc[2 + par]) {
+    // The two places of the decision take turns over the tiles that have one
+    // (an empty tile has none, and no barrier): it is written again only after
+    // the next such tile's barrier, when every thread has read it.
+    const bool listed = misc[2 + par];
+    par ^= 1;
+    if (listed) {
       if (threadIdx.x == 0) list[atomicAdd(nlist, 1u)] = tile;
       continue;
     }
