@@ -45,6 +45,7 @@
 
 #include "mlp.h"
 #include "kite_internal.h"
+#include "splitters.h"
 
 namespace kite {
 
@@ -129,11 +130,6 @@ void mlp_destroy(MlpModel* m) {
   delete m;
 }
 
-// ---- 48-bit view of a key ---------------------------------------------------
-template <class T>
-__device__ __forceinline__ uint64_t view48(T key, uint32_t key_bits) {
-  return key_bits >= 48 ? (uint64_t)(key >> (key_bits - 48)) : ((uint64_t)key << (48 - key_bits));
-}
 __device__ __forceinline__ float bit_of(uint64_t v, int i) { return (float)((v >> (kIn - 1 - i)) & 1ull); }
 // splitmix64 finalizer: the minibatch of step t draws sample mix64(t, b) mod n
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {

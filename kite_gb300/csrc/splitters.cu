@@ -15,11 +15,8 @@ namespace kite {
 template <class T>
 __global__ void k_sample_hist(const T* __restrict__ sample, uint32_t n, uint32_t key_bits, uint32_t hbits,
                               unsigned* __restrict__ hist) {
-  const uint32_t sh = key_bits - hbits;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t bin = (uint32_t)(uint64_t)(sample[i] >> sh);
-    atomicAdd(&hist[bin], 1u);
-  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    atomicAdd(&hist[sample_bin(sample[i], key_bits, hbits)], 1u);
 }
 
 // One CTA: turns the histogram into its inclusive cumulative counts (in
