@@ -1395,6 +1395,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     cudaError_t _e = (call);                                                           \
     if (_e != cudaSuccess) return fail(KITE_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
   } while (0)
+  auto bad_delta = [&]() {
+    return fail(KITE_ERR_BAD_INPUT, sizeof(T) == 8 ? "invalid u64 DVLE delta" : "invalid u128 DVLE delta");
+  };
   auto sync = [&]() { return bounded_sync(s, timeout_ms); };
   const uint32_t head_bytes = sizeof(T) + 4;
   // stage timing: [0] decode, [1] tile planning, [2] merge, [3] encode or
@@ -1420,11 +1423,13 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     uint64_t nch = 0;
     for (uint32_t p = 0; p < P; ++p) nch = std::max<uint64_t>(nch, in[i].part_first[p] + in[i].part_count[p]);
     for (uint64_t c = 0; c < nch; ++c) {
-      lo = std::min(lo, in[i].chunk_offset[c]);
-      hi = std::max(hi, in[i].chunk_offset[c] + in[i].chunk_len[c]);
+      const uint64_t off = in[i].chunk_offset[c], len = in[i].chunk_len[c];
+      if (off > in[i].base_len || len > in[i].base_len - off)
+        return fail(KITE_ERR_BAD_INPUT, "chunk out of bounds in input #" + std::to_string(i + 1));
+      lo = std::min(lo, off);
+      hi = std::max(hi, off + len);
     }
     if (nch == 0) lo = hi = 0;
-    if (hi > in[i].base_len) return fail(KITE_ERR_BAD_INPUT, "chunk out of bounds in input #" + std::to_string(i + 1));
     in_span[i] = {lo, hi};
     in_base[i] = total_bytes;
     total_bytes += (hi - lo + 15) & ~15ull;
@@ -1445,7 +1450,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
         sd.head = (codec & KITE_CODEC_DVLE) ? head_bytes : 0;
         if (sd.rows && (codec & KITE_CODEC_DVLE) && sd.byte_len < head_bytes)
           return fail(KITE_ERR_BAD_INPUT, sizeof(T) == 8 ? "u64 DVLE payload too small" : "u128 DVLE payload too small");
-        if (sd.rows && !(codec & KITE_CODEC_DVLE) && sd.byte_len < sd.rows * head_bytes)
+        // two varints a row, of a byte at least (the decode counts them)
+        if (sd.rows && sd.head && sd.rows - 1 > (sd.byte_len - head_bytes) / 2) return bad_delta();
+        if (sd.rows && !(codec & KITE_CODEC_DVLE) && sd.rows > sd.byte_len / head_bytes)
           return fail(KITE_ERR_BAD_INPUT, "raw row payload truncated");
         total_rows += sd.rows;
         streams.push_back(sd);
@@ -1622,9 +1629,6 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       if (cudaEventElapsedTime(&ms, cl.tev[2 + 2 * i], cl.tev[3 + 2 * i]) == cudaSuccess) dec += ms;
     stat->stage_ms[0] = dec;
     if (cudaEventElapsedTime(&ms, cl.tev[0], cl.tev[1]) == cudaSuccess) stat->stage_ms[5] = ms;
-  };
-  auto bad_delta = [&]() {
-    return fail(KITE_ERR_BAD_INPUT, sizeof(T) == 8 ? "invalid u64 DVLE delta" : "invalid u128 DVLE delta");
   };
   DevStatus hdec{};
   MCU(cudaMemcpyAsync(&hdec, dst, sizeof hdec, cudaMemcpyDeviceToHost, s));

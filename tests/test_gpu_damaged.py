@@ -1,6 +1,6 @@
 """Databases whose bytes are damaged: keys above 2^(2k) are merged and written as
-they are, a chunk with fewer rows than its index says is refused, and the context
-works on."""
+they are, a chunk with fewer rows than its index says is refused, as are places
+and row counts that no file has, and the context works on."""
 import random
 
 import pytest
@@ -56,3 +56,23 @@ def test_fewer_rows_than_the_index_says(gpu, orc, k):
                 call()
             assert "KITE_ERR_BAD_INPUT" in str(e.value) and "DVLE delta" in str(e.value)
             assert c.dump(KiteImage.parse(good)) == orc.dump(good)
+
+
+@pytest.mark.parametrize("k,codec", [(21, 2), (21, 1), (45, 2), (45, 1)])
+@pytest.mark.parametrize("rows,offset,length", [
+    (1 << 62, None, None), ((1 << 61) + 1, None, None), ((1 << 60) + 1, None, None), (9001, None, None),
+    (None, (1 << 64) - 8, 16), (None, 1 << 40, None), (None, None, (1 << 64) - 1)])
+def test_index_of_no_file(gpu, orc, k, codec, rows, offset, length):
+    rng = random.Random(4)
+    img = build_image(k, False, 2, [(p, _rows(rng, 900, 2 * k), codec) for p in range(2)])
+    bad = KiteImage.parse(img)
+    c1 = bad.chunks[1]
+    c1.row_count = c1.row_count if rows is None else rows
+    c1.file_offset = c1.file_offset if offset is None else offset
+    c1.encoded_bytes = c1.encoded_bytes if length is None else length
+    with gpu.Counter(k, False, 2) as c:
+        for call in (lambda: c.merge([bad]), lambda: c.dump(bad), lambda: c.histo(bad),
+                     lambda: c.query(bad, list(range(1, 65)))):
+            with pytest.raises(gpu.KiteGpuError, match="KITE_ERR_BAD_INPUT"):
+                call()
+        assert c.dump(KiteImage.parse(img)) == orc.dump(img)
