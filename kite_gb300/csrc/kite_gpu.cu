@@ -171,8 +171,10 @@ int wait_stream(kite_gpu_ctx* ctx, cudaStream_t s) {
 
 int check_status(kite_gpu_ctx* ctx, const char* where) {
   DevStatus st{};
+  int rc = wait_stream(ctx, ctx->stream);  // before the copy: to pageable memory it would wait by itself
+  if (rc) return rc;
   KCU(cudaMemcpyAsync(&st, ctx->status.p, sizeof st, cudaMemcpyDeviceToHost, ctx->stream));
-  int rc = wait_stream(ctx, ctx->stream);
+  rc = wait_stream(ctx, ctx->stream);
   if (rc) return rc;
   if (st.code != KITE_DEV_OK) {
     char buf[256];
@@ -1141,7 +1143,11 @@ int64_t kite_gpu_count_submit_sample(kite_gpu_ctx* ctx, uint32_t sample, const u
     KCU(cudaMalloc(&np, want));
     if (ctx->arena_used) {
       KCU(cudaMemcpyAsync(np, ctx->arena.p, ctx->arena_used, cudaMemcpyDeviceToDevice, ctx->copy_stream));
-      KCU(cudaStreamSynchronize(ctx->copy_stream));
+      const int rc = wait_stream(ctx, ctx->copy_stream);
+      if (rc) {
+        cudaFree(np);
+        return rc;
+      }
     }
     if (ctx->arena.p) cudaFree(ctx->arena.p);
     ctx->arena.p = np;

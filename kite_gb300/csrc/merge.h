@@ -29,13 +29,15 @@ struct MergePool {
   MergePoolSlot slot[kSlots];
   MergePoolSlot host;     // pinned host memory: the tile stream lists on their way to the device
   MergePoolSlot records;  // pinned host memory: a merge's partition records
+  MergePoolSlot results;  // pinned host memory: statuses and other fixed-size results
+  MergePoolSlot rows;     // pinned host memory: a query's keys and counts, a dump's partitions, a histogram's large counts
   MergePool() = default;
   MergePool(const MergePool&) = delete;
   MergePool& operator=(const MergePool&) = delete;
   ~MergePool() {
     for (auto& s : slot) cudaFree(s.p);
-    if (host.p) cudaFreeHost(host.p);
-    if (records.p) cudaFreeHost(records.p);
+    for (auto* h : {&host, &records, &results, &rows})
+      if (h->p) cudaFreeHost(h->p);
   }
 };
 

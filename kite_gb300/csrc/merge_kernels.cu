@@ -1381,6 +1381,36 @@ struct Dev {
   template <class U> U* as() { return static_cast<U*>(p); }
 };
 
+// Pinned host memory of the call, its own or a slot of the pool's.
+struct Pinned {
+  MergePoolSlot own;
+  MergePoolSlot* sl = &own;
+  explicit Pinned(MergePoolSlot* slot) : sl(slot ? slot : &own) {}
+  Pinned(const Pinned&) = delete;
+  Pinned& operator=(const Pinned&) = delete;
+  bool ensure(size_t b) {
+    if (b <= sl->cap) return true;
+    if (sl->p) cudaFreeHost(sl->p);
+    sl->p = nullptr;
+    sl->cap = 0;
+    if (cudaMallocHost(&sl->p, b) != cudaSuccess) return false;
+    sl->cap = b;
+    return true;
+  }
+  ~Pinned() {
+    if (own.p) cudaFreeHost(own.p);
+  }
+  template <class U> U* as() { return static_cast<U*>(sl->p); }
+};
+
+// What the host reads back in fixed sizes.
+struct HostResults {
+  DevStatus decode, run, encode;
+  unsigned plan[3];                         // see k_plan_tiles
+  unsigned long long over[8];               // per group: its first overflowing row
+  unsigned long long hist[kHistBins + 1];   // histo: the bins, and the counts listed
+};
+
 template <class T>
 int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, int n, cudaStream_t s,
                 uint32_t timeout_ms, int mode, kite_gpu_emit_fn emit, void* user, std::string* msg,
@@ -1459,6 +1489,12 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       }
   stat->h2d_bytes += total_bytes;
   MergePool* pool = ex ? ex->pool : nullptr;
+  // The host reads device memory back into pinned memory, or into its own
+  // after a wait: a copy to pageable memory that is queued behind kernels waits
+  // for them inside the copy call, without the deadline.
+  Pinned h_results(pool ? &pool->results : nullptr), h_rows(pool ? &pool->rows : nullptr);
+  if (!h_results.ensure(sizeof(HostResults))) return fail(KITE_ERR_OOM, "merge results (pinned)");
+  HostResults* hr = h_results.as<HostResults>();
   Dev d_bytes(pool, 0), d_streams(pool, 1), d_segs(pool, 2), d_terms(pool, 3), d_vstart(pool, 4), d_dsum(pool, 5),
       d_qseg(pool, 6), d_pfirst(pool, 7), d_status(pool, 8), d_sids(pool, 9), d_kstart(pool, 10), d_keys(pool, 11),
       d_counts(pool, 12), d_first(pool, 13), d_raw(pool, 14);
@@ -1630,8 +1666,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     stat->stage_ms[0] = dec;
     if (cudaEventElapsedTime(&ms, cl.tev[0], cl.tev[1]) == cudaSuccess) stat->stage_ms[5] = ms;
   };
-  DevStatus hdec{};
-  MCU(cudaMemcpyAsync(&hdec, dst, sizeof hdec, cudaMemcpyDeviceToHost, s));
+  MCU(cudaMemcpyAsync(&hr->decode, dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   MCU(cudaEventRecord(sev[1], s));
   auto stage_times = [&]() {
     static const int pairs[5][2] = {{0, 1}, {1, 2}, {2, 3}, {4, 5}, {5, 6}};
@@ -1645,15 +1680,21 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   if (mode == kModeQuery) {
     // ---- query: every key looked up in the streams of its partition ----
     const uint32_t nq = (uint32_t)ex->nq;
-    std::vector<T> qk(nq);
-    for (uint32_t q = 0; q < nq; ++q) qk[q] = (T)(((unsigned __int128)ex->keys[2 * q + 1] << 64) | ex->keys[2 * q]);
     Dev d_qk(pool, 28), d_qp(pool, 29), d_qout(pool, 30);
-    if (!d_qk.ensure(nq * sizeof(T) + 16) || !d_qp.ensure(nq * 4 + 8) || !d_qout.ensure(nq * 8 + 8))
+    if (!d_qk.ensure(nq * sizeof(T) + 16) || !d_qp.ensure(nq * 4 + 8) || !d_qout.ensure(nq * 8 + 8) ||
+        !h_rows.ensure((size_t)nq * (sizeof(T) + 12) + 16))
       return fail(KITE_ERR_OOM, "query buffers");
+    T* qk = h_rows.as<T>();
+    uint64_t* found = reinterpret_cast<uint64_t*>(qk + nq);
+    uint32_t* qp = reinterpret_cast<uint32_t*>(found + nq);
+    for (uint32_t q = 0; q < nq; ++q) {
+      qk[q] = (T)(((unsigned __int128)ex->keys[2 * q + 1] << 64) | ex->keys[2 * q]);
+      qp[q] = ex->parts[q];
+    }
     for (int i = 2; i < 5; ++i) MCU(cudaEventRecord(sev[i], s));
     if (nq) {
-      MCU(cudaMemcpyAsync(d_qk.p, qk.data(), nq * sizeof(T), cudaMemcpyHostToDevice, s));
-      MCU(cudaMemcpyAsync(d_qp.p, ex->parts, nq * 4, cudaMemcpyHostToDevice, s));
+      MCU(cudaMemcpyAsync(d_qk.p, qk, nq * sizeof(T), cudaMemcpyHostToDevice, s));
+      MCU(cudaMemcpyAsync(d_qp.p, qp, nq * 4, cudaMemcpyHostToDevice, s));
       k_query_streams<T><<<(nq + 255) / 256, 256, 0, s>>>(d_keys.as<T>(), d_counts.as<unsigned long long>(),
                                                           d_streams.as<StreamDesc>(), d_pfirst.as<uint32_t>(),
                                                           d_qk.as<T>(), d_qp.as<uint32_t>(), nq,
@@ -1661,13 +1702,12 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       launches++;
     }
     MCU(cudaEventRecord(sev[5], s));
-    std::vector<uint64_t> found(nq);
-    if (nq) MCU(cudaMemcpyAsync(found.data(), d_qout.p, nq * 8, cudaMemcpyDeviceToHost, s));
+    if (nq) MCU(cudaMemcpyAsync(found, d_qout.p, nq * 8, cudaMemcpyDeviceToHost, s));
     MCU(cudaEventRecord(sev[6], s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "query wait");
     MCU(cudaGetLastError());
-    if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
-    if (nq) std::memcpy(ex->counts_out, found.data(), nq * 8);
+    if (hr->decode.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
+    if (nq) std::memcpy(ex->counts_out, found, nq * 8);
     stage_times();
     stat->kernel_launches = launches;
     return KITE_OK;
@@ -1742,12 +1782,11 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   std::vector<uint32_t> tile_first(P + 1, 0);
   const uint64_t out_off = total_rows;  // rows reserved for the output
   uint32_t ntiles = 0;
-  TileStream* tss = nullptr;
-  std::vector<TileStream> tss_own;
+  Pinned h_lists(pool ? &pool->host : nullptr);  // the host's cut: the tiles' stream ranges on their way to the device
   size_t nts_all = 0;
   Dev d_mt(pool, 15), d_ts(pool, 16), d_tds(pool, 22);
   bool planned = false;  // the tiles are on the device
-  unsigned info[3] = {0, 0, 0};
+  unsigned* const info = hr->plan;
   if (total_rows && most_streams <= kMaxTileStreams) {
     const bool slices = most_streams <= 1;
     S = slices ? (uint32_t)((most_rows + kMergeCap - 1) / kMergeCap) : want_ranges();
@@ -1770,9 +1809,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
           d_pos.as<uint64_t>(), d_streams.as<StreamDesc>(), d_pfirst.as<uint32_t>(), P, S, d_mt.as<MergeTile>(),
           d_ts.as<TileStream>(), d_tds.as<TileDesc>(), plan_info);
       launches++;
-      MCU(cudaMemcpyAsync(info, plan_info, sizeof info, cudaMemcpyDeviceToHost, s));
+      MCU(cudaMemcpyAsync(info, plan_info, sizeof hr->plan, cudaMemcpyDeviceToHost, s));
       if (sync()) return fail(KITE_ERR_TIMEOUT, "merge tile wait");
-      if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
+      if (hr->decode.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
       planned = info[0] == 0;
       if (planned) {
         ntiles = (uint32_t)nt;
@@ -1789,7 +1828,6 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   if (S > 1) {
     if (const int rc = make_splitters()) return rc;
     spl.resize(S - 1);
-    MCU(cudaMemcpyAsync(spl.data(), d_spl.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToHost, s));
   }
   auto tp1 = wall();
   // ---- first cut on the device: the row position of every splitter in every
@@ -1798,6 +1836,8 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   std::vector<uint64_t> pos((size_t)nst * SP);
   if (nst && S > 1) {
     if (const int rc = range_positions()) return rc;
+    if (sync()) return fail(KITE_ERR_TIMEOUT, "merge range wait");
+    MCU(cudaMemcpyAsync(spl.data(), d_spl.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToHost, s));
     MCU(cudaMemcpyAsync(pos.data(), d_pos.p, pos.size() * 8, cudaMemcpyDeviceToHost, s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge range wait");
   } else {
@@ -1869,7 +1909,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   for (uint32_t p = 0; p < P; ++p) work.insert(work.end(), cut[p].work.begin(), cut[p].work.end());
   std::vector<uint64_t>().swap(pos);
   // the decode's status arrived with the sync above
-  if (hdec.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
+  if (hr->decode.code == KITE_DEV_SHORT_VARINTS) return bad_delta();
   Dev d_qlo, d_qhi, d_qkey, d_qout;
   std::vector<uint64_t> lp, hp;
   for (int round = 0; !work.empty() && round < 200; ++round) {
@@ -1896,6 +1936,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
                                                       d_qkey.as<T>(), nq, d_qout.as<uint64_t>());
     launches++;
     std::vector<uint64_t> qout(nq);
+    if (sync()) return fail(KITE_ERR_TIMEOUT, "merge tile wait");
     MCU(cudaMemcpyAsync(qout.data(), d_qout.p, nq * 8, cudaMemcpyDeviceToHost, s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge tile wait");
     std::vector<Range> next;
@@ -1990,21 +2031,8 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   nts_all = (size_t)ts_first[P];
   mts.resize(tile_first[P]);
   tds.resize(tile_first[P]);
-  if (pool) {
-    MergePoolSlot& hs = pool->host;
-    const size_t need = nts_all * sizeof(TileStream) + 64;
-    if (hs.cap < need) {
-      if (hs.p) cudaFreeHost(hs.p);
-      hs.p = nullptr;
-      hs.cap = 0;
-      if (cudaMallocHost(&hs.p, need) != cudaSuccess) return fail(KITE_ERR_OOM, "merge tile lists (pinned)");
-      hs.cap = need;
-    }
-    tss = static_cast<TileStream*>(hs.p);
-  } else {
-    tss_own.resize(nts_all + 1);
-    tss = tss_own.data();
-  }
+  if (!h_lists.ensure(nts_all * sizeof(TileStream) + 64)) return fail(KITE_ERR_OOM, "merge tile lists (pinned)");
+  TileStream* tss = h_lists.as<TileStream>();
   parallel_parts([&](uint32_t p) {
     PartTiles& o = pt[p];
     const uint32_t t0 = tile_first[p], s0 = (uint32_t)ts_first[p];
@@ -2035,7 +2063,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     return fail(KITE_ERR_OOM, "merge tile buffers");
   if (!mts.empty()) {
     MCU(cudaMemcpyAsync(d_mt.p, mts.data(), ntiles * sizeof(MergeTile), cudaMemcpyHostToDevice, s));
-    MCU(cudaMemcpyAsync(d_ts.p, tss, nts_all * sizeof(TileStream), cudaMemcpyHostToDevice, s));
+    MCU(cudaMemcpyAsync(d_ts.p, h_lists.as<TileStream>(), nts_all * sizeof(TileStream), cudaMemcpyHostToDevice, s));
     MCU(cudaMemcpyAsync(d_tds.p, tds.data(), ntiles * sizeof(TileDesc), cudaMemcpyHostToDevice, s));
   }
   MCU(cudaMemcpyAsync(d_tf.p, tile_first.data(), (P + 1) * 4, cudaMemcpyHostToDevice, s));
@@ -2128,23 +2156,10 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     }
     if (!d_over.ensure((size_t)NG * 8)) return fail(KITE_ERR_OOM, "merge tile buffers");
     MCU(cudaMemsetAsync(d_over.p, 0xff, (size_t)NG * 8, s));  // per group: its first overflowing row
-    // pinned partition records (kept by the pool)
-    MergePoolSlot hm_own;
-    MergePoolSlot& hms = pool ? pool->records : hm_own;
-    struct HostMem {
-      MergePoolSlot& own;
-      ~HostMem() {
-        if (own.p) cudaFreeHost(own.p);
-      }
-    } hmm{hm_own};
-    if (hms.cap < (size_t)P * sizeof(BucketMeta)) {
-      if (hms.p) cudaFreeHost(hms.p);
-      hms.p = nullptr;
-      hms.cap = 0;
-      MCU(cudaMallocHost(&hms.p, (size_t)P * sizeof(BucketMeta)));
-      hms.cap = (size_t)P * sizeof(BucketMeta);
-    }
-    BucketMeta* hm = static_cast<BucketMeta*>(hms.p);
+    // pinned partition records
+    Pinned h_records(pool ? &pool->records : nullptr);
+    if (!h_records.ensure((size_t)P * sizeof(BucketMeta))) return fail(KITE_ERR_OOM, "merge records (pinned)");
+    BucketMeta* hm = h_records.as<BucketMeta>();
     BucketMeta* hm_dev = nullptr;
     MCU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hm_dev), hm, 0));
     // output buffers: the inputs' payload size to start with (a merged
@@ -2226,11 +2241,11 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       total_out += gbytes;
     }
     MCU(cudaEventRecord(sev[3], s));
-    std::vector<unsigned long long> overs(NG);
-    DevStatus hst{}, hest{};
-    MCU(cudaMemcpyAsync(&hst, dst, sizeof hst, cudaMemcpyDeviceToHost, s));
-    MCU(cudaMemcpyAsync(&hest, est, sizeof hest, cudaMemcpyDeviceToHost, s));
-    MCU(cudaMemcpyAsync(overs.data(), d_over.p, (size_t)NG * 8, cudaMemcpyDeviceToHost, s));
+    unsigned long long* const overs = hr->over;
+    const DevStatus &hst = hr->run, &hest = hr->encode;
+    MCU(cudaMemcpyAsync(&hr->run, dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+    MCU(cudaMemcpyAsync(&hr->encode, est, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
+    MCU(cudaMemcpyAsync(overs, d_over.p, (size_t)NG * 8, cudaMemcpyDeviceToHost, s));
     if (bounded_sync(s, timeout_ms) || bounded_sync(cl.cs, timeout_ms)) return fail(KITE_ERR_TIMEOUT, "merge wait");
     if (hst.code) {
       char b[160];
@@ -2306,8 +2321,8 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   }
   MCU(cudaEventRecord(sev[3], s));
   stat->tiles = ntiles;
-  DevStatus hst{};
-  MCU(cudaMemcpyAsync(&hst, dst, sizeof hst, cudaMemcpyDeviceToHost, s));
+  const DevStatus& hst = hr->run;
+  MCU(cudaMemcpyAsync(&hr->run, dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   auto bad_status = [&]() {
     char b[160];
     snprintf(b, sizeof b, "%s: device status %u (%u, %u, %u)", dump ? "dump" : "merge", hst.code, hst.a, hst.b,
@@ -2316,19 +2331,20 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   };
   if (mode == kModeHisto) {
     // ---- count -> frequency: the small bins, then the listed large counts ----
-    std::vector<unsigned long long> hb(kHistBins + 1);
-    MCU(cudaMemcpyAsync(hb.data(), d_hist.p, (kHistBins + 1) * 8, cudaMemcpyDeviceToHost, s));
+    unsigned long long* const hb = hr->hist;
+    MCU(cudaMemcpyAsync(hb, d_hist.p, sizeof hr->hist, cudaMemcpyDeviceToHost, s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "histo wait");
     if (hst.code) return bad_status();
     const unsigned long long ns = std::min<unsigned long long>(hb[kHistBins], out_off);
-    std::vector<unsigned long long> big(ns);
+    if (!h_rows.ensure(ns * 8 + 8)) return fail(KITE_ERR_OOM, "histo counts (pinned)");
+    unsigned long long* const big = h_rows.as<unsigned long long>();
     MCU(cudaEventRecord(sev[4], s));
-    if (ns) MCU(cudaMemcpyAsync(big.data(), d_okeys.p, ns * 8, cudaMemcpyDeviceToHost, s));
+    if (ns) MCU(cudaMemcpyAsync(big, d_okeys.p, ns * 8, cudaMemcpyDeviceToHost, s));
     MCU(cudaEventRecord(sev[5], s));
     MCU(cudaEventRecord(sev[6], s));
     if (sync()) return fail(KITE_ERR_TIMEOUT, "histo wait");
     stage_times();
-    std::sort(big.begin(), big.end());
+    std::sort(big, big + ns);
     uint64_t keys_out = 0;
     for (uint32_t b = 0; b < kHistBins; ++b) keys_out += hb[b];
     stat->rows = keys_out + ns;
@@ -2336,9 +2352,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     if (!ex || !ex->histo) return KITE_OK;
     for (uint32_t b = 0; b < kHistBins; ++b)
       if (hb[b] && ex->histo(ex->user, b, hb[b])) return fail(KITE_ERR_CALLBACK, "histo callback aborted");
-    for (size_t i = 0; i < big.size();) {
+    for (size_t i = 0; i < ns;) {
       size_t j = i;
-      while (j < big.size() && big[j] == big[i]) ++j;
+      while (j < ns && big[j] == big[i]) ++j;
       if (ex->histo(ex->user, big[i], j - i)) return fail(KITE_ERR_CALLBACK, "histo callback aborted");
       i = j;
     }
@@ -2351,21 +2367,23 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
     if (!d_boff.ensure((ntiles + 1) * 8) || !d_lines.ensure(P * sizeof(PartLines)) ||
         !d_scan.ensure(scan_tmp_elems(ntiles + 1) * 8 + 64))
       return fail(KITE_ERR_OOM, "dump output");
-    std::vector<PartLines> lines(P);
+    if (!h_rows.ensure(P * sizeof(PartLines))) return fail(KITE_ERR_OOM, "dump records (pinned)");
+    PartLines* const lines = h_rows.as<PartLines>();
+    std::memset(lines, 0, P * sizeof(PartLines));
     if (ntiles) {
       k_part_lines<T><<<(P + 7) / 8, 256, 0, s>>>(d_tout.as<TileOut<T>>(), d_tf.as<uint32_t>(), P,
                                                   d_boff.as<unsigned long long>(), d_lines.as<PartLines>());
       launches += 1 + exclusive_scan_u64(d_boff.as<unsigned long long>(), d_boff.as<unsigned long long>(), ntiles,
                                          d_scan.as<unsigned long long>(), s);
-      MCU(cudaMemcpyAsync(lines.data(), d_lines.p, P * sizeof(PartLines), cudaMemcpyDeviceToHost, s));
+      MCU(cudaMemcpyAsync(lines, d_lines.p, P * sizeof(PartLines), cudaMemcpyDeviceToHost, s));
     }
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge wait");
     if (hst.code) return bad_status();
     unsigned long long acc = 0;
     uint64_t out_rows = 0;
-    for (const PartLines& l : lines) {
-      acc += l.bytes;
-      out_rows += l.rows;
+    for (uint32_t p = 0; p < P; ++p) {
+      acc += lines[p].bytes;
+      out_rows += lines[p].rows;
     }
     if (!d_out.ensure(acc + 16)) return fail(KITE_ERR_OOM, "dump output");
     MCU(cudaEventRecord(sev[4], s));

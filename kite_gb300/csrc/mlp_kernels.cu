@@ -579,7 +579,8 @@ int predict_imbalance(MlpModel* m, const T* d_sample, uint32_t n, const T* d_spl
   const uint32_t grid = std::min<uint32_t>((n + 255) / 256, 4 * (uint32_t)std::max(sms, 1));
   k_tile_hits<T><<<grid, 256, (size_t)S * 4, s>>>(d_sample, n, d_spl, S, m->tile_hits);
   std::vector<unsigned> h(S);
-  cudaMemcpyAsync(h.data(), m->tile_hits, (size_t)S * 4, cudaMemcpyDeviceToHost, s);
+  if (bounded_sync(s, timeout_ms)) return 1;  // before the copy: to pageable memory it would wait by itself
+  if (cudaMemcpyAsync(h.data(), m->tile_hits, (size_t)S * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return 1;
   if (bounded_sync(s, timeout_ms)) return 1;
   unsigned mx = 0;
   for (unsigned v : h) mx = std::max(mx, v);
@@ -685,7 +686,8 @@ int train(MlpModel* m, uint32_t n, cudaStream_t s, uint32_t timeout_ms, float* f
     launches++;
   }
   float l[2] = {0.f, 0.f};
-  cudaMemcpyAsync(l, m->loss, sizeof l, cudaMemcpyDeviceToHost, s);
+  if (bounded_sync(s, timeout_ms)) return -1;
+  if (cudaMemcpyAsync(l, m->loss, sizeof l, cudaMemcpyDeviceToHost, s) != cudaSuccess) return -1;
   if (bounded_sync(s, timeout_ms)) return -1;
   if (final_loss) *final_loss = l[1];
   return launches;
