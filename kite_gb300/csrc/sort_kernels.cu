@@ -680,6 +680,37 @@ __device__ __forceinline__ void list_others(const TileRetry& r, const unsigned* 
   else empty_tile(&tout[i]);
 }
 
+// Whether a tile holds one key alone (a partition of reads of one base): seen by
+// reading its keys, where counting them would be an atomic on one slot for each
+// (200,000 reads of G, 24M copies: the tile sort 28.8 -> 8.2 ms, most of it now the
+// empty tiles).  `other` is a zeroed flag, zeroed again.  Not inlined: its
+// registers in the loop over the tiles took 1.3% of the tile sort's time.
+__device__ __noinline__ bool one_key(const uint64_t* keys, uint64_t start, uint32_t n, volatile unsigned* other) {
+  constexpr int NT = TableSmem::NT, UN = 4;
+  const uint32_t lane = threadIdx.x & 31, head = (uint32_t)(start & 1u), pairs = (head + n + 1) >> 1;
+  const uint4* p4 = reinterpret_cast<const uint4*>(keys + (start & ~1ull));
+  const unsigned long long key = keys[start];
+  for (uint32_t p0 = threadIdx.x; p0 - lane < pairs; p0 += UN * NT) {
+    uint4 x[UN];
+#pragma unroll
+    for (int q = 0; q < UN; ++q) x[q] = p0 + q * NT < pairs ? p4[p0 + q * NT] : make_uint4(0, 0, 0, 0);
+    bool differs = false;
+#pragma unroll
+    for (int q = 0; q < UN; ++q) {
+      const uint32_t i0 = 2 * (p0 + q * NT) - head;  // wraps for the key before the tile
+      differs |= i0 < n && ((unsigned long long)x[q].y << 32 | x[q].x) != key;
+      differs |= i0 + 1 < n && ((unsigned long long)x[q].w << 32 | x[q].z) != key;
+    }
+    if (differs) *other = 1;
+    if (__any_sync(0xffffffffu, differs || *other)) break;
+  }
+  __syncthreads();
+  const bool one = *other == 0;
+  __syncthreads();
+  if (threadIdx.x == 0) *other = 0;
+  return one;
+}
+
 __global__ void __launch_bounds__(TableSmem::NT, 2)
     k_tile_table(uint64_t* __restrict__ keys, uint32_t* __restrict__ counts, const TileDesc* __restrict__ tiles,
                  uint32_t ntiles, TileOut<uint64_t>* __restrict__ tout, unsigned long long* fallbacks,
@@ -701,42 +732,6 @@ __global__ void __launch_bounds__(TableSmem::NT, 2)
   auto fetch = [&](const TileIn<uint64_t>& t, uint32_t p) {
     if (p < ((uint32_t)(t.start & 1u) + t.n + 1) >> 1) ka = reinterpret_cast<const uint4*>(keys + (t.start & ~1ull))[p];
   };
-  // Whether a tile above twice the capacity holds one key alone (a partition of
-  // reads of one base): seen by reading its keys, where counting them would be
-  // an atomic on one slot for each (200,000 reads of G, 24M copies: the tile sort
-  // 28.8 -> 8.2 ms, most of it now the empty tiles).
-  auto one_key = [&](const TileIn<uint64_t>& t) {
-    if (t.n <= 2u * tile_capacity<uint64_t>()) return false;
-    const uint32_t head = (uint32_t)(t.start & 1u), pairs = (head + t.n + 1) >> 1;
-    const uint4* p4 = reinterpret_cast<const uint4*>(keys + (t.start & ~1ull));
-    const unsigned long long key = keys[t.start];
-    constexpr int UN = 4;
-    for (uint32_t p0 = threadIdx.x; p0 - lane < pairs; p0 += UN * NT) {
-      uint4 x[UN];
-#pragma unroll
-      for (int q = 0; q < UN; ++q) x[q] = p0 + q * NT < pairs ? p4[p0 + q * NT] : make_uint4(0, 0, 0, 0);
-      bool other = false;
-#pragma unroll
-      for (int q = 0; q < UN; ++q) {
-        const uint32_t i0 = 2 * (p0 + q * NT) - head;  // wraps for the key before the tile
-        other |= i0 < t.n && ((unsigned long long)x[q].y << 32 | x[q].x) != key;
-        other |= i0 + 1 < t.n && ((unsigned long long)x[q].w << 32 | x[q].z) != key;
-      }
-      if (other) misc[1] = 1;
-      if (__any_sync(0xffffffffu, other || *(volatile unsigned*)&misc[1])) break;
-    }
-    __syncthreads();
-    const bool one = misc[1] == 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      misc[1] = 0;
-      if (one) {
-        counts[t.start] = t.n;  // the key is in place
-        if (fallbacks) atomicAdd(&fallbacks[1], 1ull);
-      }
-    }
-    return one;
-  };
   if (threadIdx.x < 8) misc[threadIdx.x] = threadIdx.x == 6 && (blockIdx.x & 31u) && mostly_binned(retry);
   __syncthreads();
   bool skip = misc[6] || rg.wait_polls;  // a bound on the binning sort's wait (tests of its timeout): every tile goes there
@@ -746,12 +741,15 @@ __global__ void __launch_bounds__(TableSmem::NT, 2)
   for (uint32_t i = blockIdx.x, par = 0; i < ntiles; par ^= 1) {
     const uint32_t n = t.n;
     if (threadIdx.x == 0) choose_next(retry, &misc[4]);
-    const bool one = n && !skip && one_key(t);
+    const bool one = n > 2u * tile_capacity<uint64_t>() && !skip && one_key(keys, t.start, n, &misc[1]);
     if (n == 0 || skip || one) {
       if (threadIdx.x == 0) {
         if (n == 0) empty_tile(&tout[i]);
-        else if (one) tout[i] = TileOut<uint64_t>{keys[t.start], keys[t.start], 1u, n, 0ull};
-        else retry.add(i, n);
+        else if (one) {
+          counts[t.start] = n;  // the key is in place
+          tout[i] = TileOut<uint64_t>{keys[t.start], keys[t.start], 1u, n, 0ull};
+          if (fallbacks) atomicAdd(&fallbacks[1], 1ull);
+        } else retry.add(i, n);
       }
       skip = rg.wait_polls;
       __syncthreads();
