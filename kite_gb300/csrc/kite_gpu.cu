@@ -169,13 +169,7 @@ int wait_stream(kite_gpu_ctx* ctx, cudaStream_t s) {
   return rc;
 }
 
-int check_status(kite_gpu_ctx* ctx, const char* where) {
-  DevStatus st{};
-  int rc = wait_stream(ctx, ctx->stream);  // before the copy: to pageable memory it would wait by itself
-  if (rc) return rc;
-  KCU(cudaMemcpyAsync(&st, ctx->status.p, sizeof st, cudaMemcpyDeviceToHost, ctx->stream));
-  rc = wait_stream(ctx, ctx->stream);
-  if (rc) return rc;
+int check_status(kite_gpu_ctx* ctx, const DevStatus& st, const char* where) {
   if (st.code != KITE_DEV_OK) {
     char buf[256];
     snprintf(buf, sizeof buf, "%s: device status %u (%u, %u, %u)", where, st.code, st.a, st.b, st.c);
@@ -911,6 +905,8 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   KCU(cudaEventRecord(ctx->ev[7], s));
   KCU(cudaMemcpyAsync(ctx->h_small.p, ctx->sort_stats.p, 16, cudaMemcpyDeviceToHost, s));
   KCU(cudaMemcpyAsync(ctx->h_tiles.p, ctx->tile_lists.p, lbytes, cudaMemcpyDeviceToHost, s));
+  const DevStatus* hstatus = reinterpret_cast<const DevStatus*>(ctx->h_tiles.as<uint8_t>() + lbytes);
+  KCU(cudaMemcpyAsync(ctx->h_tiles.as<uint8_t>() + lbytes, ctx->status.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   rc = wait_stream(ctx, s);
   const auto wall2 = clk::now();
   if (!rc && to_host) rc = wait_stream(ctx, ctx->copy_stream);
@@ -931,7 +927,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     st.big_tile_keys = hs2[3];
     st.range_imbalance = S > 1 ? (double)rmax / ((double)N / S) : 1.0;  // 1: one tile per bucket
   }
-  rc = check_status(ctx, "count");
+  rc = check_status(ctx, *hstatus, "count");
   if (rc) return rc;
   for (uint32_t g = 0; g < NG; ++g) {
     float a = 0, b = 0, c = 0, d = 0;
