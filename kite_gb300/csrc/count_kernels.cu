@@ -1191,8 +1191,7 @@ struct RunScatterSmem {
   static constexpr size_t o_stage = 0;
   static constexpr size_t o_gpos = o_stage + (size_t)BATCH * sizeof(T);
   static constexpr size_t o_whist = o_gpos + (size_t)RADIX * 8;
-  static constexpr size_t o_dtot = o_whist + (size_t)RADIX * 4;
-  static constexpr size_t o_dstart = o_dtot + (size_t)RADIX * 4;
+  static constexpr size_t o_dstart = o_whist + (size_t)RADIX * 4;
   static constexpr size_t o_scan = o_dstart + (size_t)RADIX * 4;
   static constexpr size_t o_dig = o_scan + 64 * 4;
   static constexpr size_t total = o_dig + (size_t)BATCH * 2;
@@ -1466,7 +1465,9 @@ struct ScatterCfg {
 
 // Calls f(ScatterCfg<...>{}) for the scatter instance of D digits and launch
 // shape 0..3 (threads x keys per thread; 0 picks 256 x 8 for up to 256 digits
-// and 512 x 8 above: twice the keys per batch for four times the destinations).
+// and 512 x 8 above: twice the keys per batch for four times the destinations.
+// u128 keys take half the keys per thread; u64 keys of stored digits above 256
+// go by runs instead, 512 x 12).
 template <class T, class F>
 static void with_scatter_cfg(uint32_t D, int shape, F&& f) {
   constexpr int W = sizeof(T) == 8 ? 1 : 2;  // u128 keys: half the keys per thread
@@ -1487,51 +1488,46 @@ static void with_scatter_cfg(uint32_t D, int shape, F&& f) {
   }
 }
 
-template <class T>
-void launch_split_scatter(const TileSplitParams<T>& p, int shape, cudaStream_t s) {
+// Calls f(kernel, threads, shared memory) for the scatter kernel of D digits and
+// the launch shape; false when there is none.
+template <class T, class F>
+static bool with_scatter_kernel(uint32_t D, int shape, bool digits, F&& f) {
   if constexpr (sizeof(T) == 8) {
-    if (p.dig && p.D > 256 && shape == 0) {
-      auto kern = k_split_scatter_runs<T, 512, 12, kMaxDigits, 2>;
-      const size_t smem = RunScatterSmem<T, 512, 12, kMaxDigits>::total;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (p.R * p.G) kern<<<p.R * p.G, 512, smem, s>>>(p);
-      return;
+    if (digits && D > 256 && shape == 0) {
+      f(k_split_scatter_runs<T, 512, 12, kMaxDigits, 2>, 512, RunScatterSmem<T, 512, 12, kMaxDigits>::total);
+      return true;
     }
   }
-  with_scatter_cfg<T>(p.D, shape, [&](auto cfg) {
+  bool found = digits;
+  with_scatter_cfg<T>(D, shape, [&](auto cfg) {
     using C = decltype(cfg);
-    if (p.dig) {
-      auto kern = k_split_scatter_bulk<T, C::NT, C::IT, C::RADIX>;
-      const size_t smem = BulkScatterSmem<T, C::NT, C::IT, C::RADIX>::total;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (p.R * p.G) kern<<<p.R * p.G, C::NT, smem, s>>>(p);
-      return;
-    }
-    if constexpr (C::RADIX == 16) {  // the first of two levels: at most four coarse ranges
-      auto kern = k_split_scatter<T, C::NT, C::IT, C::RADIX>;
-      const size_t smem = ScatterSmem<T, C::NT, C::IT, C::RADIX>::total;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (p.R * p.G) kern<<<p.R * p.G, C::NT, smem, s>>>(p);
+    if (digits) {  // a last level, whose digits the histogram pass left
+      f(k_split_scatter_bulk<T, C::NT, C::IT, C::RADIX>, C::NT, BulkScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
+    } else if constexpr (C::RADIX == 16) {  // the first of two levels: at most four coarse ranges
+      f(k_split_scatter<T, C::NT, C::IT, C::RADIX>, C::NT, ScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
+      found = true;
     }
   });
+  return found;
 }
 
 template <class T>
-uint32_t split_scatter_slots(uint32_t D, int shape) {
+cudaError_t launch_split_scatter(const TileSplitParams<T>& p, int shape, cudaStream_t s) {
+  const bool found = with_scatter_kernel<T>(p.D, shape, p.dig != nullptr, [&](auto kern, int nt, size_t smem) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (p.R * p.G) kern<<<p.R * p.G, nt, smem, s>>>(p);
+  });
+  return found ? cudaGetLastError() : cudaErrorNotSupported;
+}
+
+template <class T>
+uint32_t split_scatter_slots(uint32_t D, int shape, bool digits) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  with_scatter_cfg<T>(D, shape, [&](auto cfg) {
-    using C = decltype(cfg);
-    auto slots = [&](auto kern, size_t smem) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
-    };
-    // more than 16 digits: a last level, whose digits the histogram pass left
-    if constexpr (C::RADIX > 16)
-      slots(k_split_scatter_bulk<T, C::NT, C::IT, C::RADIX>, BulkScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
-    else
-      slots(k_split_scatter<T, C::NT, C::IT, C::RADIX>, ScatterSmem<T, C::NT, C::IT, C::RADIX>::total);
+  with_scatter_kernel<T>(D, shape, digits, [&](auto kern, int nt, size_t smem) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem);
   });
   return (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per_sm);
 }
@@ -1548,9 +1544,9 @@ void launch_region_bounds(const unsigned long long* off, uint32_t nreg, uint32_t
 
 template void launch_split_hist<uint64_t>(const TileSplitParams<uint64_t>&, cudaStream_t);
 template void launch_split_hist<u128>(const TileSplitParams<u128>&, cudaStream_t);
-template void launch_split_scatter<uint64_t>(const TileSplitParams<uint64_t>&, int, cudaStream_t);
-template void launch_split_scatter<u128>(const TileSplitParams<u128>&, int, cudaStream_t);
-template uint32_t split_scatter_slots<uint64_t>(uint32_t, int);
-template uint32_t split_scatter_slots<u128>(uint32_t, int);
+template cudaError_t launch_split_scatter<uint64_t>(const TileSplitParams<uint64_t>&, int, cudaStream_t);
+template cudaError_t launch_split_scatter<u128>(const TileSplitParams<u128>&, int, cudaStream_t);
+template uint32_t split_scatter_slots<uint64_t>(uint32_t, int, bool);
+template uint32_t split_scatter_slots<u128>(uint32_t, int, bool);
 
 }  // namespace kite

@@ -637,8 +637,8 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     // G parts per region (parts of >= 32K keys, G <= 64): the fewest parts
     // whose CTAs fill the scatter's resident slots in whole waves, as far as
     // a 2% gain in the used fraction of the last wave goes.
-    auto parts = [&](uint64_t regions, uint64_t max_region, uint32_t D) {
-      const uint64_t slots = split_scatter_slots<T>(D, ctx->cfg.scatter_shape);
+    auto parts = [&](uint64_t regions, uint64_t max_region, uint32_t D, bool digits) {
+      const uint64_t slots = split_scatter_slots<T>(D, ctx->cfg.scatter_shape, digits);
       const uint64_t gmax = std::min<uint64_t>(64, std::max<uint64_t>(1, max_region / 32768));
       uint64_t best = 1;
       double best_used = 0.0;
@@ -666,7 +666,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     T* level_out = ctx->keys_b.as<T>();
     if (D1 > 1) {
       // level 1: buckets -> (bucket, coarse range); coarse splitter c is tile splitter (c+1)*D2-1
-      const uint32_t G1 = pieces * parts((uint64_t)PT * pieces, maxpc, D1);
+      const uint32_t G1 = pieces * parts((uint64_t)PT * pieces, maxpc, D1, false);
       const size_t n1 = (size_t)PT * D1 * G1;
       KCU(ctx->lvl_count.ensure(n1 * 8));
       KCU(ctx->lvl_off.ensure(n1 * 8));
@@ -690,11 +690,11 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
       launch_split_hist<T>(t1, s);
       st.kernel_launches += 3 + exclusive_scan_u64(t1.tile_count, ctx->lvl_off.as<unsigned long long>(), n1,
                                                    ctx->scan_tmp.as<unsigned long long>(), s);
-      launch_split_scatter<T>(t1, ctx->cfg.scatter_shape, s);
+      KCU(launch_split_scatter<T>(t1, ctx->cfg.scatter_shape, s));
       launch_region_bounds(t1.tile_off, PT * D1, G1, N, ctx->reg_off.as<unsigned long long>(),
                            ctx->reg_cnt.as<unsigned long long>(), s);
       // level 2: (bucket, coarse c) -> tiles c*D2 .. c*D2+D2-1
-      G = parts((uint64_t)PT * D1, (maxb + D1 - 1) / D1 * 2, D2);
+      G = parts((uint64_t)PT * D1, (maxb + D1 - 1) / D1 * 2, D2, true);
       tp.region_off = ctx->reg_off.as<unsigned long long>();
       tp.region_count = ctx->reg_cnt.as<unsigned long long>();
       tp.R = PT * D1;
@@ -703,7 +703,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
       tp.spl_region_stride = D2;
       std::swap(level_in, level_out);
     } else {
-      G = pieces * parts((uint64_t)PT * pieces, maxpc, D2);
+      G = pieces * parts((uint64_t)PT * pieces, maxpc, D2, true);
       tp.region_off = (pieces > 1 ? ctx->piece_off : ctx->bucket_off).as<unsigned long long>();
       tp.region_count = (pieces > 1 ? ctx->piece_cnt : ctx->bucket_count).as<unsigned long long>();
       tp.pieces = pieces;
@@ -727,7 +727,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
     launch_split_hist<T>(tp, s);
     st.kernel_launches += 3 + exclusive_scan_u64(tp.tile_count, ctx->tile_off.as<unsigned long long>(), ntg,
                                                  ctx->scan_tmp.as<unsigned long long>(), s);
-    launch_split_scatter<T>(tp, ctx->cfg.scatter_shape, s);
+    KCU(launch_split_scatter<T>(tp, ctx->cfg.scatter_shape, s));
     KCU(ctx->tiles.ensure(nt * sizeof(TileDesc)));
     KCU(ctx->tile_fill.ensure(nt * 4));
     launch_make_tiles(ctx->tile_off.as<unsigned long long>(), (uint32_t)nt, S, G, N, ctx->tiles.as<TileDesc>(),

@@ -91,7 +91,7 @@ struct ExtractParams {
 };
 
 // One level of the key-range split.  Region r (a hash bucket, or one coarse
-// key range of a bucket) is cut into D <= 256 digits by D-1 of the global
+// key range of a bucket) is cut into D <= 1024 digits by D-1 of the global
 // splitters: spl[spl_first + (r % spl_mod) * spl_region_stride + i * spl_step]
 // for i < D-1 (spl_total splitters in all).  Each region is processed in G
 // parts.
@@ -104,7 +104,7 @@ struct TileSplitParams {
   const T* splitters;     // spl_total ascending keys
   uint32_t spl_total;
   uint32_t R;             // regions
-  uint32_t D;             // digits per region (2..256)
+  uint32_t D;             // digits per region (2..1024)
   uint32_t G;             // parts per region
   uint32_t spl_first, spl_step, spl_mod, spl_region_stride;
   uint32_t key_bits;      // 2k: significant key bits
@@ -150,10 +150,13 @@ void launch_sample_bucket_counts(const unsigned* m, const unsigned long long* co
                                  unsigned long long* bucket_count, cudaStream_t s);
 template <class T>
 void launch_split_hist(const TileSplitParams<T>& p, cudaStream_t s);
+// shape 0..3: threads x keys.  Without stored digits (p.dig null) at most 16
+// digits; more are refused (cudaErrorNotSupported).
 template <class T>
-void launch_split_scatter(const TileSplitParams<T>& p, int shape, cudaStream_t s);  // shape 0..3: threads x keys
+cudaError_t launch_split_scatter(const TileSplitParams<T>& p, int shape, cudaStream_t s);
+// Resident CTAs on the device of the kernel that launch_split_scatter takes.
 template <class T>
-uint32_t split_scatter_slots(uint32_t D, int shape);  // resident scatter CTAs on the device
+uint32_t split_scatter_slots(uint32_t D, int shape, bool digits);
 void launch_make_tiles(const unsigned long long* off, uint32_t ntiles, uint32_t S, uint32_t G,
                        unsigned long long n_keys, TileDesc* tiles, uint32_t* lens, cudaStream_t s);
 void launch_region_bounds(const unsigned long long* off, uint32_t nreg, uint32_t G, unsigned long long n_keys,
