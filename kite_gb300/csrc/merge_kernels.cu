@@ -1786,6 +1786,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   size_t nts_all = 0;
   Dev d_mt(pool, 15), d_ts(pool, 16), d_tds(pool, 22);
   bool planned = false;  // the tiles are on the device
+  uint32_t cut = 1;      // ranges whose splitters and positions are on the device
   unsigned* const info = hr->plan;
   if (total_rows && most_streams <= kMaxTileStreams) {
     const bool slices = most_streams <= 1;
@@ -1795,6 +1796,7 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
       if (!slices && S > 1) {
         if (const int rc = make_splitters()) return rc;
         if (const int rc = range_positions()) return rc;
+        cut = S;
       } else {
         if (!d_pos.ensure(npos * 8)) return fail(KITE_ERR_OOM, "merge range positions");
         k_slice_positions<T><<<(unsigned)((npos + 255) / 256), 256, 0, s>>>(
@@ -1824,10 +1826,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   if (!planned) {
   // ---- the host's cut ----
   S = total_rows ? want_ranges() : 1;
-  std::vector<T> spl;
-  if (S > 1) {
+  std::vector<T> spl(S - 1);
+  if (S > 1 && S != cut) {  // else the plan's are the same
     if (const int rc = make_splitters()) return rc;
-    spl.resize(S - 1);
   }
   auto tp1 = wall();
   // ---- first cut on the device: the row position of every splitter in every
@@ -1835,7 +1836,9 @@ int merge_typed(uint32_t P, uint32_t key_bits, const kite_gpu_merge_input* in, i
   const size_t SP = (size_t)S + 1;
   std::vector<uint64_t> pos((size_t)nst * SP);
   if (nst && S > 1) {
-    if (const int rc = range_positions()) return rc;
+    if (S != cut) {
+      if (const int rc = range_positions()) return rc;
+    }
     if (sync()) return fail(KITE_ERR_TIMEOUT, "merge range wait");
     MCU(cudaMemcpyAsync(spl.data(), d_spl.p, (S - 1) * sizeof(T), cudaMemcpyDeviceToHost, s));
     MCU(cudaMemcpyAsync(pos.data(), d_pos.p, pos.size() * 8, cudaMemcpyDeviceToHost, s));
