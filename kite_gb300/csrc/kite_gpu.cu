@@ -816,11 +816,12 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
                         s);
     launch_tile_sort_listed<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_1 + t0, walk_grid,
                                lcnt + 4 * g + 2, tout, sstats,
-                               TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls}, s);
+                               TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls},
+                               ctx->status.as<DevStatus>(), s);
     cudaEventRecord(gev[8 * g + 1], s);
     if (some_above) launch_tile_sort_large<T>(sorted, ctx->counts.as<uint32_t>(), ctx->tiles.as<TileDesc>(), ids_a + t0, walk_grid,
                               lcnt + 4 * g, tout, sstats, TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls},
-                              s);
+                              ctx->status.as<DevStatus>(), s);
     if (some_above) launch_big_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), scratch, ctx->tiles.as<TileDesc>(), ids_b + t0,
                             walk_grid, lcnt + 4 * g + 1, tout, ctx->status.as<DevStatus>(), sstats, s);
     cudaEventRecord(gev[8 * g + 2], s);

@@ -249,19 +249,20 @@ struct TileRetry {
 template <class T>
 void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t ntiles, TileOut<T>* out,
                       unsigned long long* fallbacks, TileRanges<T> rg, TileRetry retry, cudaStream_t s);
-// The binning sort of the tiles listed in ids (at most tile_capacity keys each),
-// their number on the device; two CTAs for each of `grid`.
+// The binning sort of the tiles listed in ids (at most tile_capacity keys each; a
+// larger one is reported in st, as KITE_DEV_TILE_OVERFLOW, and left without
+// rows), their number on the device; two CTAs for each of `grid`.
 template <class T>
 void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
                              const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
-                             TileRanges<T> rg, cudaStream_t s);
+                             TileRanges<T> rg, DevStatus* st, cudaStream_t s);
 // Tiles of tile_capacity < len <= 2 * tile_capacity, listed in ids: the same
 // binning sort with twice the shared memory (one CTA per SM).  With nids_dev,
 // the list's length is on the device and the nids CTAs walk it in turn.
 template <class T>
 void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
-                            TileRanges<T> rg, cudaStream_t s);
+                            TileRanges<T> rg, DevStatus* st, cudaStream_t s);
 // Oversized tiles (more keys than 2 * tile_capacity): one CTA per tile, LSD
 // passes through global memory with `scratch` (>= largest tile keys); with
 // nbig_dev as above; sort_stats[1] gains the rows they make.

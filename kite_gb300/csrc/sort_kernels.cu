@@ -335,7 +335,7 @@ constexpr unsigned long long kBulkTimeoutFlag = 1ull << 40;  // added to the sor
 template <class T, int MULT>
 __device__ __forceinline__ void sort_tile(uint32_t tid, T* __restrict__ keys, uint32_t* __restrict__ counts,
                                           const TileDesc* __restrict__ tiles, TileOut<T>* __restrict__ tout,
-                                          unsigned long long* fallbacks, const TileRanges<T>& rg) {
+                                          unsigned long long* fallbacks, const TileRanges<T>& rg, DevStatus* st) {
   using L = BinSmem<T, MULT>;
   constexpr int NT = L::NT, NW = L::NW, ITEMS = L::ITEMS;
   extern __shared__ __align__(16) uint8_t sm[];
@@ -350,15 +350,10 @@ __device__ __forceinline__ void sort_tile(uint32_t tid, T* __restrict__ keys, ui
 
   const TileDesc td = tiles[tid];
   const unsigned n = td.len;
-  if (n > (unsigned)L::CAP) return;  // oversized tiles take a larger path
-  if (n == 0) {
+  if (n == 0 || n > (unsigned)L::CAP) {  // the lists have no such tile
     if (threadIdx.x == 0) {
-      TileOut<T> o;
-      o.first_key = o.last_key = T(0);
-      o.rows = 0;
-      o.first_count = 0;
-      o.rest_bytes = 0;
-      tout[tid] = o;
+      empty_tile(&tout[tid]);
+      dev_fail(st, KITE_DEV_TILE_OVERFLOW, tid, n, L::CAP);
     }
     return;
   }
@@ -1200,26 +1195,26 @@ template <class T, int MULT>
 __global__ void __launch_bounds__(kTileThreads * MULT, MULT == 1 ? 2 : 1)
     k_tile_sort(T* __restrict__ keys, uint32_t* __restrict__ counts, const TileDesc* __restrict__ tiles,
                 const uint32_t* __restrict__ ids, const unsigned* __restrict__ nids, TileOut<T>* __restrict__ tout,
-                unsigned long long* fallbacks, TileRanges<T> rg) {
+                unsigned long long* fallbacks, TileRanges<T> rg, DevStatus* st) {
   if (nids) {
     const unsigned cnt = *nids;
     for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
-      sort_tile<T, MULT>(ids[i], keys, counts, tiles, tout, fallbacks, rg);
+      sort_tile<T, MULT>(ids[i], keys, counts, tiles, tout, fallbacks, rg, st);
       __syncthreads();  // shared memory is reused by the next tile
     }
   } else {
-    sort_tile<T, MULT>(ids ? ids[blockIdx.x] : blockIdx.x, keys, counts, tiles, tout, fallbacks, rg);
+    sort_tile<T, MULT>(ids ? ids[blockIdx.x] : blockIdx.x, keys, counts, tiles, tout, fallbacks, rg, st);
   }
 }
 
 template <class T, int MULT>
 static void tile_sort_with(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids,
                            const unsigned* nids, uint32_t n, TileOut<T>* out, unsigned long long* fallbacks,
-                           TileRanges<T> rg, cudaStream_t s) {
+                           TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
   const size_t smem = BinSmem<T, MULT>::total;
   cudaFuncSetAttribute(k_tile_sort<T, MULT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(k_tile_sort<T, MULT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (n) k_tile_sort<T, MULT><<<n, BinSmem<T, MULT>::NT, smem, s>>>(keys, counts, tiles, ids, nids, out, fallbacks, rg);
+  if (n) k_tile_sort<T, MULT><<<n, BinSmem<T, MULT>::NT, smem, s>>>(keys, counts, tiles, ids, nids, out, fallbacks, rg, st);
 }
 
 template <class T>
@@ -1241,14 +1236,14 @@ void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t
 template <class T>
 void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
                              const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
-                             TileRanges<T> rg, cudaStream_t s) {
-  tile_sort_with<T, 1>(keys, counts, tiles, ids, nids_dev, 2 * grid, out, fallbacks, rg, s);
+                             TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
+  tile_sort_with<T, 1>(keys, counts, tiles, ids, nids_dev, 2 * grid, out, fallbacks, rg, st, s);
 }
 template <class T>
 void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
-                            TileRanges<T> rg, cudaStream_t s) {
-  tile_sort_with<T, 2>(keys, counts, tiles, ids, nids_dev, nids, out, fallbacks, rg, s);
+                            TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
+  tile_sort_with<T, 2>(keys, counts, tiles, ids, nids_dev, nids, out, fallbacks, rg, st, s);
 }
 template void launch_tile_sort<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, uint32_t, TileOut<uint64_t>*,
                                          unsigned long long*, TileRanges<uint64_t>, TileRetry, cudaStream_t);
@@ -1256,16 +1251,16 @@ template void launch_tile_sort<u128>(u128*, uint32_t*, const TileDesc*, uint32_t
                                      TileRanges<u128>, TileRetry, cudaStream_t);
 template void launch_tile_sort_listed<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
                                                 const unsigned*, TileOut<uint64_t>*, unsigned long long*,
-                                                TileRanges<uint64_t>, cudaStream_t);
+                                                TileRanges<uint64_t>, DevStatus*, cudaStream_t);
 template void launch_tile_sort_listed<u128>(u128*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
                                             const unsigned*, TileOut<u128>*, unsigned long long*, TileRanges<u128>,
-                                            cudaStream_t);
+                                            DevStatus*, cudaStream_t);
 template void launch_tile_sort_large<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
                                                const unsigned*, TileOut<uint64_t>*, unsigned long long*,
-                                               TileRanges<uint64_t>, cudaStream_t);
+                                               TileRanges<uint64_t>, DevStatus*, cudaStream_t);
 template void launch_tile_sort_large<u128>(u128*, uint32_t*, const TileDesc*, const uint32_t*, uint32_t,
                                            const unsigned*, TileOut<u128>*, unsigned long long*, TileRanges<u128>,
-                                           cudaStream_t);
+                                            DevStatus*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Oversized tiles: one CTA, LSD passes through global memory.  Each pass
