@@ -823,7 +823,7 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
                               lcnt + 4 * g, tout, sstats, TileRanges<T>{tile_spl, S, 0, kmax, ctx->cfg.tile_wait_polls},
                               ctx->status.as<DevStatus>(), s);
     if (some_above) launch_big_tile_sort<T>(sorted, ctx->counts.as<uint32_t>(), scratch, ctx->tiles.as<TileDesc>(), ids_b + t0,
-                            walk_grid, lcnt + 4 * g + 1, tout, ctx->status.as<DevStatus>(), sstats, s);
+                            walk_grid, lcnt + 4 * g + 1, tout, sstats, s);
     cudaEventRecord(gev[8 * g + 2], s);
     // ---- K5: per-bucket tile links, byte offsets from the group's start
     launch_tile_link<T>(tout + t0, nb, S, ctx->tile_boff.as<unsigned long long>() + t0, ctx->tile_prev.as<T>() + t0,

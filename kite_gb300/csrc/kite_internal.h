@@ -221,9 +221,6 @@ struct TileRanges {
   uint32_t wait_polls;  // bound of the first wait for a tile's bulk load (1: a single non-blocking test)
 };
 
-// `fallbacks` (device counters): [0] tiles that took the LSD fallback (plus
-// 2^40 for a tile whose bulk load did not complete), [1] rows of the tiles
-// above the on-chip capacity (double-capacity and global-memory sorts).
 // The lists of the tiles that the tile sort's tables leave to the binning sort.
 struct TileRetry {
   uint32_t* ids1;   // tiles of at most tile_capacity keys
@@ -246,6 +243,11 @@ struct TileRetry {
   }
 #endif
 };
+// The sort of all tiles by tables of distinct keys; what a table does not suit
+// is listed in `retry`.  `fallbacks` (device counters, for this and the two
+// binning sorts): [0] tiles counted with hashed homes (u64) and tiles of the
+// binning sort that took LSD passes, plus 2^40 for a tile whose bulk load did
+// not complete; [1] rows of the tiles above the on-chip capacity, by any sort.
 template <class T>
 void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t ntiles, TileOut<T>* out,
                       unsigned long long* fallbacks, TileRanges<T> rg, TileRetry retry, cudaStream_t s);
@@ -254,22 +256,22 @@ void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t
 // rows), their number on the device; two CTAs for each of `grid`.
 template <class T>
 void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
-                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+                             const unsigned* nids, TileOut<T>* out, unsigned long long* fallbacks,
                              TileRanges<T> rg, DevStatus* st, cudaStream_t s);
 // Tiles of tile_capacity < len <= 2 * tile_capacity, listed in ids: the same
-// binning sort with twice the shared memory (one CTA per SM).  With nids_dev,
-// the list's length is on the device and the nids CTAs walk it in turn.
+// binning sort with twice the shared memory (one CTA per SM); `grid` CTAs walk
+// the list.
 template <class T>
-void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
-                            const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
+                            const unsigned* nids, TileOut<T>* out, unsigned long long* fallbacks,
                             TileRanges<T> rg, DevStatus* st, cudaStream_t s);
 // Oversized tiles (more keys than 2 * tile_capacity): one CTA per tile, LSD
-// passes through global memory with `scratch` (>= largest tile keys); with
-// nbig_dev as above; sort_stats[1] gains the rows they make.
+// passes through global memory with `scratch` (as long as the keys); the list
+// and `grid` as above; sort_stats[1] gains the rows they make.
 template <class T>
 void launch_big_tile_sort(T* keys, uint32_t* counts, T* scratch, const TileDesc* tiles, const uint32_t* big_ids,
-                          uint32_t nbig, const unsigned* nbig_dev, TileOut<T>* out, DevStatus* st,
-                          unsigned long long* sort_stats, cudaStream_t s);
+                          uint32_t grid, const unsigned* nbig, TileOut<T>* out, unsigned long long* sort_stats,
+                          cudaStream_t s);
 // Tile statistics; see k_tile_stats.
 void launch_tile_stats(const uint32_t* lens, uint32_t ntiles, uint32_t S, uint32_t cap, unsigned long long* stats,
                        unsigned long long* range, cudaStream_t s);

@@ -395,12 +395,7 @@ __device__ __forceinline__ void sort_tile(uint32_t tid, T* __restrict__ keys, ui
     if (threadIdx.x == 0) {
       mbar_wait(bar, 0, kBulkDrainPolls);
       if (fallbacks) atomicAdd(fallbacks, kBulkTimeoutFlag);
-      TileOut<T> o;  // an empty tile for the link and encode kernels that follow
-      o.first_key = o.last_key = T(0);
-      o.rows = 0;
-      o.first_count = 0;
-      o.rest_bytes = 0;
-      tout[tid] = o;
+      empty_tile(&tout[tid]);  // for the link and encode kernels that follow
     }
     __syncthreads();
     return;
@@ -656,7 +651,7 @@ __device__ __forceinline__ TileIn<T> tile_in(const TileDesc* tiles, uint32_t i, 
 // the tables have met 16 tiles and more than a quarter of them were better
 // binned; one tile in 32 (and, of the CTAs' first ones, one CTA in 32) still
 // tries.  (1M random 150 bp reads, every key once:
-// 1.68 ms binned, 6.9 ms when every tile tried the u64 table first, 1.72 ms so.)
+// 1.68 ms binned, 6.9 ms when every tile tried the u64 table first, 1.64-1.72 ms so.)
 __device__ __forceinline__ bool mostly_binned(const TileRetry& r) {
   const unsigned a = *(volatile unsigned*)&r.met[0], f = *(volatile unsigned*)&r.met[1];
   return a >= 16 && 4 * f > a;
@@ -1189,32 +1184,27 @@ __global__ void __launch_bounds__(HashSmem::NT, 2)
   }
 }
 
-// One CTA per tile: tile blockIdx.x (+ the launch's first) or ids[blockIdx.x];
-// with a device count, CTAs walk ids[0 .. *nids) in turn.
+// CTAs walk the tiles ids[0 .. *nids) in turn.
 template <class T, int MULT>
 __global__ void __launch_bounds__(kTileThreads * MULT, MULT == 1 ? 2 : 1)
     k_tile_sort(T* __restrict__ keys, uint32_t* __restrict__ counts, const TileDesc* __restrict__ tiles,
                 const uint32_t* __restrict__ ids, const unsigned* __restrict__ nids, TileOut<T>* __restrict__ tout,
                 unsigned long long* fallbacks, TileRanges<T> rg, DevStatus* st) {
-  if (nids) {
-    const unsigned cnt = *nids;
-    for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
-      sort_tile<T, MULT>(ids[i], keys, counts, tiles, tout, fallbacks, rg, st);
-      __syncthreads();  // shared memory is reused by the next tile
-    }
-  } else {
-    sort_tile<T, MULT>(ids ? ids[blockIdx.x] : blockIdx.x, keys, counts, tiles, tout, fallbacks, rg, st);
+  const unsigned cnt = *nids;
+  for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
+    sort_tile<T, MULT>(ids[i], keys, counts, tiles, tout, fallbacks, rg, st);
+    __syncthreads();  // shared memory is reused by the next tile
   }
 }
 
 template <class T, int MULT>
 static void tile_sort_with(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids,
-                           const unsigned* nids, uint32_t n, TileOut<T>* out, unsigned long long* fallbacks,
+                           const unsigned* nids, uint32_t grid, TileOut<T>* out, unsigned long long* fallbacks,
                            TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
   const size_t smem = BinSmem<T, MULT>::total;
   cudaFuncSetAttribute(k_tile_sort<T, MULT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(k_tile_sort<T, MULT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (n) k_tile_sort<T, MULT><<<n, BinSmem<T, MULT>::NT, smem, s>>>(keys, counts, tiles, ids, nids, out, fallbacks, rg, st);
+  k_tile_sort<T, MULT><<<grid, BinSmem<T, MULT>::NT, smem, s>>>(keys, counts, tiles, ids, nids, out, fallbacks, rg, st);
 }
 
 template <class T>
@@ -1235,15 +1225,15 @@ void launch_tile_sort(T* keys, uint32_t* counts, const TileDesc* tiles, uint32_t
 }
 template <class T>
 void launch_tile_sort_listed(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
-                             const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+                             const unsigned* nids, TileOut<T>* out, unsigned long long* fallbacks,
                              TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
-  tile_sort_with<T, 1>(keys, counts, tiles, ids, nids_dev, 2 * grid, out, fallbacks, rg, st, s);
+  tile_sort_with<T, 1>(keys, counts, tiles, ids, nids, 2 * grid, out, fallbacks, rg, st, s);
 }
 template <class T>
-void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t nids,
-                            const unsigned* nids_dev, TileOut<T>* out, unsigned long long* fallbacks,
+void launch_tile_sort_large(T* keys, uint32_t* counts, const TileDesc* tiles, const uint32_t* ids, uint32_t grid,
+                            const unsigned* nids, TileOut<T>* out, unsigned long long* fallbacks,
                             TileRanges<T> rg, DevStatus* st, cudaStream_t s) {
-  tile_sort_with<T, 2>(keys, counts, tiles, ids, nids_dev, nids, out, fallbacks, rg, st, s);
+  tile_sort_with<T, 2>(keys, counts, tiles, ids, nids, grid, out, fallbacks, rg, st, s);
 }
 template void launch_tile_sort<uint64_t>(uint64_t*, uint32_t*, const TileDesc*, uint32_t, TileOut<uint64_t>*,
                                          unsigned long long*, TileRanges<uint64_t>, TileRetry, cudaStream_t);
@@ -1271,8 +1261,7 @@ template void launch_tile_sort_large<u128>(u128*, uint32_t*, const TileDesc*, co
 template <class T>
 __device__ __forceinline__ void big_sort_tile(uint32_t tid, T* __restrict__ keys, uint32_t* __restrict__ counts,
                                               T* __restrict__ scratch, const TileDesc* __restrict__ tiles,
-                                              TileOut<T>* __restrict__ tout, DevStatus* st,
-                                              unsigned long long* sstats) {
+                                              TileOut<T>* __restrict__ tout, unsigned long long* sstats) {
   using L = TileSmem<T>;
   constexpr int NT = L::NT, ITEMS = L::ITEMS, CAP = L::CAP;
   extern __shared__ __align__(16) uint8_t sm[];
@@ -1430,43 +1419,34 @@ __device__ __forceinline__ void big_sort_tile(uint32_t tid, T* __restrict__ keys
     o.rest_bytes = rest_total;
     tout[tid] = o;
   }
-  (void)st;
 }
 
-// One CTA per listed tile, or (device count) CTAs walking the list in turn.
+// CTAs walk the tiles big_ids[0 .. *nids) in turn.
 template <class T>
 __global__ void __launch_bounds__(kTileThreads, 1)
     k_big_tile_sort(T* __restrict__ keys, uint32_t* __restrict__ counts, T* __restrict__ scratch,
                     const TileDesc* __restrict__ tiles, const uint32_t* __restrict__ big_ids,
-                    const unsigned* __restrict__ nids, TileOut<T>* __restrict__ tout, DevStatus* st,
-                    unsigned long long* sstats) {
-  if (nids) {
-    const unsigned cnt = *nids;
-    for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
-      big_sort_tile<T>(big_ids[i], keys, counts, scratch, tiles, tout, st, sstats);
-      __syncthreads();  // shared memory is reused by the next tile
-    }
-  } else {
-    big_sort_tile<T>(big_ids[blockIdx.x], keys, counts, scratch, tiles, tout, st, sstats);
+                    const unsigned* __restrict__ nids, TileOut<T>* __restrict__ tout, unsigned long long* sstats) {
+  const unsigned cnt = *nids;
+  for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
+    big_sort_tile<T>(big_ids[i], keys, counts, scratch, tiles, tout, sstats);
+    __syncthreads();  // shared memory is reused by the next tile
   }
 }
 
 template <class T>
 void launch_big_tile_sort(T* keys, uint32_t* counts, T* scratch, const TileDesc* tiles, const uint32_t* big_ids,
-                          uint32_t nbig, const unsigned* nbig_dev, TileOut<T>* out, DevStatus* st,
-                          unsigned long long* sort_stats, cudaStream_t s) {
+                          uint32_t grid, const unsigned* nbig, TileOut<T>* out, unsigned long long* sort_stats,
+                          cudaStream_t s) {
   const size_t smem = TileSmem<T>::total;
   cudaFuncSetAttribute(k_big_tile_sort<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (nbig)
-    k_big_tile_sort<T><<<nbig, kTileThreads, smem, s>>>(keys, counts, scratch, tiles, big_ids, nbig_dev, out, st,
-                                                         sort_stats);
+  k_big_tile_sort<T><<<grid, kTileThreads, smem, s>>>(keys, counts, scratch, tiles, big_ids, nbig, out, sort_stats);
 }
 template void launch_big_tile_sort<uint64_t>(uint64_t*, uint32_t*, uint64_t*, const TileDesc*, const uint32_t*,
-                                             uint32_t, const unsigned*, TileOut<uint64_t>*, DevStatus*,
-                                             unsigned long long*, cudaStream_t);
+                                             uint32_t, const unsigned*, TileOut<uint64_t>*, unsigned long long*,
+                                             cudaStream_t);
 template void launch_big_tile_sort<u128>(u128*, uint32_t*, u128*, const TileDesc*, const uint32_t*, uint32_t,
-                                         const unsigned*, TileOut<u128>*, DevStatus*, unsigned long long*,
-                                         cudaStream_t);
+                                         const unsigned*, TileOut<u128>*, unsigned long long*, cudaStream_t);
 
 // Statistics of the tiles: stats[0] largest tile, [1] keys, [2] non-empty
 // tiles, [3] keys in the tiles above `cap`, [4] those tiles, range[t] keys in
