@@ -521,13 +521,18 @@ int run_count(kite_gpu_ctx* ctx, bool to_host) {
   // tiles) as it is; beyond that a power of two, so that the two levels divide
   // it evenly.  (A tile's fixed cost is that of about 1,500 keys: 16 samples of
   // 50,000 reads in 6 tiles per bucket instead of 32 sort in 1.03 ms instead of
-  // 2.28.)
+  // 2.28.)  A load that brings tiles above twice the capacity (from 1.8: the
+  // largest are some 1.1 times the mean) is sorted through global memory where
+  // it does; there the tiles are a multiple of 32, mostly smaller than asked for
+  // (500,000 reads at k = 51 and a load of 2.6: 3.5 ms, 10.1 in as few tiles as the
+  // load allows).
   const double fill = std::min(4.0, std::max(0.05, ctx->cfg.tile_fill));
   uint32_t S = 1;
   if ((double)maxb > fill * CAP) {
     const double want = std::ceil((double)maxb / (fill * CAP));
     if (want <= 1024.0) {
       S = (uint32_t)want;
+      if (fill > 1.8) S = std::min<uint32_t>(1024, (S + 31) & ~31u);
     } else {
       S = 2048;
       while ((double)S < want && S < 4096) S <<= 1;
